@@ -429,19 +429,17 @@ static int ensure_batch_scratch(spmx_handle_t h, int total) {
     dfree(p);
     p = nullptr;
   }
-  dfree(h->batch_hist);
-  dfree(h->batch_hoff);
+  dfree(h->batch_radix);
   dfree(h->batch_invptr);
   dfree(h->batch_rec);
   h->batch_rec = nullptr;
-  h->batch_hist = h->batch_hoff = h->batch_invptr = nullptr;
+  h->batch_radix = nullptr;
+  h->batch_invptr = nullptr;
   h->batch_cap = 0;
   const char* what[6] = {"batch keys", "batch keys alt", "batch entries", "batch entries alt",
                          "batch vectors", "batch vectors alt"};
   for (int b = 0; b < 6; ++b) SPMX_TRY(dalloc(&h->batch_buf[b], 4 * (size_t)cap, what[b]));
-  const size_t hn = radix_hist_ints(cap);
-  SPMX_TRY(dalloc((void**)&h->batch_hist, 4 * hn, "batch hist"));
-  SPMX_TRY(dalloc((void**)&h->batch_hoff, 4 * hn, "batch hist off"));
+  SPMX_TRY(dalloc(&h->batch_radix, radix_scratch_bytes(cap), "batch radix scratch"));
   SPMX_TRY(dalloc((void**)&h->batch_invptr, 4 * ((size_t)h->n + 1), "batch inverse pointers"));
   SPMX_TRY(dalloc(&h->batch_rec, batch_rec4_offset(cap) + 16 * (size_t)cap, "batch pair records"));
   h->batch_cap = cap;
@@ -478,10 +476,10 @@ static int batch_invert(spmx_handle_t h, int nvec, int total, const int* xptr, c
     batch_keys_kernel<<<std::min((total + 255) / 256, h->num_sms * 8), 256, 0, st>>>(
         h->n, nvec, total, xptr, xkey, b[0], b[2], b[4], h->d_err);
   }
-  RadixBuffers rb{b[0], b[1], b[2], b[3], b[4], b[5], h->batch_hist, h->batch_hoff, false};
+  RadixBuffers rb{b[0], b[1], b[2], b[3], b[4], b[5], h->batch_radix};
   int bits = 1;
   while ((1LL << bits) <= (long long)h->n) ++bits;  // keys in [0, n]
-  if (radix_sort_pairs(rb, total, bits, h->ls, h->d_err, st))
+  if (radix_sort_pairs(rb, total, bits, h->d_err, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "batch sort capacity");
   const unsigned* skey = rb.result_in_alt ? b[1] : b[0];
   *inv_ent = rb.result_in_alt ? b[3] : b[2];

@@ -190,12 +190,13 @@ extern "C" int spmx_create(int m, int n, int nnz, spmx_handle_t* out) {
 
 static void free_sort_scratch(spmx_handle_t h) {
   dfree(h->sk); dfree(h->sk_alt); dfree(h->sv); dfree(h->sv_alt);
-  dfree(h->shist); dfree(h->shist_off); dfree(h->sslot);
+  dfree(h->sradix); dfree(h->sslot);
   dfree(h->sy_key); dfree(h->sy_val);
   dfree(h->bk_gcount); dfree(h->bk_boff); dfree(h->bk_cursor);
   h->bk_gcount = h->bk_boff = h->bk_cursor = nullptr;
   h->sk = h->sk_alt = h->sv = h->sv_alt = nullptr;
-  h->shist = h->shist_off = h->sslot = nullptr;
+  h->sradix = nullptr;
+  h->sslot = nullptr;
   h->sy_key = nullptr;
   h->sy_val = nullptr;
   h->sort_ready = false;
@@ -237,7 +238,7 @@ extern "C" int spmx_destroy(spmx_handle_t h) {
   dfree(h->ms_q0); dfree(h->ms_q1); dfree(h->ms_srcs); dfree(h->ms_tmp); dfree(h->ms_ctrl);
   dfree(h->ms_hchunk); dfree(h->ms_hcnt); dfree(h->ms_hacc); dfree(h->ms_hleft); dfree(h->ms_hcounters);
   for (void* p : h->batch_buf) dfree(p);
-  dfree(h->batch_hist); dfree(h->batch_hoff); dfree(h->batch_invptr); dfree(h->batch_rec);
+  dfree(h->batch_radix); dfree(h->batch_invptr); dfree(h->batch_rec);
   dfree(h->batch_chunk); dfree(h->batch_ctr);
   delete h;
   return SPMX_SUCCESS;
@@ -324,9 +325,7 @@ static int ensure_sort_scratch(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&h->sv, 4 * cap, "sort vals"));
   SPMX_TRY(dalloc((void**)&h->sv_alt, 4 * cap, "sort vals alt"));
   SPMX_TRY(dalloc((void**)&h->sslot, 4 * cap, "sort slots"));
-  const size_t hn = radix_hist_ints((int)cap);
-  SPMX_TRY(dalloc((void**)&h->shist, 4 * hn, "radix hist"));
-  SPMX_TRY(dalloc((void**)&h->shist_off, 4 * hn, "radix hist off"));
+  SPMX_TRY(dalloc(&h->sradix, radix_scratch_bytes((int)cap), "radix scratch"));
   const size_t ycap = (size_t)std::max(h->m, 1);
   SPMX_TRY(dalloc((void**)&h->sy_key, 4 * ycap, "sparse y keys"));
   SPMX_TRY(dalloc((void**)&h->sy_val, 4 * ycap, "sparse y vals"));
@@ -363,9 +362,8 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
   if (nnz > 0) {
     // stable sort of the row-major COO by column
     unsigned *k0 = nullptr, *k1 = nullptr, *r0 = nullptr, *r1 = nullptr, *v0 = nullptr, *v1 = nullptr;
-    int *hist = nullptr, *hoff = nullptr;
+    void* radix = nullptr;
     const size_t b = 4 * (size_t)nnz;
-    const size_t hn = radix_hist_ints(nnz);
     int rc = SPMX_SUCCESS;
     rc = rc ? rc : dalloc((void**)&k0, b, "t keys");
     rc = rc ? rc : dalloc((void**)&k1, b, "t keys alt");
@@ -375,14 +373,13 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
       rc = rc ? rc : dalloc((void**)&v0, b, "t vals");
       rc = rc ? rc : dalloc((void**)&v1, b, "t vals alt");
     }
-    rc = rc ? rc : dalloc((void**)&hist, 4 * hn, "t hist");
-    rc = rc ? rc : dalloc((void**)&hoff, 4 * hn, "t hist off");
+    rc = rc ? rc : dalloc(&radix, radix_scratch_bytes(nnz), "t radix scratch");
     if (!rc) {
       cudaMemcpyAsync(k0, h->col, b, cudaMemcpyDeviceToDevice, st);
       if (h->val) cudaMemcpyAsync(v0, h->val, b, cudaMemcpyDeviceToDevice, st);
       launch_expand_rows(m, h->rowptr, r0, st);
-      RadixBuffers rb{k0, k1, r0, r1, v0, v1, hist, hoff, false};
-      if (radix_sort_pairs(rb, nnz, ceil_log2(std::max(n, 2)), h->ls, h->d_err, st))
+      RadixBuffers rb{k0, k1, r0, r1, v0, v1, radix};
+      if (radix_sort_pairs(rb, nnz, ceil_log2(std::max(n, 2)), h->d_err, st))
         rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
       if (!rc) {
         unsigned* rr = rb.result_in_alt ? r1 : r0;
@@ -392,7 +389,7 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
       }
     }
     cudaError_t se = cudaStreamSynchronize(st);
-    dfree(k0); dfree(k1); dfree(r0); dfree(r1); dfree(v0); dfree(v1); dfree(hist); dfree(hoff);
+    dfree(k0); dfree(k1); dfree(r0); dfree(r1); dfree(v0); dfree(v1); dfree(radix);
     if (rc) { dfree(cnt); return rc; }
     if (se != cudaSuccess) { dfree(cnt); return set_error(SPMX_ERR_CUDA, cudaGetErrorString(se)); }
   }
@@ -861,8 +858,8 @@ static int csc_sort(spmx_handle_t h, int variant, float alpha, float* y, int* yk
     launch_csc_lb(a, h->cs, variant == SPMX_CSC_LB_MERGE ? 1 : 2, nullptr, (int*)h->sk,
                   (float*)h->sv, h->lb_grid, st);
   }
-  RadixBuffers rb{h->sk, h->sk_alt, h->sv, h->sv_alt, nullptr, nullptr, h->shist, h->shist_off, false};
-  if (radix_sort_pairs(rb, bin_len, ceil_log2(std::max(h->m, 2)), h->ls, h->d_err, st))
+  RadixBuffers rb{h->sk, h->sk_alt, h->sv, h->sv_alt, nullptr, nullptr, h->sradix};
+  if (radix_sort_pairs(rb, bin_len, ceil_log2(std::max(h->m, 2)), h->d_err, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
   const unsigned* keys = rb.result_in_alt ? h->sk_alt : h->sk;
   const float* vals = (const float*)(rb.result_in_alt ? h->sv_alt : h->sv);

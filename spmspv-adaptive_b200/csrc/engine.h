@@ -65,8 +65,7 @@ struct spmx_handle_s {
   unsigned* sk_alt = nullptr;
   unsigned* sv = nullptr;
   unsigned* sv_alt = nullptr;
-  int* shist = nullptr;
-  int* shist_off = nullptr;
+  void* sradix = nullptr;     // radix_scratch_bytes
   int* sslot = nullptr;
   int* sy_key = nullptr;      // internal sparse y (adaptive path)
   float* sy_val = nullptr;
@@ -123,8 +122,7 @@ struct spmx_handle_s {
   // batched SpMSpV: the batch inverted by column (radix sort buffers for
   // keys / entries / vectors and their alternates, column pointers)
   void* batch_buf[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  int* batch_hist = nullptr;
-  int* batch_hoff = nullptr;
+  void* batch_radix = nullptr;  // radix_scratch_bytes
   int* batch_invptr = nullptr;
   int batch_cap = 0;
   int batch_invptr_n = -1;

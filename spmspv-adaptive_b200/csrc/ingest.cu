@@ -121,10 +121,9 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
     const int bits_c = key_bits(n), bits_r = key_bits(m);
     const int passes = (col_desc ? (bits_c + 7) / 8 : 0) + (bits_r + 7) / 8;
     const int fin = passes & 1;  // set holding the result after the last pass
-    const size_t hn = radix_hist_ints(nnz);
     const size_t al = (b + 255) & ~(size_t)255;
-    const size_t hb = (4 * hn + 255) & ~(size_t)255;
-    rc = dalloc((void**)&scratch, al * (val ? 4 : 3) + 2 * hb, "coo sort scratch");
+    const size_t hb = radix_scratch_bytes(nnz);
+    rc = dalloc((void**)&scratch, al * (val ? 4 : 3) + hb, "coo sort scratch");
     if (!rc) {
       unsigned *k[2], *r[2], *v[2] = {nullptr, nullptr};
       char* q = scratch;
@@ -136,21 +135,20 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
         v[fin] = (unsigned*)nval;
         v[1 - fin] = (unsigned*)q; q += al;
       }
-      int* hist = (int*)q; q += hb;
-      int* hoff = (int*)q;
+      void* radix = q;
       cudaMemcpyAsync(k[0], col, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
       cudaMemcpyAsync(r[0], row, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
       if (val) cudaMemcpyAsync(v[0], val, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
       int s = 0;  // set holding the current order
       if (col_desc) {
-        RadixBuffers ra{k[s], k[1 - s], r[s], r[1 - s], v[s], v[1 - s], hist, hoff, false};
-        if (radix_sort_pairs(ra, nnz, bits_c, h->ls, h->d_err, st))
+        RadixBuffers ra{k[s], k[1 - s], r[s], r[1 - s], v[s], v[1 - s], radix};
+        if (radix_sort_pairs(ra, nnz, bits_c, h->d_err, st))
           rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
         if (ra.result_in_alt) s = 1 - s;
       }
       if (!rc) {
-        RadixBuffers rb{r[s], r[1 - s], k[s], k[1 - s], v[s], v[1 - s], hist, hoff, false};
-        if (radix_sort_pairs(rb, nnz, bits_r, h->ls, h->d_err, st))
+        RadixBuffers rb{r[s], r[1 - s], k[s], k[1 - s], v[s], v[1 - s], radix};
+        if (radix_sort_pairs(rb, nnz, bits_r, h->d_err, st))
           rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
         if (rb.result_in_alt) s = 1 - s;
       }

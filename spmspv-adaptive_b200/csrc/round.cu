@@ -721,22 +721,23 @@ static int round_build(spmx_handle_t h, long long rcap, long long avail, int par
   const size_t b4 = 4 * (size_t)std::max(nnz, 1);
   unsigned *k0 = nullptr, *k1 = nullptr, *a0 = nullptr, *a1 = nullptr, *v0 = nullptr, *v1 = nullptr;
   unsigned *q0 = nullptr, *q1 = nullptr;
-  int *hist = nullptr, *hoff = nullptr, *flags = nullptr, *d_bounds = nullptr, *spr = nullptr;
-  const size_t hn = radix_hist_ints(std::max(nnz, 1));
+  void* radix = nullptr;
+  int *flags = nullptr, *d_bounds = nullptr, *spr = nullptr;
+  const size_t rsb = radix_scratch_bytes(std::max(nnz, 1));
   int rc = SPMX_SUCCESS;
   // the build's temporaries whose sizes are known now, carved from one
   // allocation (one cudaMalloc and one cudaFree per build instead of one per
   // array: the build took 31 ms of host time around 3.7 ms of kernels)
   int *occ = nullptr, *ppos = nullptr, *d_bslots = nullptr, *d_segb = nullptr;
   Arena tmp;
-  tmp.plan(8 * b4 + 2 * 4 * hn + 16 + 4 * ((size_t)nrb + 1) + 4 * ((size_t)m + 1) + b4 + 4 * ((size_t)nrb + 1));
+  tmp.plan(8 * b4 + rsb + 16 + 4 * ((size_t)nrb + 1) + 4 * ((size_t)m + 1) + b4 + 4 * ((size_t)nrb + 1));
   rc = rc ? rc : tmp.alloc("round build scratch");
   if (!rc) {
     k0 = tmp.take<unsigned>(b4); k1 = tmp.take<unsigned>(b4);
     a0 = tmp.take<unsigned>(b4); a1 = tmp.take<unsigned>(b4);
     v0 = tmp.take<unsigned>(b4); v1 = tmp.take<unsigned>(b4);
     q0 = tmp.take<unsigned>(b4); q1 = tmp.take<unsigned>(b4);
-    hist = tmp.take<int>(4 * hn); hoff = tmp.take<int>(4 * hn);
+    radix = tmp.take<char>(rsb);
     flags = tmp.take<int>(16);
     d_bounds = tmp.take<int>(4 * ((size_t)nrb + 1));
     spr = tmp.take<int>(4 * ((size_t)m + 1));
@@ -756,8 +757,8 @@ static int round_build(spmx_handle_t h, long long rcap, long long avail, int par
     note_launch();
     round_keys_kernel<<<(unsigned)(((long long)m * 32 + 255) / 256), 256, 0, st>>>(
         m, n, h->rowptr, h->col, h->val, t->rb_row, nrb, cbits, k0, a0, v0, flags);
-    RadixBuffers rbuf{k0, k1, a0, a1, v0, v1, hist, hoff, false};
-    if (radix_sort_pairs(rbuf, nnz, cbits + bbits, h->ls, h->d_err, st))
+    RadixBuffers rbuf{k0, k1, a0, a1, v0, v1, radix};
+    if (radix_sort_pairs(rbuf, nnz, cbits + bbits, h->d_err, st))
       rc = set_error(SPMX_ERR_INVALID_VALUE, "round SpMV: sort capacity");
     if (!rc) {
       skey = rbuf.result_in_alt ? k1 : k0;
@@ -912,8 +913,8 @@ static int round_build(spmx_handle_t h, long long rcap, long long avail, int par
       note_launch();
       round_key2_kernel<<<nrounds, 256, 0, st>>>(d_rstart, d_rlen, slrow, q0, pos_in);
       // second stable sort: by (round, local row), payload the column-order position
-      RadixBuffers r2{q0, q1, pos_in, pos_alt, nullptr, nullptr, hist, hoff, false};
-      if (radix_sort_pairs(r2, nvalid, 16 + bits_for((long long)nrounds), h->ls, h->d_err, st))
+      RadixBuffers r2{q0, q1, pos_in, pos_alt, nullptr, nullptr, radix};
+      if (radix_sort_pairs(r2, nvalid, 16 + bits_for((long long)nrounds), h->d_err, st))
         rc = set_error(SPMX_ERR_INVALID_VALUE, "round SpMV: sort capacity");
       if (!rc) {
         const unsigned* key2 = r2.result_in_alt ? q1 : q0;

@@ -6,11 +6,25 @@
 // :412) and cuSPARSE csr2csc inside ToCSC (H:409): a transpose is a stable
 // sort of the row-major COO by column.
 //
-// One pass = 8 key bits: (1) per-tile digit histograms, stored digit-major,
-// (2) exclusive scan of the histograms, (3) stable scatter.  Inside a tile each
-// warp owns 512 consecutive items and ranks them round by round with
-// __match_any_sync; warp-private digit counters are then offset across warps,
-// so the order of equal digits follows the input order (stability).
+// A sort is one histogram kernel, which reads the keys once and counts the
+// digits of every pass, and one kernel per pass of at most 8 bits (the bits
+// are spread evenly over the passes: fewer digits, longer runs of equal digits
+// in the output).  A pass reads and writes every array once.  Its tiles chain
+// through per-digit decoupled look-back words, so the digit counts of a tile
+// never make a round trip through memory; the tile is put in digit order in
+// shared memory first, so a warp's stores cover runs of consecutive addresses.
+//
+// What bounds a pass: instruction issue and the shared-memory exchange (about
+// 130 warp instructions per 32 items with two payloads) ahead of DRAM, which
+// moves 2 x 12 bytes per item.  16.8M items with two payloads: 119 us per pass
+// (3.4 TB/s) and 34 us for the histogram; the form before (per-tile histogram,
+// scan of the histograms, scatter straight from registers, each 4-byte store in
+// a sector of its own) took 430 + 37 + 13 us per pass.  Measured beside it:
+// peers by __match_any_sync 210 us, by one ballot per digit bit 143 us, by the
+// shared match word 128 us (512 threads, 6,144 items); 256 threads and 4,096
+// items 119 us, 5,120 items 128 us, 384 threads and 4,608 items 126 us.
+#include <algorithm>
+
 #include "kernels.h"
 #include "sort.h"
 #include "common.cuh"
@@ -18,83 +32,231 @@
 namespace spmx {
 
 constexpr int kRadixNT = 256;
-constexpr int kRadixIPT = 16;                       // items per thread
-constexpr int kRadixTile = kRadixNT * kRadixIPT;    // 4096
+constexpr int kRadixWarps = kRadixNT / 32;
 constexpr int kRadixDigits = 256;
+constexpr int kRadixMaxPasses = 8;  // two 31-bit keys
 
-__global__ void __launch_bounds__(kRadixNT)
-radix_hist_kernel(const unsigned* __restrict__ keys, int n, int shift,
-                  int ntiles, int* __restrict__ hist) {
-  __shared__ int s_h[kRadixDigits];
-  const int tile = blockIdx.x;
-  s_h[threadIdx.x] = 0;
-  __syncthreads();
-  const int base = tile * kRadixTile;
-#pragma unroll 4
-  for (int j = 0; j < kRadixIPT; ++j) {
-    const int i = base + j * kRadixNT + threadIdx.x;
-    if (i < n) atomicAdd(&s_h[(__ldg(keys + i) >> shift) & 0xff], 1);
+// look-back words: [63:34] pass + 1, [33:32] 1 = tile count, 2 = inclusive
+// prefix, [31:0] value; cleared once per sort, the pass number tells the
+// passes apart
+struct RadixPass {
+  const unsigned *k_in, *p1_in, *p2_in;
+  unsigned *k_out, *p1_out, *p2_out;
+  int n, shift, bits, lo_bits, pass, ntiles;
+  unsigned long long* status;  // [ntiles][256]
+  unsigned* ticket;
+  const unsigned* ghist;       // [256] digit counts of this pass
+  int* err;
+};
+
+// digit of an item; with two keys the sort key is (p1 << lo_bits) | key
+template <bool TWO>
+__device__ __forceinline__ unsigned radix_digit(unsigned lo, unsigned hi, int lo_bits, int shift, unsigned mask) {
+  if (TWO) {
+    const unsigned long long k = ((unsigned long long)hi << lo_bits) | lo;
+    return (unsigned)(k >> shift) & mask;
   }
-  __syncthreads();
-  hist[threadIdx.x * ntiles + tile] = s_h[threadIdx.x];
+  return (lo >> shift) & mask;
 }
 
-template <int NPAY>
+// digit counts of all passes: pass p has the bits [first + p * bits, first +
+// (p + 1) * bits)
+template <bool TWO>
 __global__ void __launch_bounds__(kRadixNT)
-radix_scatter_kernel(const unsigned* __restrict__ keys_in,
-                     const unsigned* __restrict__ p1_in,
-                     const unsigned* __restrict__ p2_in, int n, int shift,
-                     int ntiles, const int* __restrict__ goff,
-                     unsigned* __restrict__ keys_out, unsigned* __restrict__ p1_out,
-                     unsigned* __restrict__ p2_out) {
-  constexpr int NW = kRadixNT / 32;
-  constexpr int WITEMS = kRadixTile / NW;  // 512 items per warp
-  constexpr int ROUNDS = WITEMS / 32;      // 16
-  __shared__ int s_wc[NW][kRadixDigits];
-  const int tile = blockIdx.x;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int d = threadIdx.x; d < NW * kRadixDigits; d += kRadixNT)
-    (&s_wc[0][0])[d] = 0;
+radix_hist_kernel(const unsigned* keys, const unsigned* hi, int n, int first, int bits, int lo_bits, int passes,
+                  unsigned* ghist) {
+  __shared__ unsigned s_h[kRadixMaxPasses * kRadixDigits];
+  constexpr int U = 8;
+  for (int i = threadIdx.x; i < passes * kRadixDigits; i += kRadixNT) s_h[i] = 0u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   __syncthreads();
-  const int wbase = tile * kRadixTile + w * WITEMS;
-  unsigned k[ROUNDS];
-  int rank[ROUNDS];
+  const unsigned mask = (1u << bits) - 1u;
+  const int lane = threadIdx.x & 31;
+  for (long long b = (long long)blockIdx.x * kRadixNT * U; b < n; b += (long long)gridDim.x * kRadixNT * U) {
+    unsigned k[U], h[U];
 #pragma unroll
-  for (int j = 0; j < ROUNDS; ++j) {
-    const int i = wbase + j * 32 + lane;
-    const bool valid = i < n;
-    k[j] = valid ? __ldg(keys_in + i) : 0xffffffffu;
-    const int d = valid ? (int)((k[j] >> shift) & 0xff) : -1 - lane;  // invalid items never match
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    int base = 0;
-    if (valid) base = s_wc[w][d];
-    __syncwarp();
-    if (valid && (peers & lanemask_lt()) == 0) s_wc[w][d] += __popc(peers);
-    __syncwarp();
-    rank[j] = base + __popc(peers & lanemask_lt());
+    for (int u = 0; u < U; ++u) {
+      const long long i = b + u * kRadixNT + threadIdx.x;
+      k[u] = i < n ? keys[i] : 0u;
+      h[u] = TWO && i < n ? hi[i] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool valid = b + u * kRadixNT + threadIdx.x < n;
+      const unsigned act = __ballot_sync(0xffffffffu, valid);
+      for (int p = 0; p < passes; ++p) {
+        const unsigned d = radix_digit<TWO>(k[u], h[u], lo_bits, first + p * bits, mask);
+        // a warp of one digit (sorted or constant keys) adds once
+        const unsigned d0 = __shfl_sync(0xffffffffu, d, 0);
+        if (__all_sync(0xffffffffu, !valid || d == d0)) {
+          if (lane == 0 && act) atomicAdd(&s_h[p * kRadixDigits + d0], (unsigned)__popc(act));
+        } else if (valid) {
+          atomicAdd(&s_h[p * kRadixDigits + d], 1u);
+        }
+      }
+    }
   }
   __syncthreads();
-  {
-    const int d = threadIdx.x;  // kRadixNT == kRadixDigits
-    int run = 0;
+  for (int i = threadIdx.x; i < passes * kRadixDigits; i += kRadixNT)
+    if (s_h[i]) atomicAdd(ghist + i, s_h[i]);
+}
+
+// One pass over one tile of kRadixNT * IPT items.  Each warp owns 32 * IPT
+// consecutive items and ranks them round by round: each lane sets its bit in
+// its digit's match word, the word then names the lanes of equal digit, and
+// warp-private digit counters carry the rank from round to round, so equal
+// digits keep their input order.
+template <int IPT, int NPAY, bool TWO, int BITS>
+__global__ void __launch_bounds__(kRadixNT, 4) radix_pass_kernel(RadixPass a) {
+  constexpr int TILE = kRadixNT * IPT;
+  __shared__ unsigned s_stage[TILE > (kRadixWarps << BITS) ? TILE : kRadixWarps << BITS];
+  __shared__ unsigned short s_wc[kRadixWarps][1 << BITS];
+  __shared__ unsigned char s_dig[TWO ? TILE : 4];
+  __shared__ int s_gb[1 << BITS];  // output position of local position 0 of the digit's run
+  __shared__ unsigned long long s_wtmp[kRadixWarps + 1];
+  __shared__ int s_tile;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const unsigned mask = (1u << a.bits) - 1u;
+  constexpr int ND = 1 << BITS;
+  for (int i = tid; i < kRadixWarps * ND / 2; i += kRadixNT) reinterpret_cast<unsigned*>(s_wc)[i] = 0u;
+  // the lanes that hold each digit, one word per digit and warp (in the stage,
+  // which is not in use yet)
+  unsigned* const s_match = s_stage + w * ND;
+  for (int i = tid; i < kRadixWarps * ND; i += kRadixNT) s_stage[i] = 0u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (tid == 0) s_tile = (int)atomicAdd(a.ticket, 1u);
+  __syncthreads();
+  const int tile = s_tile;
+  const size_t tbase = (size_t)tile * TILE;
+  const int valid = (int)min((long long)TILE, a.n - (long long)tbase);
+  const int li = w * 32 * IPT + lane;  // the thread's items: li + 32 j of the tile
+  const unsigned* kin = a.k_in + tbase;
+  unsigned k[IPT];
+  unsigned pos[IPT];  // digit << 16 | rank, then the local position
 #pragma unroll
-    for (int ww = 0; ww < NW; ++ww) {
-      const int t = s_wc[ww][d];
-      s_wc[ww][d] = run;
+  for (int j = 0; j < IPT; ++j) {
+    // items past the end take the largest digit: they are the tile's last
+    // items, so they end up behind every valid one
+    const bool in = li + j * 32 < valid;
+    k[j] = in ? kin[li + j * 32] : 0xffffffffu;
+    if (TWO) pos[j] = in ? a.p1_in[tbase + li + j * 32] : 0xffffffffu;
+  }
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const unsigned d = radix_digit<TWO>(k[j], TWO ? pos[j] : 0u, a.lo_bits, a.shift, mask);
+    atomicOr(&s_match[d], 1u << lane);
+    __syncwarp();
+    const unsigned peers = s_match[d];
+    const int base = s_wc[w][d];
+    __syncwarp();
+    if ((peers & lanemask_lt()) == 0u) {
+      s_wc[w][d] = (unsigned short)(base + __popc(peers));
+      s_match[d] = 0u;
+    }
+    pos[j] = (d << 16) | (unsigned)(base + __popc(peers & lanemask_lt()));
+    __syncwarp();
+  }
+  __syncthreads();
+  // thread d: the tile's count of digit d, published at once; then the digit
+  // offsets inside the tile (low word) and in the output (high word)
+  unsigned cnt = 0;
+  if (tid < ND) {
+#pragma unroll
+    for (int q = 0; q < kRadixWarps; ++q) cnt += s_wc[q][tid];
+    st_volatile_u64(a.status + (size_t)tile * ND + tid,
+                    lb_pack((unsigned)a.pass + 1u, tile == 0 ? 2u : 1u, cnt));
+  }
+  unsigned long long both = 0;
+  if (tid < ND) both = ((unsigned long long)a.ghist[tid] << 32) | cnt;
+  unsigned long long total;
+  const unsigned long long ex = block_exclusive_sum<kRadixNT>(both, s_wtmp, &total);
+  const unsigned off = (unsigned)ex;
+  if (tid < ND) {
+    unsigned run = off;
+#pragma unroll
+    for (int q = 0; q < kRadixWarps; ++q) {
+      const unsigned t = s_wc[q][tid];
+      s_wc[q][tid] = (unsigned short)run;
       run += t;
     }
   }
   __syncthreads();
+  // local positions; keys into digit order; the first payload's loads in
+  // flight during the look-back
 #pragma unroll
-  for (int j = 0; j < ROUNDS; ++j) {
-    const int i = wbase + j * 32 + lane;
-    if (i < n) {
-      const int d = (int)((k[j] >> shift) & 0xff);
-      const int dst = goff[d * ntiles + tile] + s_wc[w][d] + rank[j];
-      keys_out[dst] = k[j];
-      if (NPAY >= 1) p1_out[dst] = __ldg(p1_in + i);
-      if (NPAY >= 2) p2_out[dst] = __ldg(p2_in + i);
+  for (int j = 0; j < IPT; ++j) {
+    const unsigned d = pos[j] >> 16;
+    pos[j] = s_wc[w][d] + (pos[j] & 0xffffu);
+    s_stage[pos[j]] = k[j];
+    if (TWO) s_dig[pos[j]] = (unsigned char)d;
+  }
+  if (NPAY > 0) {
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) k[j] = li + j * 32 < valid ? a.p1_in[tbase + li + j * 32] : 0u;
+  }
+  int fail = 0;
+  if (tid < ND) {
+    // look-back, four predecessors per round trip
+    constexpr int LW = 4;
+    unsigned before = 0;
+    int j = tile - 1;
+    long long spins = 0;
+    bool done = tile == 0;
+    while (!done) {
+      unsigned long long word[LW];
+#pragma unroll
+      for (int q = 0; q < LW; ++q)
+        word[q] = j - q >= 0 ? ld_volatile_u64(a.status + (size_t)(j - q) * ND + tid)
+                             : lb_pack((unsigned)a.pass + 1u, 2u, 0u);
+      int used = 0;
+#pragma unroll
+      for (int q = 0; q < LW; ++q) {
+        if (done || used < q) continue;  // behind a prefix, or behind a tile not yet published
+        if ((unsigned)(word[q] >> 34) != (unsigned)a.pass + 1u) continue;
+        before += (unsigned)word[q];
+        ++used;
+        done = ((word[q] >> 32) & 3u) == 2u;
+      }
+      j -= used;
+      if (!done && used == 0) {
+        if (++spins > kSpinLimit) {
+          flag_error(a.err, kDevErrTimeout);
+          fail = 1;
+          break;
+        }
+        __nanosleep(20);
+      }
     }
+    if (tile > 0 && !fail)
+      st_volatile_u64(a.status + (size_t)tile * ND + tid, lb_pack((unsigned)a.pass + 1u, 2u, before + cnt));
+    s_gb[tid] = (int)((unsigned)(ex >> 32) + before - off);
+  }
+  if (__syncthreads_or(fail)) return;  // nothing is written after a wait that gave up
+  int dst[IPT];
+#pragma unroll
+  for (int r = 0; r < IPT; ++r) {
+    const int i = r * kRadixNT + tid;
+    const unsigned key = s_stage[i];
+    const unsigned d = TWO ? s_dig[i] : radix_digit<false>(key, 0u, 0, a.shift, mask);
+    dst[r] = s_gb[d] + i;
+    if (i < valid) a.k_out[dst[r]] = key;
+  }
+#pragma unroll
+  for (int p = 0; p < NPAY; ++p) {
+    unsigned* out = p == 0 ? a.p1_out : a.p2_out;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) s_stage[pos[j]] = k[j];
+    __syncthreads();
+    if (p + 1 < NPAY) {
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) k[j] = li + j * 32 < valid ? a.p2_in[tbase + li + j * 32] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < IPT; ++r)
+      if (r * kRadixNT + tid < valid) out[dst[r]] = s_stage[r * kRadixNT + tid];
   }
 }
 
@@ -152,42 +314,118 @@ int launch_scan_exclusive(const int* in, int* out, int n, int* total_out,
   return 0;
 }
 
-size_t radix_hist_ints(int n) {
-  const int ntiles = (n + kRadixTile - 1) / kRadixTile;
-  return (size_t)ntiles * kRadixDigits;
+// items per thread: tiles of 4,096 items while they fill the 592 resident CTAs
+// (4 per SM), of 2,048 or 1,024 below.  A run of equal digits is 32 items long
+// in a tile of 4,096 and 7-bit digits, and a short input needs the tiles more
+// (0.56M items, three passes: 31 us in tiles of 2,048, 36 us in tiles of 6,144)
+constexpr int kRadixFrom16 = 148 * 4 * 4096, kRadixFrom8 = 148 * 2048;
+static int radix_ipt(int n) { return n >= kRadixFrom16 ? 16 : n >= kRadixFrom8 ? 8 : 4; }
+
+static int radix_tiles(int n) {
+  const int tile = kRadixNT * radix_ipt(n);
+  return (int)(((long long)n + tile - 1) / tile);
 }
 
-int radix_sort_pairs(RadixBuffers& b, int n, int key_bits, ScanScratch& ls,
-                     int* err, cudaStream_t st) {
+// scratch of a sort: look-back words, digit counts, tickets
+static size_t radix_status_bytes(int ntiles) { return (size_t)ntiles * kRadixDigits * 8; }
+
+// enough for every sort of at most n items: the tile count is not monotonic
+// where the tile grows
+size_t radix_scratch_bytes(int n) {
+  int t = radix_tiles(n);
+  if (n >= kRadixFrom8) t = std::max(t, radix_tiles(kRadixFrom8 - 1));
+  if (n >= kRadixFrom16) t = std::max(t, radix_tiles(kRadixFrom16 - 1));
+  return radix_status_bytes(t) + 4 * (size_t)kRadixMaxPasses * (kRadixDigits + 1);
+}
+
+template <int IPT, int BITS>
+static cudaError_t launch_radix_pass(const RadixPass& a, int npay, bool two, cudaStream_t st) {
+  const dim3 grid((unsigned)a.ntiles), block(kRadixNT);
+  if (two && npay == 2) return launch_pdl(radix_pass_kernel<IPT, 2, true, BITS>, grid, block, 0, st, a);
+  if (two) return launch_pdl(radix_pass_kernel<IPT, 1, true, BITS>, grid, block, 0, st, a);
+  if (npay == 2) return launch_pdl(radix_pass_kernel<IPT, 2, false, BITS>, grid, block, 0, st, a);
+  if (npay == 1) return launch_pdl(radix_pass_kernel<IPT, 1, false, BITS>, grid, block, 0, st, a);
+  return launch_pdl(radix_pass_kernel<IPT, 0, false, BITS>, grid, block, 0, st, a);
+}
+
+template <int IPT>
+static cudaError_t launch_radix_pass(const RadixPass& a, int npay, bool two, cudaStream_t st) {
+  return a.bits <= 7 ? launch_radix_pass<IPT, 7>(a, npay, two, st) : launch_radix_pass<IPT, 8>(a, npay, two, st);
+}
+
+int radix_sort_passes(int first_bit, int end_bit) {
+  return std::max(1, (end_bit - first_bit + 7) / 8);
+}
+
+int radix_sort_pairs(RadixBuffers& b, int n, int key_bits, int* err, cudaStream_t st) {
   b.result_in_alt = false;
-  if (n <= 1) return 0;
-  const int ntiles = (n + kRadixTile - 1) / kRadixTile;
-  const int hn = ntiles * kRadixDigits;
-  int passes = (key_bits + 7) / 8;
-  if (passes < 1) passes = 1;
-  unsigned *kin = b.keys, *kout = b.keys_alt;
-  unsigned *p1in = b.p1, *p1out = b.p1_alt;
-  unsigned *p2in = b.p2, *p2out = b.p2_alt;
-  for (int p = 0; p < passes; ++p) {
-    const int shift = p * 8;
-    note_launch(2);  // histogram + scatter (the scan counts itself)
-    radix_hist_kernel<<<ntiles, kRadixNT, 0, st>>>(kin, n, shift, ntiles, b.hist);
-    if (launch_scan_exclusive(b.hist, b.hist_off, hn, nullptr, ls, err, st)) return -1;
-    if (b.p2)
-      radix_scatter_kernel<2><<<ntiles, kRadixNT, 0, st>>>(kin, p1in, p2in, n, shift, ntiles,
-                                                          b.hist_off, kout, p1out, p2out);
-    else if (b.p1)
-      radix_scatter_kernel<1><<<ntiles, kRadixNT, 0, st>>>(kin, p1in, p2in, n, shift, ntiles,
-                                                          b.hist_off, kout, p1out, p2out);
-    else
-      radix_scatter_kernel<0><<<ntiles, kRadixNT, 0, st>>>(kin, p1in, p2in, n, shift, ntiles,
-                                                          b.hist_off, kout, p1out, p2out);
-    unsigned* t;
-    t = kin; kin = kout; kout = t;
-    t = p1in; p1in = p1out; p1out = t;
-    t = p2in; p2in = p2out; p2out = t;
-    b.result_in_alt = !b.result_in_alt;
+  const bool two = b.lo_bits > 0;
+  const int passes = radix_sort_passes(b.first_bit, key_bits);
+  if (passes > kRadixMaxPasses || (two && !b.p1)) return -1;
+  if (n <= 0 || (n == 1 && !b.src_keys)) return 0;
+  const int bits = std::max(1, (key_bits - b.first_bit + passes - 1) / passes);
+  const int npay = b.p2 ? 2 : b.p1 ? 1 : 0;
+  const int ipt = radix_ipt(n), ntiles = radix_tiles(n);
+  unsigned long long* status = reinterpret_cast<unsigned long long*>(b.scratch);
+  unsigned* ghist = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(b.scratch) + radix_status_bytes(ntiles));
+  unsigned* ticket = ghist + kRadixMaxPasses * kRadixDigits;
+  if (cudaMemsetAsync(b.scratch, 0, radix_status_bytes(ntiles) + 4 * (size_t)kRadixMaxPasses * (kRadixDigits + 1),
+                      st) != cudaSuccess)
+    return -1;
+  const unsigned *kin = b.src_keys ? b.src_keys : b.keys, *p1in = b.src_keys ? b.src_p1 : b.p1,
+                 *p2in = b.src_keys ? b.src_p2 : b.p2;
+  unsigned *kout = b.keys_alt, *p1out = b.p1_alt, *p2out = b.p2_alt;
+  note_launch(1 + passes);
+  const int hgrid = (int)std::min<long long>(((long long)n + kRadixNT * 8 - 1) / (kRadixNT * 8), 148 * 4);
+  cudaError_t e = two ? launch_pdl(radix_hist_kernel<true>, dim3(hgrid), dim3(kRadixNT), 0, st, kin, p1in, n,
+                                   b.first_bit, bits, b.lo_bits, passes, ghist)
+                      : launch_pdl(radix_hist_kernel<false>, dim3(hgrid), dim3(kRadixNT), 0, st, kin,
+                                   (const unsigned*)nullptr, n, b.first_bit, bits, 0, passes, ghist);
+  for (int p = 0; p < passes && e == cudaSuccess; ++p) {
+    const RadixPass a{kin, p1in, p2in, kout, p1out, p2out, n, b.first_bit + p * bits, bits, b.lo_bits, p, ntiles,
+                      status, ticket + p, ghist + p * kRadixDigits, err};
+    e = ipt == 16 ? launch_radix_pass<16>(a, npay, two, st)
+        : ipt == 8 ? launch_radix_pass<8>(a, npay, two, st)
+                   : launch_radix_pass<4>(a, npay, two, st);
+    const bool alt = (p & 1) == 0;  // this pass wrote the alternate set
+    kin = alt ? b.keys_alt : b.keys;
+    p1in = alt ? b.p1_alt : b.p1;
+    p2in = alt ? b.p2_alt : b.p2;
+    kout = alt ? b.keys : b.keys_alt;
+    p1out = alt ? b.p1 : b.p1_alt;
+    p2out = alt ? b.p2 : b.p2_alt;
+    b.result_in_alt = alt;
   }
+  return e == cudaSuccess ? 0 : -1;
+}
+
+// ptr[j] = first position whose key is >= j, j in [0, extent], of `cnt` sorted
+// keys (keys past the extent end the last range): position i owns the entries
+// after its predecessor's key up to its own key (extent at i = cnt), so every
+// entry is written once, empty ranges included.  Four positions per thread in
+// flight.
+__global__ void __launch_bounds__(256)
+sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int* __restrict__ ptr) {
+  constexpr int U = 4;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b <= cnt; b += step * U) {
+    int lo[U], hi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = b + u * step;
+      lo[u] = i == 0 || i > cnt ? 0 : (int)min(__ldg(key + i - 1), (unsigned)extent) + 1;
+      hi[u] = i > cnt ? -1 : i == cnt ? extent : (int)min(__ldg(key + i), (unsigned)extent);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      for (int j = lo[u]; j <= hi[u]; ++j) ptr[j] = (int)(b + u * step);
+  }
+}
+
+int launch_sorted_bounds(int cnt, const unsigned* key, int extent, int* ptr, cudaStream_t st) {
+  note_launch();
+  const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)cnt + 1 + 1023) / 1024, 148LL * 8));
+  sorted_bounds_kernel<<<grid, 256, 0, st>>>(cnt, key, extent, ptr);
   return 0;
 }
 

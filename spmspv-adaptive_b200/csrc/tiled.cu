@@ -695,9 +695,9 @@ extern "C" int spmx_tiled_preprocess(spmx_handle_t h, int rb_rows, int win, int 
   }
   const size_t b = 4 * (size_t)std::max(nnz, 1);
   unsigned *k0 = nullptr, *k1 = nullptr, *p0 = nullptr, *p1 = nullptr, *v0 = nullptr, *v1 = nullptr;
-  int *hist = nullptr, *hoff = nullptr, *tptr = nullptr, *d_wsp = nullptr;
+  void* radix = nullptr;
+  int *tptr = nullptr, *d_wsp = nullptr;
   long long* d_pad = nullptr;
-  const size_t hn = radix_hist_ints(std::max(nnz, 1));
   int rc = SPMX_SUCCESS;
   rc = rc ? rc : dalloc((void**)&k0, b, "tiled keys");
   rc = rc ? rc : dalloc((void**)&k1, b, "tiled keys alt");
@@ -705,8 +705,7 @@ extern "C" int spmx_tiled_preprocess(spmx_handle_t h, int rb_rows, int win, int 
   rc = rc ? rc : dalloc((void**)&p1, b, "tiled packed alt");
   rc = rc ? rc : dalloc((void**)&v0, b, "tiled vals");
   rc = rc ? rc : dalloc((void**)&v1, b, "tiled vals alt");
-  rc = rc ? rc : dalloc((void**)&hist, 4 * hn, "tiled hist");
-  rc = rc ? rc : dalloc((void**)&hoff, 4 * hn, "tiled hist off");
+  rc = rc ? rc : dalloc(&radix, radix_scratch_bytes(std::max(nnz, 1)), "tiled radix scratch");
   rc = rc ? rc : dalloc((void**)&tptr, 4 * (size_t)(ntiles + 2), "tiled pointers");
   rc = rc ? rc : dalloc((void**)&t->rb_row, 4 * (size_t)(nrb + 1), "tiled row blocks");
   rc = rc ? rc : dalloc((void**)&d_wsp, 4 * wsp.size(), "tiled warp splits");
@@ -724,8 +723,8 @@ extern "C" int spmx_tiled_preprocess(spmx_handle_t h, int rb_rows, int win, int 
     tile_keys_kernel<<<(unsigned)(((long long)m * 32 + 255) / 256), 256, 0, st>>>(
         m, n, h->rowptr, h->col, h->val, t->rb_row, nrb, win, nwin, (unsigned)ntiles, k0, p0, (float*)v0,
         h->d_err);
-    RadixBuffers rbuf{k0, k1, p0, p1, v0, v1, hist, hoff, false};
-    if (radix_sort_pairs(rbuf, nnz, std::max(1, log2_ceil(ntiles + 1)), h->ls, h->d_err, st))
+    RadixBuffers rbuf{k0, k1, p0, p1, v0, v1, radix};
+    if (radix_sort_pairs(rbuf, nnz, std::max(1, log2_ceil(ntiles + 1)), h->d_err, st))
       rc = set_error(SPMX_ERR_INVALID_VALUE, "tiled SpMV: sort capacity");
     if (!rc) {
       skey = rbuf.result_in_alt ? k1 : k0;
@@ -825,7 +824,7 @@ extern "C" int spmx_tiled_preprocess(spmx_handle_t h, int rb_rows, int win, int 
   se = cudaStreamSynchronize(st);
   if (!rc && se != cudaSuccess) rc = set_error(SPMX_ERR_CUDA, cudaGetErrorString(se));
   dfree(k0); dfree(k1); dfree(p0); dfree(p1); dfree(v0); dfree(v1);
-  dfree(hist); dfree(hoff); dfree(tptr); dfree(d_wsp); dfree(d_pad);
+  dfree(radix); dfree(tptr); dfree(d_wsp); dfree(d_pad);
   if (rc) {
     spmx_tiled_postprocess(h);
     return rc;
