@@ -44,6 +44,66 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
+// One pool per device.  cudaMalloc and cudaFree of a sort's buffers (470 MB for
+// the transpose of 16.8M nonzeros) took about 10 ms of host time around 2 ms of
+// kernels; memory that the pool still holds is handed out without mapping it
+// again, ordered across streams and threads by the runtime.
+namespace {
+constexpr int kMaxDev = 64;
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  int handles = 0;
+};
+std::mutex g_pool_mu;
+ScratchPool g_pool[kMaxDev];
+
+void pool_enter(int dev) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (dev >= 0 && dev < kMaxDev) ++g_pool[dev].handles;
+}
+
+void pool_leave(int dev) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (dev < 0 || dev >= kMaxDev || --g_pool[dev].handles > 0) return;
+  if (g_pool[dev].pool && cudaMemPoolTrimTo(g_pool[dev].pool, 0) != cudaSuccess) cudaGetLastError();
+}
+}  // namespace
+
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st, const char* what) {
+  *p = nullptr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  cudaMemPool_t pool = nullptr;
+  if (e == cudaSuccess && (dev < 0 || dev >= kMaxDev)) e = cudaErrorInvalidDevice;
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pool[dev].pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      e = cudaMemPoolCreate(&g_pool[dev].pool, &props);
+      if (e == cudaSuccess) {
+        unsigned long long keep = kScratchKeep;
+        e = cudaMemPoolSetAttribute(g_pool[dev].pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      } else {
+        g_pool[dev].pool = nullptr;
+      }
+    }
+    pool = g_pool[dev].pool;
+  }
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, st);
+  if (e == cudaSuccess) return SPMX_SUCCESS;
+  cudaGetLastError();
+  *p = nullptr;
+  return set_error(SPMX_ERR_ALLOC, std::string("scratch(") + what + ", " + std::to_string(bytes) + " B): " +
+                                       cudaGetErrorString(e));
+}
+
+void scratch_free(void* p, cudaStream_t st) {
+  if (p && cudaFreeAsync(p, st) != cudaSuccess) cudaGetLastError();
+}
+
 cudaError_t kernel_smem_limit(const void* kernel, size_t bytes) {
   static std::mutex mu;
   static std::vector<std::pair<std::pair<const void*, int>, size_t>> set;  // (kernel, device) -> bytes
@@ -154,6 +214,7 @@ extern "C" int spmx_create(int m, int n, int nnz, spmx_handle_t* out) {
   h->nnz = nnz;
   h->num_ints = (n + 31) / 32;
   cudaGetDevice(&h->device);
+  pool_enter(h->device);
   cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
   int rc = SPMX_SUCCESS;
   rc = rc ? rc : dalloc((void**)&h->d_counts, sizeof(int) * kCntTotal, "counts");
@@ -240,6 +301,7 @@ extern "C" int spmx_destroy(spmx_handle_t h) {
   for (void* p : h->batch_buf) dfree(p);
   dfree(h->batch_radix); dfree(h->batch_invptr); dfree(h->batch_rec);
   dfree(h->batch_chunk); dfree(h->batch_ctr);
+  pool_leave(h->device);
   delete h;
   return SPMX_SUCCESS;
 }
@@ -340,61 +402,49 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
   SPMX_CHECK_HANDLE(h);
   if (!h->has_csr) return set_error(SPMX_ERR_NOT_READY, "ToCSC needs the CSR input");
   const int m = h->m, n = h->n, nnz = h->nnz;
-  dfree(h->own_colptr); dfree(h->own_row); dfree(h->own_cval);
-  h->own_colptr = nullptr; h->own_row = nullptr; h->own_cval = nullptr;
-  SPMX_TRY(dalloc((void**)&h->own_colptr, 4 * (size_t)(n + 1), "csc colptr"));
-  SPMX_TRY(dalloc((void**)&h->own_row, 4 * (size_t)std::max(nnz, 1), "csc row"));
-  if (h->val) SPMX_TRY(dalloc((void**)&h->own_cval, 4 * (size_t)std::max(nnz, 1), "csc val"));
+  // the handle's sizes never change, so a second ToCSC writes into the arrays
+  // of the first; a caller's work on another stream may still read them
+  if (h->own_colptr) SPMX_CUDA(cudaDeviceSynchronize());
+  if (!h->val && h->own_cval) {
+    dfree(h->own_cval);
+    h->own_cval = nullptr;
+  }
+  if (h->csc_colptr == h->own_colptr) h->has_csc = false;
+  if (!h->own_colptr) SPMX_TRY(dalloc((void**)&h->own_colptr, 4 * (size_t)(n + 1), "csc colptr"));
+  if (!h->own_row) SPMX_TRY(dalloc((void**)&h->own_row, 4 * (size_t)std::max(nnz, 1), "csc row"));
+  if (h->val && !h->own_cval) SPMX_TRY(dalloc((void**)&h->own_cval, 4 * (size_t)std::max(nnz, 1), "csc val"));
   cudaStream_t st = h->stream;
-  // column counts -> colptr
-  int* cnt = nullptr;
-  SPMX_TRY(dalloc((void**)&cnt, 4 * (size_t)std::max(n, 1), "col counts"));
-  SPMX_CUDA(cudaMemsetAsync(cnt, 0, 4 * (size_t)std::max(n, 1), st));
-  launch_count_keys(nnz, n, h->col, cnt, h->d_err, st);
-  if (n > 0) {
-    if (launch_scan_exclusive(cnt, h->own_colptr, n, h->own_colptr + n, h->ls, h->d_err, st)) {
-      dfree(cnt);
-      return set_error(SPMX_ERR_INVALID_VALUE, "scan capacity");
-    }
-  } else {
-    SPMX_CUDA(cudaMemsetAsync(h->own_colptr, 0, 4, st));
-  }
+  int rc = SPMX_SUCCESS;
   if (nnz > 0) {
-    // stable sort of the row-major COO by column
-    unsigned *k0 = nullptr, *k1 = nullptr, *r0 = nullptr, *r1 = nullptr, *v0 = nullptr, *v1 = nullptr;
-    void* radix = nullptr;
-    const size_t b = 4 * (size_t)nnz;
-    int rc = SPMX_SUCCESS;
-    rc = rc ? rc : dalloc((void**)&k0, b, "t keys");
-    rc = rc ? rc : dalloc((void**)&k1, b, "t keys alt");
-    rc = rc ? rc : dalloc((void**)&r0, b, "t rows");
-    rc = rc ? rc : dalloc((void**)&r1, b, "t rows alt");
-    if (h->val) {
-      rc = rc ? rc : dalloc((void**)&v0, b, "t vals");
-      rc = rc ? rc : dalloc((void**)&v1, b, "t vals alt");
-    }
-    rc = rc ? rc : dalloc(&radix, radix_scratch_bytes(nnz), "t radix scratch");
-    if (!rc) {
-      cudaMemcpyAsync(k0, h->col, b, cudaMemcpyDeviceToDevice, st);
-      if (h->val) cudaMemcpyAsync(v0, h->val, b, cudaMemcpyDeviceToDevice, st);
-      launch_expand_rows(m, h->rowptr, r0, st);
-      RadixBuffers rb{k0, k1, r0, r1, v0, v1, radix};
-      if (radix_sort_pairs(rb, nnz, ceil_log2(std::max(n, 2)), h->d_err, st))
-        rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
-      if (!rc) {
-        unsigned* rr = rb.result_in_alt ? r1 : r0;
-        unsigned* vv = rb.result_in_alt ? v1 : v0;
-        cudaMemcpyAsync(h->own_row, rr, b, cudaMemcpyDeviceToDevice, st);
-        if (h->val) cudaMemcpyAsync(h->own_cval, vv, b, cudaMemcpyDeviceToDevice, st);
-      }
-    }
-    cudaError_t se = cudaStreamSynchronize(st);
-    dfree(k0); dfree(k1); dfree(r0); dfree(r1); dfree(v0); dfree(v1); dfree(radix);
-    if (rc) { dfree(cnt); return rc; }
-    if (se != cudaSuccess) { dfree(cnt); return set_error(SPMX_ERR_CUDA, cudaGetErrorString(se)); }
+    // stable sort of the row-major COO by column; a column out of range gets
+    // the key n (behind every column), so the keys need the bits of n itself
+    const int bits = ceil_log2((long long)n + 1);
+    const bool odd = radix_sort_passes(0, bits) & 1;  // the last pass writes the alternate set
+    const size_t b = (4 * (size_t)nnz + 255) & ~(size_t)255;
+    char* tmp = nullptr;
+    SPMX_TRY(scratch_alloc((void**)&tmp, b * (h->val ? 4 : 3) + radix_scratch_bytes(nnz), st, "transpose"));
+    unsigned *k0 = (unsigned*)tmp, *k1 = (unsigned*)(tmp + b), *r = (unsigned*)(tmp + 2 * b);
+    unsigned* v = h->val ? (unsigned*)(tmp + 3 * b) : nullptr;
+    RadixBuffers rb{};
+    rb.keys = k0;
+    rb.keys_alt = k1;
+    rb.p1 = odd ? r : (unsigned*)h->own_row;
+    rb.p1_alt = odd ? (unsigned*)h->own_row : r;
+    rb.p2 = odd ? v : (unsigned*)h->own_cval;
+    rb.p2_alt = odd ? (unsigned*)h->own_cval : v;
+    rb.scratch = tmp + b * (h->val ? 4 : 3);
+    rb.src_keys = k0;
+    rb.src_p1 = rb.p1;
+    rb.src_p2 = (const unsigned*)h->val;
+    launch_expand_rows(m, n, nnz, h->rowptr, h->col, rb.p1, k0, h->d_err, st);
+    if (radix_sort_pairs(rb, nnz, bits, h->d_err, st)) rc = set_error(SPMX_ERR_CUDA, "ToCSC sort launch");
+    if (!rc) launch_sorted_bounds(nnz, rb.result_in_alt ? k1 : k0, n, h->own_colptr, st);
+    scratch_free(tmp, st);
+  } else {
+    SPMX_CUDA(cudaMemsetAsync(h->own_colptr, 0, 4 * (size_t)(n + 1), st));
   }
+  if (rc) return rc;
   SPMX_CUDA(cudaStreamSynchronize(st));
-  dfree(cnt);
   h->csc_colptr = h->own_colptr;
   h->csc_row = h->own_row;
   h->csc_val = h->own_cval;

@@ -167,6 +167,12 @@ namespace spmx {
 int set_error(int code, const std::string& msg);
 int dalloc(void** p, size_t bytes, const char* what);
 void dfree(void* p);
+// Temporaries of one call, stream-ordered, from a memory pool of the handle's
+// device that keeps at most kScratchKeep bytes between calls and is emptied
+// when the device's last handle is destroyed.
+constexpr size_t kScratchKeep = (size_t)1 << 30;
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st, const char* what);
+void scratch_free(void* p, cudaStream_t st);
 // A kernel's dynamic shared-memory limit is a property of the function on a
 // device, shared by every handle: set it to `bytes` unless it already is
 // (cached per function and device), right before a launch that needs it.

@@ -13,9 +13,8 @@ int launch_gini_sum(int maxdeg, const int* hist, const int* pref,
 int launch_vec_features(int x_nnz, int n, const int* x_key, const int* colptr,
                         unsigned long long* out64, int* out32, int* err,
                         cudaStream_t st);
-int launch_expand_rows(int m, const int* rowptr, unsigned* rows, cudaStream_t st);
-int launch_count_keys(int nnz, int n, const int* keys, int* cnt, int* err,
-                      cudaStream_t st);
+int launch_expand_rows(int m, int n, int nnz, const int* rowptr, const int* col, unsigned* rows, unsigned* keys,
+                       int* err, cudaStream_t st);
 int launch_set_int(int* p, int v, cudaStream_t st);
 
 }  // namespace spmx

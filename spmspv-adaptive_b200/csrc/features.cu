@@ -103,24 +103,82 @@ __global__ void vec_features_kernel(int x_nnz, int n, const int* __restrict__ x_
 }
 
 // ---- utility kernels -------------------------------------------------------
-__global__ void expand_rows_kernel(int m, const int* __restrict__ rowptr,
-                                   unsigned* __restrict__ rows) {
-  // one warp per row
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= m) return;
-  const int r = (int)gw;
-  const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
-  for (int k = a + lane; k < b; k += 32) rows[k] = (unsigned)r;
-}
-
-__global__ void count_keys_kernel(int nnz, int n, const int* __restrict__ keys,
-                                  int* __restrict__ cnt, int* err) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
-       i += gridDim.x * blockDim.x) {
-    const int k = __ldg(keys + i);
-    if ((unsigned)k < (unsigned)n) atomicAdd(cnt + k, 1);
-    else flag_error(err, kDevErrOob);
+// The row of every nonzero of a CSR, and its column as a sort key (n for a
+// column out of range).  Each CTA owns K consecutive nonzeros: the rows that
+// start among them leave marks in shared memory, and a max-scan of the marks
+// gives every position its row, so all traffic is coalesced whatever the row
+// lengths.  16.8M nonzeros of Zipf rows: 45 us for 201 MB; one warp
+// per row took 107 us for the rows alone.
+template <int NT, int VT>
+__global__ void __launch_bounds__(NT)
+expand_rows_kernel(int m, int n, int nnz, const int* __restrict__ rowptr, const int* __restrict__ col,
+                   unsigned* __restrict__ rows, unsigned* __restrict__ keys, int* err) {
+  constexpr int K = NT * VT;
+  static_assert(VT % 4 == 0, "vector access to the marks");
+  __shared__ __align__(16) int s_mark[K];
+  __shared__ int s_wtmp[NT / 32 + 1];
+  __shared__ int s_lo[2];
+  const int tid = threadIdx.x;
+  const long long s = (long long)blockIdx.x * K;
+  const int cnt = (int)min((long long)K, nnz - s);
+  unsigned key[VT];
+#pragma unroll
+  for (int j = 0; j < VT; ++j) {
+    const int q = j * NT + tid;
+    key[j] = q < cnt ? (unsigned)__ldg(col + s + q) : 0u;
+  }
+  for (int q = tid; q < K / 4; q += NT) reinterpret_cast<int4*>(s_mark)[q] = make_int4(-1, -1, -1, -1);
+  // warps 0 and 1: the first row that starts at or after the chunk's first
+  // position, and after its last, 32 probes per step
+  if (tid < 64) {
+    const long long target = s + (tid >= 32 ? cnt : 0);
+    int l = 0, r = m;  // the answer is in [l, r]
+    while (l < r) {
+      const int span = r - l, q = l + (int)(((long long)span * (tid & 31)) >> 5);
+      const unsigned below = __ballot_sync(0xffffffffu, __ldg(rowptr + q) < target);
+      const int c = __popc(below);  // the probes are sorted: the first c are below
+      const int nl = c ? l + (int)(((long long)span * (c - 1)) >> 5) + 1 : l;
+      r = c < 32 ? l + (int)(((long long)span * c) >> 5) : r;
+      l = nl;
+    }
+    if ((tid & 31) == 0) s_lo[tid >> 5] = l;
+  }
+  __syncthreads();
+  const int lo = s_lo[0], hi = s_lo[1];
+  for (int r = lo + tid; r < hi; r += NT) {
+    const long long p = __ldg(rowptr + r) - s;
+    if (p >= 0 && p < cnt) atomicMax(&s_mark[p], r);  // empty rows share a position with the row that owns it
+  }
+  __syncthreads();
+  int v[VT];
+  int run = tid == 0 ? lo - 1 : -1;  // the row open at the chunk's start
+#pragma unroll
+  for (int q = 0; q < VT / 4; ++q) {
+    const int4 t = reinterpret_cast<const int4*>(s_mark)[tid * (VT / 4) + q];
+    run = max(run, t.x); v[4 * q] = run;
+    run = max(run, t.y); v[4 * q + 1] = run;
+    run = max(run, t.z); v[4 * q + 2] = run;
+    run = max(run, t.w); v[4 * q + 3] = run;
+  }
+  // inclusive max over the threads, then the previous thread's value
+  const int inc = block_inclusive_max<NT>(run, s_wtmp);
+  int carry = __shfl_up_sync(0xffffffffu, inc, 1);
+  if ((tid & 31) == 31) s_wtmp[tid >> 5] = inc;
+  __syncthreads();
+  if ((tid & 31) == 0) carry = tid ? s_wtmp[(tid >> 5) - 1] : -1;
+#pragma unroll
+  for (int q = 0; q < VT / 4; ++q)
+    reinterpret_cast<int4*>(s_mark)[tid * (VT / 4) + q] =
+        make_int4(max(v[4 * q], carry), max(v[4 * q + 1], carry), max(v[4 * q + 2], carry), max(v[4 * q + 3], carry));
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < VT; ++j) {
+    const int q = j * NT + tid;
+    if (q < cnt) {
+      rows[s + q] = (unsigned)s_mark[q];
+      if (key[j] >= (unsigned)n) flag_error(err, kDevErrOob);
+      keys[s + q] = min(key[j], (unsigned)n);
+    }
   }
 }
 
@@ -167,19 +225,13 @@ int launch_vec_features(int x_nnz, int n, const int* x_key, const int* colptr,
   return 0;
 }
 
-int launch_expand_rows(int m, const int* rowptr, unsigned* rows, cudaStream_t st) {
-  if (m <= 0) return 0;
-  const long long threads = (long long)m * 32;
+int launch_expand_rows(int m, int n, int nnz, const int* rowptr, const int* col, unsigned* rows, unsigned* keys,
+                       int* err, cudaStream_t st) {
+  if (m <= 0 || nnz <= 0) return 0;
+  constexpr int NT = 256, VT = 8;
   note_launch();
-  expand_rows_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(m, rowptr, rows);
-  return 0;
-}
-
-int launch_count_keys(int nnz, int n, const int* keys, int* cnt, int* err,
-                      cudaStream_t st) {
-  if (nnz <= 0) return 0;
-  note_launch();
-  count_keys_kernel<<<grid_for(nnz, 256, 148 * 16), 256, 0, st>>>(nnz, n, keys, cnt, err);
+  expand_rows_kernel<NT, VT><<<(unsigned)(((long long)nnz + NT * VT - 1) / (NT * VT)), NT, 0, st>>>(
+      m, n, nnz, rowptr, col, rows, keys, err);
   return 0;
 }
 

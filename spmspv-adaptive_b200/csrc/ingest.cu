@@ -6,12 +6,12 @@
 // 1. coo_check_kernel: range check of every index, and whether the entries
 //    are already in (row, col) order, or at least in non-decreasing column
 //    order (a column-major file such as a SuiteSparse export).
-// 2. stable LSD radix sort (sort.cu): by column, skipped when the columns are
-//    already non-decreasing, then by row, both skipped when the input is
+// 2. one stable LSD radix sort (sort.cu) by (row, col), over the row bits alone
+//    when the columns are already non-decreasing, none when the input is
 //    already in (row, col) order.  Stability keeps duplicates in input order.
-// 3. coo_rowptr_kernel: position i writes the row pointers of the rows that
-//    start there (rows[i-1]+1 .. rows[i]); every rowptr entry is written
-//    once, empty rows included, with no atomics and no search.
+// 3. sorted_bounds_kernel (sort.cu): the row pointers from the sorted rows;
+//    every entry is written once, empty rows included, with no atomics and no
+//    search.
 #include <algorithm>
 
 #include "common.cuh"
@@ -27,14 +27,23 @@ __global__ void __launch_bounds__(kIngestNT)
 coo_check_kernel(int nnz, int m, int n, const int* __restrict__ row,
                  const int* __restrict__ col, int* __restrict__ flags) {
   int oob = 0, unsorted = 0, col_desc = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nnz;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int r = __ldg(row + i), c = __ldg(col + i);
-    oob |= (unsigned)r >= (unsigned)m || (unsigned)c >= (unsigned)n;
-    if (i > 0) {
-      const int rp = __ldg(row + i - 1), cp = __ldg(col + i - 1);
-      unsorted |= rp > r || (rp == r && cp > c);
-      col_desc |= cp > c;
+  constexpr int U = 4;  // entries in flight per thread
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < nnz; b += U * step) {
+    int r[U], c[U], rp[U], cp[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = min(b + u * step, (long long)nnz - 1), p = max(i - 1, 0LL);
+      r[u] = __ldg(row + i);
+      c[u] = __ldg(col + i);
+      rp[u] = __ldg(row + p);
+      cp[u] = __ldg(col + p);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      oob |= (unsigned)r[u] >= (unsigned)m || (unsigned)c[u] >= (unsigned)n;
+      unsorted |= rp[u] > r[u] || (rp[u] == r[u] && cp[u] > c[u]);
+      col_desc |= cp[u] > c[u];
     }
   }
   oob = __syncthreads_or(oob);
@@ -44,16 +53,6 @@ coo_check_kernel(int nnz, int m, int n, const int* __restrict__ row,
     if (oob) atomicOr(flags + 0, 1);
     if (unsorted) atomicOr(flags + 1, 1);
     if (col_desc) atomicOr(flags + 2, 1);
-  }
-}
-
-__global__ void __launch_bounds__(kIngestNT)
-coo_rowptr_kernel(int nnz, int m, const int* __restrict__ rows, int* __restrict__ rowptr) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= nnz;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int lo = i == 0 ? 0 : __ldg(rows + i - 1) + 1;
-    const int hi = i == nnz ? m : __ldg(rows + i);
-    for (int r = lo; r <= hi; ++r) rowptr[r] = (int)i;
   }
 }
 
@@ -82,106 +81,74 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   cudaStream_t st = h->stream;
   const size_t b = 4 * (size_t)std::max(nnz, 1);
 
-  // 1. range and order check (synchronous: the result picks the sort passes)
-  int* flags = nullptr;
-  SPMX_TRY(dalloc((void**)&flags, 4 * sizeof(int), "coo flags"));
-  int oob = 0, unsorted = 0, col_desc = 0;
-  cudaError_t ce = cudaMemsetAsync(flags, 0, 4 * sizeof(int), st);
-  if (ce == cudaSuccess && nnz > 0) {
-    note_launch();
-    coo_check_kernel<<<ingest_grid(nnz), kIngestNT, 0, st>>>(nnz, m, n, row, col, flags);
-    ce = cudaGetLastError();
-  }
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(h->h_pinned, flags, 3 * sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  dfree(flags);
-  if (ce != cudaSuccess) return set_error(SPMX_ERR_CUDA, std::string("coo check: ") + cudaGetErrorString(ce));
+  // 1. range and order check (synchronous: the result picks the sort passes);
+  // the feature accumulators hold the three flags
+  SPMX_CUDA(cudaMemsetAsync(h->d_iacc, 0, 4 * sizeof(int), st));
   if (nnz > 0) {
-    oob = h->h_pinned[0];
-    unsorted = h->h_pinned[1];
-    col_desc = h->h_pinned[2];
+    note_launch();
+    coo_check_kernel<<<ingest_grid(nnz), kIngestNT, 0, st>>>(nnz, m, n, row, col, h->d_iacc);
+    SPMX_TRY(launch_ok("coo check"));
   }
-  if (oob) return set_error(SPMX_ERR_INVALID_VALUE, "COO index out of range");
+  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned, h->d_iacc, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  SPMX_CUDA(cudaStreamSynchronize(st));
+  const int unsorted = h->h_pinned[1], col_desc = h->h_pinned[2];
+  if (h->h_pinned[0]) return set_error(SPMX_ERR_INVALID_VALUE, "COO index out of range");
 
-  // 2. the new CSR (swapped in only on success).  The radix passes alternate
-  // between two buffer sets; the pass count is known here, so the set the
-  // last pass writes is the new CSR's column / value arrays themselves.  All
-  // other scratch is one allocation.
-  int *nrp = nullptr, *ncol = nullptr;
-  float* nval = nullptr;
-  int rc = SPMX_SUCCESS;
-  rc = rc ? rc : dalloc((void**)&nrp, 4 * ((size_t)m + 1), "csr rowptr");
-  rc = rc ? rc : dalloc((void**)&ncol, b, "csr col");
-  if (val) rc = rc ? rc : dalloc((void**)&nval, b, "csr val");
+  // 2. the new CSR, in the handle's own arrays (its sizes never change); all
+  // memory is there before the first of them is written.  The radix passes
+  // alternate between two buffer sets; the pass count is known here, so the
+  // set the last pass writes is the column / value arrays themselves.
   char* scratch = nullptr;
-  const int* rows_sorted = row;
-  const void* cols_sorted = col;
-  const void* vals_sorted = val;
+  const size_t al = (b + 255) & ~(size_t)255;
+  if (unsorted)
+    SPMX_TRY(scratch_alloc((void**)&scratch, al * (val ? 4 : 3) + radix_scratch_bytes(nnz), st, "coo sort"));
+  int *nrp = h->own_csr_rowptr, *ncol = h->own_csr_col;
+  float* nval = val ? h->own_csr_val : nullptr;
+  int rc = SPMX_SUCCESS;
+  // a caller's work on another stream may still read the previous CSR
+  if (nrp && cudaDeviceSynchronize() != cudaSuccess) rc = set_error(SPMX_ERR_CUDA, "coo to csr");
+  if (!nrp) rc = rc ? rc : dalloc((void**)&nrp, 4 * ((size_t)m + 1), "csr rowptr");
+  if (!ncol) rc = rc ? rc : dalloc((void**)&ncol, b, "csr col");
+  if (val && !nval) rc = rc ? rc : dalloc((void**)&nval, b, "csr val");
+  const unsigned* rows_sorted = (const unsigned*)row;
   if (!rc && unsorted) {
     const int bits_c = key_bits(n), bits_r = key_bits(m);
-    const int passes = (col_desc ? (bits_c + 7) / 8 : 0) + (bits_r + 7) / 8;
-    const int fin = passes & 1;  // set holding the result after the last pass
-    const size_t al = (b + 255) & ~(size_t)255;
-    const size_t hb = radix_scratch_bytes(nnz);
-    rc = dalloc((void**)&scratch, al * (val ? 4 : 3) + hb, "coo sort scratch");
-    if (!rc) {
-      unsigned *k[2], *r[2], *v[2] = {nullptr, nullptr};
-      char* q = scratch;
-      k[fin] = (unsigned*)ncol;
-      k[1 - fin] = (unsigned*)q; q += al;
-      r[0] = (unsigned*)q; q += al;
-      r[1] = (unsigned*)q; q += al;
-      if (val) {
-        v[fin] = (unsigned*)nval;
-        v[1 - fin] = (unsigned*)q; q += al;
-      }
-      void* radix = q;
-      cudaMemcpyAsync(k[0], col, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
-      cudaMemcpyAsync(r[0], row, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
-      if (val) cudaMemcpyAsync(v[0], val, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
-      int s = 0;  // set holding the current order
-      if (col_desc) {
-        RadixBuffers ra{k[s], k[1 - s], r[s], r[1 - s], v[s], v[1 - s], radix};
-        if (radix_sort_pairs(ra, nnz, bits_c, h->d_err, st))
-          rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
-        if (ra.result_in_alt) s = 1 - s;
-      }
-      if (!rc) {
-        RadixBuffers rb{r[s], r[1 - s], k[s], k[1 - s], v[s], v[1 - s], radix};
-        if (radix_sort_pairs(rb, nnz, bits_r, h->d_err, st))
-          rc = set_error(SPMX_ERR_INVALID_VALUE, "radix capacity");
-        if (rb.result_in_alt) s = 1 - s;
-      }
-      if (!rc && s != fin) rc = set_error(SPMX_ERR_INVALID_VALUE, "radix pass count");
-      rows_sorted = (const int*)r[s];
-      cols_sorted = k[s];
-      vals_sorted = v[s];
+    const int first = col_desc ? 0 : bits_c;
+    const int fin = radix_sort_passes(first, bits_c + bits_r) & 1;  // set holding the result after the last pass
+    unsigned *k[2], *r[2], *v[2] = {nullptr, nullptr};
+    char* q = scratch;
+    k[fin] = (unsigned*)ncol;
+    k[1 - fin] = (unsigned*)q; q += al;
+    r[0] = (unsigned*)q; q += al;
+    r[1] = (unsigned*)q; q += al;
+    if (val) {
+      v[fin] = (unsigned*)nval;
+      v[1 - fin] = (unsigned*)q; q += al;
     }
+    RadixBuffers rb{k[0], k[1], r[0], r[1], v[0], v[1], q, false, (const unsigned*)col, (const unsigned*)row,
+                    (const unsigned*)val, first, bits_c};
+    if (radix_sort_pairs(rb, nnz, bits_c + bits_r, h->d_err, st)) rc = set_error(SPMX_ERR_CUDA, "coo sort launch");
+    rows_sorted = r[fin];
   }
   // 3. row pointers from the sorted rows; columns and values into place
   if (!rc) {
-    note_launch();
-    coo_rowptr_kernel<<<ingest_grid((long long)nnz + 1), kIngestNT, 0, st>>>(nnz, m, rows_sorted, nrp);
-    if (nnz > 0 && cols_sorted != ncol) {
-      cudaMemcpyAsync(ncol, cols_sorted, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
-      if (val) cudaMemcpyAsync(nval, vals_sorted, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
+    launch_sorted_bounds(nnz, rows_sorted, m, nrp, st);
+    if (nnz > 0 && !unsorted) {
+      cudaMemcpyAsync(ncol, col, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
+      if (val) cudaMemcpyAsync(nval, val, 4 * (size_t)nnz, cudaMemcpyDeviceToDevice, st);
     }
-    ce = cudaGetLastError();
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-    if (ce != cudaSuccess) rc = set_error(SPMX_ERR_CUDA, std::string("coo to csr: ") + cudaGetErrorString(ce));
-  } else {
-    cudaStreamSynchronize(st);
+    rc = launch_ok("coo to csr");
   }
-  dfree(scratch);
+  scratch_free(scratch, st);
+  const cudaError_t ce = cudaStreamSynchronize(st);
+  if (!rc && ce != cudaSuccess) rc = set_error(SPMX_ERR_CUDA, std::string("coo to csr: ") + cudaGetErrorString(ce));
   if (rc) {
-    dfree(nrp);
-    dfree(ncol);
-    dfree(nval);
+    if (nrp != h->own_csr_rowptr) dfree(nrp);
+    if (ncol != h->own_csr_col) dfree(ncol);
+    if (nval && nval != h->own_csr_val) dfree(nval);
     return rc;
   }
-  dfree(h->own_csr_rowptr);
-  dfree(h->own_csr_col);
-  dfree(h->own_csr_val);
+  if (!val) dfree(h->own_csr_val);
   h->own_csr_rowptr = nrp;
   h->own_csr_col = ncol;
   h->own_csr_val = nval;
@@ -191,6 +158,8 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   h->has_csr = true;
   h->mat_feat_ready = false;
   h->std_row_ready = false;
+  h->batch_chunk_ready = false;
+  h->ms_hub_rowptr = nullptr;  // the arrays stay where they are: tables kept by address are not the new matrix's
   // a CSC derived from the previous CSR by spmx_to_csc is stale now
   if (h->has_csc && h->csc_colptr == h->own_colptr) h->has_csc = false;
   return SPMX_SUCCESS;

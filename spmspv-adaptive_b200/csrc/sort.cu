@@ -402,30 +402,50 @@ int radix_sort_pairs(RadixBuffers& b, int n, int key_bits, int* err, cudaStream_
 // ptr[j] = first position whose key is >= j, j in [0, extent], of `cnt` sorted
 // keys (keys past the extent end the last range): position i owns the entries
 // after its predecessor's key up to its own key (extent at i = cnt), so every
-// entry is written once, empty ranges included.  Four positions per thread in
-// flight.
+// entry is written once, empty ranges included.  A thread owns four consecutive
+// positions, a warp reads 512 bytes per load, and the key before a thread's
+// first comes from its neighbour lane.
 __global__ void __launch_bounds__(256)
-sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int* __restrict__ ptr) {
-  constexpr int U = 4;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b <= cnt; b += step * U) {
-    int lo[U], hi[U];
+sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int* __restrict__ ptr, int vec_ok) {
+  constexpr int U = 2;
+  const long long step = (long long)gridDim.x * blockDim.x * 4;
+  const int lane = threadIdx.x & 31;
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  // whole warps stay in the loop: the condition is that of the warp's first lane
+  for (long long b = first; b - 4 * lane <= cnt; b += U * step) {
+    unsigned k[U][5];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = b + u * step;
-      lo[u] = i == 0 || i > cnt ? 0 : (int)min(__ldg(key + i - 1), (unsigned)extent) + 1;
-      hi[u] = i > cnt ? -1 : i == cnt ? extent : (int)min(__ldg(key + i), (unsigned)extent);
+      if (vec_ok && i + 4 <= cnt) {
+        const uint4 t = __ldg(reinterpret_cast<const uint4*>(key + i));
+        k[u][1] = t.x; k[u][2] = t.y; k[u][3] = t.z; k[u][4] = t.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) k[u][q + 1] = i + q < cnt ? __ldg(key + i + q) : (unsigned)extent;
+      }
+      k[u][0] = __shfl_up_sync(0xffffffffu, k[u][4], 1);
+      if (lane == 0 && i > 0 && i <= cnt) k[u][0] = __ldg(key + i - 1);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      for (int j = lo[u]; j <= hi[u]; ++j) ptr[j] = (int)(b + u * step);
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long i = b + u * step + q;
+        if (i > cnt) continue;
+        const int lo = i == 0 ? 0 : (int)min(k[u][q], (unsigned)extent) + 1;
+        const int hi = i == cnt ? extent : (int)min(k[u][q + 1], (unsigned)extent);
+        for (int j = lo; j <= hi; ++j) ptr[j] = (int)i;
+      }
+    }
   }
 }
 
 int launch_sorted_bounds(int cnt, const unsigned* key, int extent, int* ptr, cudaStream_t st) {
+  if (cnt <= 0) return cudaMemsetAsync(ptr, 0, 4 * ((size_t)extent + 1), st) == cudaSuccess ? 0 : -1;
   note_launch();
-  const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)cnt + 1 + 1023) / 1024, 148LL * 8));
-  sorted_bounds_kernel<<<grid, 256, 0, st>>>(cnt, key, extent, ptr);
+  const int grid = (int)std::min<long long>(((long long)cnt + 1 + 2047) / 2048, 148LL * 8);
+  sorted_bounds_kernel<<<grid, 256, 0, st>>>(cnt, key, extent, ptr, ((uintptr_t)key & 15u) == 0);
   return 0;
 }
 
