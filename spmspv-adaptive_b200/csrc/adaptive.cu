@@ -348,42 +348,43 @@ extern "C" int spmx_bfs(spmx_handle_t h, int source, int* levels, int* depth) {
 
 static int ensure_msbfs(spmx_handle_t h) {
   if (h->ms_n == h->n && h->ms_visit) return SPMX_SUCCESS;
-  dfree(h->ms_visit); dfree(h->ms_front0); dfree(h->ms_front1); dfree(h->ms_next);
-  dfree(h->ms_q0); dfree(h->ms_q1); dfree(h->ms_srcs); dfree(h->ms_ctrl);
+  dfree(h->ms_visit); dfree(h->ms_planes); dfree(h->ms_q0); dfree(h->ms_q1); dfree(h->ms_ctrl);
+  h->ms_visit = nullptr;
+  h->ms_planes = h->ms_ctrl = nullptr;
+  h->ms_q0 = h->ms_q1 = nullptr;
   const size_t n = (size_t)std::max(h->n, 1);
-  SPMX_TRY(dalloc((void**)&h->ms_visit, 8 * n, "msbfs visit"));
-  SPMX_TRY(dalloc((void**)&h->ms_front0, 8 * n, "msbfs front 0"));
-  SPMX_TRY(dalloc((void**)&h->ms_front1, 8 * n, "msbfs front 1"));
-  SPMX_TRY(dalloc((void**)&h->ms_next, 8 * n, "msbfs next"));
   SPMX_TRY(dalloc((void**)&h->ms_q0, 4 * n, "msbfs queue 0"));
   SPMX_TRY(dalloc((void**)&h->ms_q1, 4 * n, "msbfs queue 1"));
-  SPMX_TRY(dalloc((void**)&h->ms_srcs, 4 * 64, "msbfs sources"));
-  SPMX_TRY(dalloc((void**)&h->ms_ctrl, sizeof(BfsCtrl), "msbfs ctrl"));
+  SPMX_TRY(dalloc(&h->ms_planes, 32 * n, "msbfs level planes"));
+  SPMX_TRY(dalloc(&h->ms_ctrl, sizeof(BfsCtrl), "msbfs ctrl"));
+  SPMX_TRY(dalloc((void**)&h->ms_visit, 32 * n, "msbfs words"));
+  h->ms_front0 = h->ms_visit + n;
+  h->ms_front1 = h->ms_visit + 2 * n;
+  h->ms_next = h->ms_visit + 3 * n;
   h->ms_n = h->n;
   return SPMX_SUCCESS;
 }
 
 // vertices of degree above this are pulled in chunks of this many edges
-constexpr int kHubDegree = 1024;
+constexpr int kHubDegree = 256;
 
 // hub chunk list of the multi-source pull, built once per matrix
 static int ensure_hubs(spmx_handle_t h) {
   if (h->ms_hub_rowptr == h->rowptr && h->ms_hub_nnz == h->nnz && h->ms_hcounters) return SPMX_SUCCESS;
   cudaStream_t st = h->stream;
   SPMX_CUDA(cudaStreamSynchronize(st));
-  dfree(h->ms_hchunk); dfree(h->ms_hcnt); dfree(h->ms_hacc); dfree(h->ms_hleft); dfree(h->ms_hcounters);
-  h->ms_hchunk = nullptr; h->ms_hcnt = nullptr; h->ms_hacc = nullptr; h->ms_hleft = nullptr;
+  dfree(h->ms_hchunk); dfree(h->ms_hvert); dfree(h->ms_hacc); dfree(h->ms_hcounters);
+  h->ms_hchunk = nullptr; h->ms_hvert = nullptr; h->ms_hacc = nullptr;
   h->ms_hcounters = nullptr;
   const long long nnz = std::max(h->nnz, 0);
   const int max_hubs = (int)(nnz / (kHubDegree + 1) + 1);
   const long long max_chunks = nnz / kHubDegree + max_hubs + 1;
   SPMX_TRY(dalloc((void**)&h->ms_hchunk, sizeof(int4) * (size_t)max_chunks, "msbfs hub chunks"));
-  SPMX_TRY(dalloc((void**)&h->ms_hcnt, 4 * (size_t)max_hubs, "msbfs hub chunk counts"));
+  SPMX_TRY(dalloc((void**)&h->ms_hvert, 4 * (size_t)max_hubs, "msbfs hub vertices"));
   SPMX_TRY(dalloc((void**)&h->ms_hacc, 8 * (size_t)max_hubs, "msbfs hub accumulators"));
-  SPMX_TRY(dalloc((void**)&h->ms_hleft, 4 * (size_t)max_hubs, "msbfs hub counters"));
   SPMX_TRY(dalloc((void**)&h->ms_hcounters, 8, "msbfs hub totals"));
   SPMX_CUDA(cudaMemsetAsync(h->ms_hcounters, 0, 8, st));
-  launch_hub_chunks(h->n, h->rowptr, kHubDegree, h->ms_hchunk, h->ms_hcnt, h->ms_hcounters, max_hubs,
+  launch_hub_chunks(h->n, h->rowptr, kHubDegree, h->ms_hchunk, h->ms_hvert, h->ms_hcounters, max_hubs,
                     (int)max_chunks, st);
   int cnt[2] = {0, 0};
   SPMX_CUDA(cudaMemcpyAsync(cnt, h->ms_hcounters, 8, cudaMemcpyDeviceToHost, st));
@@ -409,37 +410,16 @@ extern "C" int spmx_bfs_batched(spmx_handle_t h, const int* srcs, int nsrc, int*
   SPMX_TRY(ensure_hubs(h));
   cudaStream_t st = h->stream;
   const size_t n = (size_t)h->n;
-  const size_t total = n * (size_t)nsrc;
-  int* vmajor = levels;
-  if (layout == 1) {
-    if (h->ms_tmp_len < total) {
-      SPMX_CUDA(cudaStreamSynchronize(st));
-      dfree(h->ms_tmp);
-      h->ms_tmp = nullptr;
-      h->ms_tmp_len = 0;
-      SPMX_TRY(dalloc((void**)&h->ms_tmp, 4 * total, "msbfs levels"));
-      h->ms_tmp_len = total;
-    }
-    vmajor = h->ms_tmp;
-  }
-  SPMX_CUDA(cudaMemcpyAsync(h->ms_srcs, srcs, 4 * (size_t)nsrc, cudaMemcpyHostToDevice, st));
-  SPMX_CUDA(cudaMemsetAsync(vmajor, 0xff, 4 * total, st));
-  SPMX_CUDA(cudaMemsetAsync(h->ms_visit, 0, 8 * n, st));
-  SPMX_CUDA(cudaMemsetAsync(h->ms_front0, 0, 8 * n, st));
-  SPMX_CUDA(cudaMemsetAsync(h->ms_front1, 0, 8 * n, st));
-  SPMX_CUDA(cudaMemsetAsync(h->ms_next, 0, 8 * n, st));
-  if (h->ms_nhubs > 0) {
-    SPMX_CUDA(cudaMemsetAsync(h->ms_hacc, 0, 8 * (size_t)h->ms_nhubs, st));
-    SPMX_CUDA(cudaMemcpyAsync(h->ms_hleft, h->ms_hcnt, 4 * (size_t)h->ms_nhubs, cudaMemcpyDeviceToDevice, st));
-  }
-  HubChunks hub{h->ms_hchunk, h->ms_nhchunks, h->ms_hcnt, h->ms_hacc, h->ms_hleft, h->ms_nhubs, kHubDegree};
-  MsBfsArgs a{h->n, nsrc, h->num_sms, (long long)h->nnz, h->msbfs_alpha, h->ms_srcs, h->rowptr,
-              h->col, vmajor, h->ms_visit, h->ms_front0, h->ms_front1, h->ms_next, h->ms_q0,
-              h->ms_q1, (BfsCtrl*)h->ms_ctrl, hub, h->d_err};
-  if (launch_msbfs_persistent(a, st))
+  SPMX_CUDA(cudaMemsetAsync(h->ms_visit, 0, 32 * n, st));
+  if (h->ms_nhubs > 0) SPMX_CUDA(cudaMemsetAsync(h->ms_hacc, 0, 8 * (size_t)h->ms_nhubs, st));
+  HubChunks hub{h->ms_hchunk, h->ms_nhchunks, h->ms_hvert, h->ms_hacc, h->ms_nhubs, kHubDegree};
+  MsBfsArgs a{h->n, nsrc, layout, h->num_sms, (long long)h->nnz, h->msbfs_alpha, {}, h->rowptr, h->col, levels,
+              h->ms_visit, h->ms_front0, h->ms_front1, h->ms_next, (ulonglong4*)h->ms_planes, h->ms_q0, h->ms_q1,
+              (BfsCtrl*)h->ms_ctrl, hub, h->d_err};
+  std::copy(srcs, srcs + nsrc, a.srcs.v);
+  if (launch_msbfs(a, st))
     return set_error(SPMX_ERR_CUDA, std::string("cooperative multi-source BFS launch: ") +
                                         cudaGetErrorString(cudaGetLastError()));
-  if (layout == 1) launch_levels_transpose(h->n, nsrc, vmajor, levels, st);
   SPMX_TRY(launch_ok("batched bfs"));
   if (depth) {
     SPMX_CUDA(cudaMemcpyAsync(h->h_pinned + 1, &((BfsCtrl*)h->ms_ctrl)->depth, sizeof(int),

@@ -8,10 +8,10 @@ namespace spmx {
 struct BfsCtrl {
   int cnt[3];                    // next-frontier sizes, by level % 3
   int depth;                     // number of levels, written at the end
-  unsigned long long edges[3];   // sum of degrees of the next frontier
+  unsigned long long edges[3];   // sum of degrees of the next frontier (multi-source: size << 32 | sum)
   unsigned bar_count, bar_gen;   // grid barrier
   int abort_flag;
-  int pad;
+  int pad;                       // multi-source: levels already expanded
 };
 
 struct BfsPersistentArgs {
@@ -32,32 +32,35 @@ struct BfsPersistentArgs {
   int* err;
 };
 
-// Hubs for the multi-source pull: every vertex of degree > deg is cut into
-// chunks of deg edges that all warps share; acc / left are per-hub OR
-// accumulators and outstanding-chunk counters, reset to 0 / nchunk_of each
-// level.
+// Hubs of the multi-source BFS: every vertex of degree > deg is cut into
+// chunks of deg edges that all warps share; acc holds per-hub OR accumulators
+// of a pull level, zero between levels.
 struct HubChunks {
   const int4* chunk;     // {vertex, first edge, end edge, hub index}
   long long nchunks;
-  const int* nchunk_of;  // chunks per hub
+  const int* vertex;     // [nhubs]
   unsigned long long* acc;
-  int* left;
   int nhubs;
   int deg;
 };
 
+struct MsSources {
+  int v[64];
+};
+
 struct MsBfsArgs {
-  int n, ns, num_sms;
+  int n, ns, layout, num_sms;
   long long total_edges;
   double alpha;        // pull when the frontier's edges exceed total/alpha
-  const int* srcs;     // device [ns]
+  MsSources srcs;      // by value: no copy to the device
   const int* rowptr;
   const int* col;
-  int* levels;         // device [n * ns], vertex-major
-  unsigned long long* visit;
+  int* levels;         // device [n * ns], layout 1: [s][v], 0: [v][s]
+  unsigned long long* visit;   // the four arrays start zeroed
   unsigned long long* front0;
   unsigned long long* front1;
   unsigned long long* next;
+  ulonglong4* planes;  // [n]
   int* q0;
   int* q1;
   BfsCtrl* ctrl;
@@ -65,11 +68,10 @@ struct MsBfsArgs {
   int* err;
 };
 
-int launch_hub_chunks(int n, const int* rowptr, int deg_cut, int4* chunk, int* nchunk_of,
+int launch_hub_chunks(int n, const int* rowptr, int deg_cut, int4* chunk, int* vertex,
                       int* counters, int max_hubs, int max_chunks, cudaStream_t st);
 int launch_bfs_persistent(const BfsPersistentArgs& a, cudaStream_t st);
-int launch_msbfs_persistent(const MsBfsArgs& a, cudaStream_t st);
-int launch_levels_transpose(int n, int ns, const int* vmajor, int* smajor, cudaStream_t st);
+int launch_msbfs(const MsBfsArgs& a, cudaStream_t st);
 
 int launch_bfs_init(int src, int* levels, unsigned* visited, int* q,
                     int* q_count, cudaStream_t st);

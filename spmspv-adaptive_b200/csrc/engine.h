@@ -108,15 +108,13 @@ struct spmx_handle_s {
   unsigned* bfs_fb1 = nullptr;
   void* bfs_ctrl = nullptr;                // BfsCtrl
   // batched (multi-source) BFS buffers
-  unsigned long long* ms_visit = nullptr;
+  unsigned long long* ms_visit = nullptr;  // one allocation: visit, front 0, front 1, next
   unsigned long long* ms_front0 = nullptr;
   unsigned long long* ms_front1 = nullptr;
   unsigned long long* ms_next = nullptr;
   int* ms_q0 = nullptr;
   int* ms_q1 = nullptr;
-  int* ms_srcs = nullptr;
-  int* ms_tmp = nullptr;                   // vertex-major levels for layout 1
-  size_t ms_tmp_len = 0;
+  void* ms_planes = nullptr;               // level bits, 32 bytes per vertex
   void* ms_ctrl = nullptr;
   int ms_n = 0;
   // batched SpMSpV: the batch inverted by column (radix sort buffers for
@@ -145,9 +143,8 @@ struct spmx_handle_s {
   int* batch_ctr = nullptr;  // [0] the forward walk's chunk counter, [1] the dvals walk's
   // hub chunks of the multi-source pull (built once per matrix)
   int4* ms_hchunk = nullptr;
-  int* ms_hcnt = nullptr;
+  int* ms_hvert = nullptr;
   unsigned long long* ms_hacc = nullptr;
-  int* ms_hleft = nullptr;
   int* ms_hcounters = nullptr;
   long long ms_nhchunks = 0;
   int ms_nhubs = 0;
