@@ -10,7 +10,11 @@
 //   DEV/csc_sort_load_balance.cuh:295) whose look-back spins without bound on
 //   `sum[gid-1]==0` (scan_kernel.cuh:99).
 //
-// Stage 2, csc_lb_kernel: persistent CTAs take blocks of 2048 work items.
+// The dense-y (atomic) write-back of a handle needs no global scan:
+// csc_flat_kernel.
+//
+// Stage 2 of the sort write-back and of the allocation-free entry point (the
+//   bucket kernels share the block mapping), csc_lb_kernel: persistent CTAs take blocks of 2048 work items.
 //   "twolayer" blocks hold 2048 nonzeros (DEV/csc_two_layer_load_balance_
 //   fuse_reduction_modify.cuh:155); "merge" blocks hold 2048 merge-path items
 //   = nonzeros + column ends (DEV/csc_sort_load_balance_fuse_reduction_
@@ -182,6 +186,145 @@ csc_naive_kernel(CscArgs a, float* __restrict__ y) {
   }
 }
 
+// Load-balanced SpMSpV with atomic write-back, without a scan: a warp takes E
+// consecutive x entries (E = 2^elog <= 32), scans their column lengths with
+// shuffles and spreads the nonzeros over its lanes, U per lane in flight; a
+// column above kFlatCut nonzeros is handed to csc_flat_long_kernel in chunks, so
+// no warp serialises on a hub.  Everything up to the first U nonzeros is read
+// before the wait for the zero fill.  The owner of a nonzero is found by binary
+// search over the lanes' prefix.
+//
+// What bounds it: the latency of x key -> column bounds -> nonzeros over three
+// chained grids (5 us for a handful of entries), then the L2 reductions, which
+// serialise on the rows of hubs.  1M-vertex Chung-Lu graph, x of 10,000 entries
+// (0.3M nonzeros): 13.4 us against 43 for memset, scan, block tables and
+// csc_lb_kernel (27 of it the scan in 5 CTAs); x of 100,000: 96 against 161;
+// Zipf 1M, x of 105,000: 19.8 against 43.6.  Cut and chunk (10,000 / 100,000
+// entries): 512 and 256 16.7 / 141 us, 256 and 256 14.7 / 106, 128 and 128 13.4 /
+// 96, 64 and 64 13.6 / 85.  Two nonzeros in flight per lane instead of four 14.2 /
+// 108, eight 15.6 / 122.
+template <int U>
+__global__ void __launch_bounds__(256)
+csc_flat_kernel(CscArgs a, int elog, float* __restrict__ y, CscLong* queue, int qcap, int defer) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ unsigned s_bin[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long i = (((long long)blockIdx.x * 8 + w) << elog) + lane;
+  const bool mine = lane < (1 << elog) && i < a.x_nnz;
+  const int key = mine ? __ldg(a.x_key + i) : -1;
+  float xv = mine ? __ldg(a.x_val + i) : 0.f;
+  const bool ok = (unsigned)key < (unsigned)a.n;
+  if (mine && !ok) flag_error(a.err, kDevErrOob);
+  int cs = 0, len = 0;
+  if (ok) {
+    cs = __ldg(a.colptr + key);
+    len = __ldg(a.colptr + key + 1) - cs;
+  }
+  xv = (float)(a.alpha * (double)xv);
+  const bool is_long = defer && len > kFlatCut;
+  const int flat = is_long ? 0 : len;
+  const int incl = warp_inclusive_sum(flat);
+  const int base = cs - (incl - flat);  // position of the warp's item q: base of its owner + q
+  const int total = __shfl_sync(FULL, incl, 31);
+  const unsigned bins = __reduce_add_sync(FULL, (unsigned)len);
+  if (lane == 0) s_bin[w] = bins;
+  int r[U];
+  float v[U];
+  auto load = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * 32 + lane;
+      int o = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int t = __shfl_sync(FULL, incl, o + step - 1);
+        if (t <= q) o += step;
+      }
+      const int p = __shfl_sync(FULL, base, o) + q;
+      const float x = __shfl_sync(FULL, xv, o);
+      r[u] = -1;
+      v[u] = 0.f;
+      if (q < total) {
+        r[u] = __ldg(a.row + p);
+        v[u] = __ldg(a.val + p) * x;
+      }
+    }
+  };
+  load(0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  for (int q0 = 0;;) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (q0 + u * 32 + lane >= total) continue;
+      if ((unsigned)r[u] < (unsigned)a.m) atomicAdd(y + r[u], v[u]);
+      else flag_error(a.err, kDevErrOob);
+    }
+    q0 += 32 * U;
+    if (q0 >= total) break;
+    load(q0);
+  }
+  // hand the long columns over, chunk by chunk
+  for (unsigned lm = __ballot_sync(FULL, is_long); lm; lm &= lm - 1) {
+    const int sl = __ffs(lm) - 1;
+    const int c0 = __shfl_sync(FULL, cs, sl), c1 = c0 + __shfl_sync(FULL, len, sl);
+    const float x = __shfl_sync(FULL, xv, sl);
+    const int nch = (c1 - c0 + kFlatChunk - 1) / kFlatChunk;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(a.counts + kCntLong, nch);
+    at = __shfl_sync(FULL, at, 0);
+    for (int j = lane; j < nch; j += 32) {
+      const int s0 = c0 + j * kFlatChunk, s1 = min(c1, s0 + kFlatChunk);
+      if (at + j < qcap) {
+        queue[at + j] = CscLong{s0, s1, x};
+      } else {  // only with repeated x keys: this lane's chunk on the spot
+        for (int k = s0; k < s1; ++k) {
+          const int rr = __ldg(a.row + k);
+          if ((unsigned)rr < (unsigned)a.m) atomicAdd(y + rr, __ldg(a.val + k) * x);
+          else flag_error(a.err, kDevErrOob);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned t = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t += s_bin[q];
+    if (t) atomicAdd(a.counts + kCntBinlen, (int)t);
+  }
+}
+
+// the chunks of the long columns, one warp each
+__global__ void __launch_bounds__(256)
+csc_flat_long_kernel(CscArgs a, float* __restrict__ y, const CscLong* queue, int qcap) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  constexpr int U = 8;
+  const int cnt = min(*(volatile int*)(a.counts + kCntLong), qcap);
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < cnt; c += nw) {
+    const CscLong ch = queue[c];
+    for (int kb = ch.k0; kb < ch.k1; kb += 32 * U) {
+      int r[U];
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = kb + u * 32 + lane;
+        r[u] = k < ch.k1 ? __ldg(a.row + k) : -1;
+        v[u] = k < ch.k1 ? __ldg(a.val + k) * ch.x : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (kb + u * 32 + lane >= ch.k1) continue;
+        if ((unsigned)r[u] < (unsigned)a.m) atomicAdd(y + r[u], v[u]);
+        else flag_error(a.err, kDevErrOob);
+      }
+    }
+  }
+}
+
 template <int G>
 __global__ void __launch_bounds__(256)
 csc_naive_pairs_kernel(CscArgs a, CscScratch s, int* __restrict__ prow,
@@ -241,9 +384,14 @@ int launch_csc_lb(const CscArgs& a, const CscScratch& s, int variant, float* y,
 // lets the next grid launch: a dependent that reads its inputs before its own
 // wait (x keys, column bounds) therefore never starts while a grid that
 // writes them is still running.
-__global__ void zero_fill_kernel(float* __restrict__ y, long long m) {
+// c0 / c1 (optional) are cleared too: counters of the grid that follows.
+__global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, int* c1) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (c0) *c0 = 0;
+    if (c1) *c1 = 0;
+  }
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nt = (long long)gridDim.x * blockDim.x;
   if ((((uintptr_t)y) & 15u) == 0) {
@@ -260,11 +408,11 @@ __global__ void zero_fill_kernel(float* __restrict__ y, long long m) {
 // whatever grid ran before it (the previous call's last kernel): its launch
 // and CTA start-up overlap that grid's tail (2.4 -> 1.2 us per kernel boundary
 // measured on B200), and its griddepcontrol.wait keeps the order.
-int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st) {
-  if (m <= 0) return 0;
+int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0, int* c1) {
+  if (m <= 0 && !c0 && !c1) return 0;
   const long long blocks = std::min<long long>((m + 1023) / 1024, (long long)num_sms * 4);
   note_launch();
-  return launch_pdl(zero_fill_kernel, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st, y, m) ==
+  return launch_pdl(zero_fill_kernel, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st, y, m, c0, c1) ==
                  cudaSuccess
              ? 0
              : -2;
@@ -300,6 +448,25 @@ int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, 
   return e == cudaSuccess ? 0 : -2;
 }
 
+int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
+                    cudaStream_t st) {
+  if (launch_zero_fill(y, a.m, num_sms, st, a.counts + kCntBinlen, a.counts + kCntLong)) return -2;
+  if (a.x_nnz <= 0) return 0;
+  // entries per warp: enough that the grid is about one wave of warps
+  const long long resident = (long long)num_sms * 64;
+  int elog = 0;
+  while (elog < 5 && ((long long)a.x_nnz >> elog) > resident) ++elog;
+  const long long warps = ((long long)a.x_nnz + (1 << elog) - 1) >> elog;
+  const int defer = col_max < 0 || col_max > kFlatCut;  // the longest column, where it is known
+  note_launch(1 + defer);
+  cudaError_t e = launch_pdl(csc_flat_kernel<4>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, a, elog, y,
+                             s.longq, s.long_cap, defer);
+  if (e == cudaSuccess && defer)
+    e = launch_pdl(csc_flat_long_kernel, dim3((unsigned)num_sms * 4), dim3(256), 0, st, a, y,
+                   (const CscLong*)s.longq, s.long_cap);
+  return e == cudaSuccess ? 0 : -2;
+}
+
 int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st) {
   if (a.x_nnz <= 0) return 0;
   const long long threads = (long long)a.x_nnz * group;
@@ -325,7 +492,7 @@ namespace spmx {
 int csc_lb_blocks_per_sm() {
   int b = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &b, csc_lb_kernel<kCscLbNT, kCscLbVT, false>, kCscLbNT, 0) != cudaSuccess) {
+          &b, csc_lb_kernel<kCscLbNT, kCscLbVT, true>, kCscLbNT, 0) != cudaSuccess) {
     cudaGetLastError();
     return 2;
   }

@@ -265,6 +265,7 @@ static void free_sort_scratch(spmx_handle_t h) {
 
 static void free_csc_scratch(spmx_handle_t h) {
   dfree(h->cs.off); dfree(h->cs.colstart); dfree(h->cs.bstart_tl); dfree(h->cs.bstart_mg);
+  dfree(h->cs.longq);
   h->cs = CscScratch{};
   h->cs_ready = false;
 }
@@ -376,6 +377,7 @@ extern "C" int spmx_input_csc(spmx_handle_t h, int nnz, const int* csc_row,
   h->csc_colptr = csc_col;
   h->csc_val = csc_val;
   h->has_csc = true;
+  h->col_max = -1;
   return SPMX_SUCCESS;
 }
 
@@ -449,6 +451,7 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
   h->csc_row = h->own_row;
   h->csc_val = h->own_cval;
   h->has_csc = true;
+  h->col_max = -1;
   return launch_ok("ToCSC");
 }
 
@@ -665,6 +668,9 @@ static int ensure_csc_scratch(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&h->cs.colstart, 4 * (size_t)n, "csc colstart"));
   SPMX_TRY(dalloc((void**)&h->cs.bstart_tl, 4 * (size_t)h->cs.tl_cap, "bstart tl"));
   SPMX_TRY(dalloc((void**)&h->cs.bstart_mg, 4 * (size_t)h->cs.mg_cap, "bstart mg"));
+  // a long column has more than kFlatCut nonzeros, so rounding up adds at most half a chunk per two
+  h->cs.long_cap = (int)(h->nnz / kFlatChunk + h->nnz / kFlatCut + 1);
+  SPMX_TRY(dalloc((void**)&h->cs.longq, sizeof(CscLong) * (size_t)h->cs.long_cap, "csc long columns"));
   if (h->lb_grid <= 0) h->lb_grid = h->num_sms * std::max(1, csc_lb_blocks_per_sm());
   h->cs_ready = true;
   return SPMX_SUCCESS;
@@ -876,11 +882,8 @@ static int csc_atomic(spmx_handle_t h, int variant, float alpha, float* y, int* 
     if (launch_csc_naive_zeroed(a, col_group(h), y, h->num_sms, st))
       return set_error(SPMX_ERR_INVALID_VALUE, "bad column group");
   } else {
-    SPMX_CUDA(cudaMemsetAsync(y, 0, 4 * (size_t)h->m, st));
     SPMX_TRY(ensure_csc_scratch(h));
-    if (launch_csc_scan(a, h->cs, h->ls, kCscLbNT * kCscLbVT, st))
-      return set_error(SPMX_ERR_INVALID_VALUE, "scan capacity");
-    launch_csc_lb(a, h->cs, variant == SPMX_CSC_LB_MERGE ? 1 : 2, y, nullptr, nullptr, h->lb_grid, st);
+    if (launch_csc_flat(a, h->cs, y, h->col_max, h->num_sms, st)) return set_error(SPMX_ERR_CUDA, "csc spmspv launch");
   }
   SPMX_TRY(launch_ok("csc spmspv"));
   if (ykey && yval) return dense_to_sparse(h, h->m, y, ykey, yval, kCntYnnz, ynnz);

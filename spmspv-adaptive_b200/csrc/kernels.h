@@ -65,6 +65,7 @@ enum CounterSlot : int {
   kCntXnnz = 2,
   kCntBlocksTL = 3,
   kCntBlocksMG = 4,
+  kCntLong = 5,        // chunks of long columns
   kCntFeatSum = 8,   // 64-bit (slots 8..9)
   kCntFeatMax = 10,
   kCntFeatMinInv = 11,
@@ -91,7 +92,17 @@ struct CscScratch {
   int* bstart_tl;  // block -> first x entry (fixed nnz per block)
   int* bstart_mg;  // block -> first x entry (merge-path items)
   int tl_cap, mg_cap;  // capacities of the two tables
+  struct CscLong* longq;  // chunks of long columns (csc_flat_kernel)
+  int long_cap;
 };
+
+// kFlatChunk nonzeros of one column and its x value
+struct CscLong {
+  int k0, k1;
+  float x;
+};
+constexpr int kFlatCut = 128;    // columns above this are cut into chunks of
+constexpr int kFlatChunk = 128;  // this many nonzeros
 
 constexpr int kCscScanNT = 256, kCscScanVT = 8;   // 2048 x entries per tile
 constexpr int kCscLbNT = 256, kCscLbVT = 8;       // 2048 items per LB block
@@ -103,6 +114,11 @@ int launch_csc_scan(const CscArgs& a, const CscScratch& s, ScanScratch& ls,
 int launch_csc_lb(const CscArgs& a, const CscScratch& s, int variant, float* y,
                   int* pairs_row, float* pairs_val, int grid, cudaStream_t st);
 int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st);
+// y = 0, then the load-balanced SpMSpV with atomic write-back; col_max: the
+// longest column of the matrix, -1 where it is not known.  bin_len goes to
+// counts[kCntBinlen].
+int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
+                    cudaStream_t st);
 // y = 0 then the naive CSC SpMSpV, as a programmatic dependent launch pair
 int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, cudaStream_t st);
 int launch_csc_naive_pairs(const CscArgs& a, const CscScratch& s, int group,
@@ -110,7 +126,7 @@ int launch_csc_naive_pairs(const CscArgs& a, const CscScratch& s, int group,
 
 // ---- vecconv.cu
 // y[0..m) = 0 with a kernel that lets the next grid launch early
-int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st);
+int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0 = nullptr, int* c1 = nullptr);
 // dense[0..len) from (key, val): a zero fill, then the scatter as a
 // programmatic dependent launch that reads its keys and values while the
 // fill runs; the scatter in turn lets the next grid start early

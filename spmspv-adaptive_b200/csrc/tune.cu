@@ -277,13 +277,6 @@ extern "C" int spmx_autotune(spmx_handle_t h, const char* cache_path, int* spmv_
         if (t < bt) { bt = t; best.col_group = g; }
       }
       bt = 1e30f;
-      for (int v : {SPMX_CSC_LB_MERGE, SPMX_CSC_LB_TWOLAYER}) {
-        const float t = time_us([&] {
-          return spmx_spmspv_csc(h, v, SPMX_WB_ATOMIC, 1.0f, y, nullptr, nullptr, nullptr);
-        });
-        if (t < bt) { bt = t; best.lb_variant = v; }
-      }
-      bt = 1e30f;
       for (int b : {64, 256, 1024}) {
         const float t = time_us([&] { return spmx_csc_bucket(h, 1.0f, nullptr, y, nullptr, nullptr, b); });
         if (t < bt) { bt = t; best.buckets = b; }
