@@ -281,16 +281,6 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
   }
 }
 
-// 16-byte asynchronous copy global -> shared (L2 only), and its group waits
-__device__ __forceinline__ void batch_cp16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void batch_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void batch_cp_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // dvals[k] = alpha * sum over column col_k's pairs of xval[e] * dY[i][v(e)],
 // one warp per row with dY's row in shared memory.  With dxval (fused form,
 // dxval zeroed before) every pair also adds alpha * a[k] * dY[i][v(e)] into
@@ -316,10 +306,10 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     if (r < m && a0 < a1) {
       const float4* d4 = reinterpret_cast<const float4*>(dY + (size_t)r * nvec);
       float4* s4 = reinterpret_cast<float4*>(g0 + into * nvec);
-      if (lane < n4) batch_cp16(s4 + lane, d4 + lane);
-      if (lane + 32 < n4) batch_cp16(s4 + lane + 32, d4 + lane + 32);
+      if (lane < n4) cp_async16(s4 + lane, d4 + lane);
+      if (lane + 32 < n4) cp_async16(s4 + lane + 32, d4 + lane + 32);
     }
-    batch_cp_commit();
+    cp_async_commit();
   };
   BatchRowIter it;
   it.init(ctr, nch, chunk_row, m, lane);
@@ -341,7 +331,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     if (cur.a0 < cur.a1) {  // warp-uniform
       float* const g = g0 + (pre ? buf * nvec : 0);
       if (pre) {
-        batch_cp_wait<1>();  // every group but the next row's: this row's dY has landed
+        cp_async_wait<1>();  // every group but the next row's: this row's dY has landed
       } else if (vec4) {
         const float4* d4 = reinterpret_cast<const float4*>(dY + (size_t)i * nvec);
         for (int v = lane; v < n4; v += 32) reinterpret_cast<float4*>(g)[v] = __ldg(d4 + v);
@@ -376,7 +366,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     i = i1;
     i1 = i2;
   }
-  batch_cp_wait<0>();
+  cp_async_wait<0>();
 }
 
 // dxval[e] = alpha * sum_i A[i][xkey[e]] * dY[i][v(e)], one warp per entry

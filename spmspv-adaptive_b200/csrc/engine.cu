@@ -702,10 +702,16 @@ extern "C" int spmx_hola_preprocess(spmx_handle_t h) {
   t.K = hola_chunk_nnz(t.vt);
   t.nchunks = (h->nnz + t.K - 1) / t.K;
   SPMX_TRY(dalloc((void**)&t.chunk_row, 4 * (size_t)(t.nchunks + 1), "hola chunk rows"));
+  SPMX_TRY(dalloc((void**)&t.list, sizeof(int4) * (size_t)std::max(t.nchunks, 1), "hola chunk list"));
   SPMX_TRY(dalloc((void**)&t.carry, 8 * (size_t)std::max(2 * t.nchunks, 1), "hola carry"));
   SPMX_TRY(dalloc((void**)&t.arrive, 4 * (size_t)std::max(t.nchunks, 1), "hola arrive"));
   SPMX_CUDA(cudaMemsetAsync(t.arrive, 0, 4 * (size_t)std::max(t.nchunks, 1), h->stream));
-  launch_chunk_rows(h->m, h->rowptr, t.K, t.nchunks, t.chunk_row, h->stream);
+  // d_iacc: how many chunks have only short rows, how many have not
+  SPMX_CUDA(cudaMemsetAsync(h->d_iacc, 0, 2 * sizeof(int), h->stream));
+  launch_chunk_rows(h->m, h->nnz, h->rowptr, t.K, t.nchunks, t.chunk_row, t.list, h->d_iacc, h->stream);
+  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned + 2, h->d_iacc, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  SPMX_CUDA(cudaStreamSynchronize(h->stream));
+  t.n_short = h->h_pinned[2] >= t.nchunks / 4 ? h->h_pinned[2] : 0;
   h->hola = t;
   h->hola_ready = true;
   return launch_ok("holaPreprocess");
@@ -715,7 +721,7 @@ extern "C" int spmx_hola_postprocess(spmx_handle_t h) {
   SPMX_CHECK_HANDLE(h);
   if (h->hola_ready) {
     cudaStreamSynchronize(h->stream);
-    dfree(h->hola.chunk_row); dfree(h->hola.carry); dfree(h->hola.arrive);
+    dfree(h->hola.chunk_row); dfree(h->hola.list); dfree(h->hola.carry); dfree(h->hola.arrive);
   }
   h->hola = HolaTables{};
   h->hola_ready = false;
@@ -757,7 +763,7 @@ static int hola_spmv_impl(spmx_handle_t h, float alpha, float* y, bool gated) {
   SpmvArgs a;
   SPMX_TRY(spmv_common(h, alpha, y, gated, &a));
   if (!h->hola_ready) return set_error(SPMX_ERR_NOT_READY, "call spmx_hola_preprocess first");
-  if (launch_spmv_hola(a, h->hola, h->stream)) return set_error(SPMX_ERR_INVALID_VALUE, "bad Hola tile");
+  if (launch_spmv_hola(a, h->hola, h->stream)) return set_error(SPMX_ERR_INVALID_VALUE, "bad Hola tile or launch");
   return launch_ok("hola spmv");
 }
 

@@ -26,15 +26,20 @@ struct HolaTables {
   int K;         // nonzeros per CTA = 256 * vt
   int nchunks;   // ceil(nnz / K)
   int* chunk_row;  // [nchunks + 1]
+  int4* list;      // [nchunks] chunk descriptors: n_short chunks of short rows, then the others
+  int n_short;     // 0: not worth their own kernel
   double* carry;   // [2 * nchunks]
   unsigned* arrive;  // [nchunks], zero between calls
 };
 
+// a chunk none of whose rows has more nonzeros in it is worked row by row
+constexpr int kShortRow = 32;
+
 // ---- spmv.cu
 int launch_spmv_naive(const SpmvArgs& a, int group, cudaStream_t st);
 int launch_spmv_hola(const SpmvArgs& a, const HolaTables& t, cudaStream_t st);
-int launch_chunk_rows(int m, const int* rowptr, int K, int nchunks,
-                      int* chunk_row, cudaStream_t st);
+int launch_chunk_rows(int m, int nnz, const int* rowptr, int K, int nchunks, int* chunk_row,
+                      int4* list, int* counts, cudaStream_t st);
 int hola_chunk_nnz(int vt);
 
 // ---- adjoint.cu

@@ -14,8 +14,11 @@
 //   (atomic counter per row) adds the partials in chunk order and writes y, so
 //   the result is deterministic and needs no zero-fill of y and no second
 //   launch.
-#include "kernels.h"
+#include <algorithm>
+
 #include "common.cuh"
+#include "engine.h"
+#include "kernels.h"
 
 namespace spmx {
 
@@ -59,6 +62,26 @@ spmv_rowgroup_kernel(int m, int n, const int* __restrict__ rowptr,
 // hola: fixed nnz per CTA
 // --------------------------------------------------------------------------
 
+// Splits the chunks into those of short rows (no row has more than kShortRow
+// nonzeros in the chunk, the row that continues from the chunk before included;
+// list[0 ..)) and the others (from the back of the list): one warp per chunk.
+__global__ void chunk_split_kernel(const int* __restrict__ rowptr, int nnz, int K, int nchunks,
+                                   const int* __restrict__ chunk_row, int4* __restrict__ list, int* counts) {
+  const int lane = threadIdx.x & 31;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nchunks) return;
+  const int s = c * K, e = (int)min((long long)s + K, (long long)nnz);
+  const int lo = __ldg(chunk_row + c), hi = __ldg(chunk_row + c + 1);
+  bool is_long = lane == 0 && lo > 0 && min(__ldg(rowptr + lo), e) - s > kShortRow;
+  for (int r = lo + lane; r < hi && !is_long; r += 32)
+    is_long = min(__ldg(rowptr + r + 1), e) - __ldg(rowptr + r) > kShortRow;
+  is_long = __any_sync(0xffffffffu, is_long);
+  if (lane == 0) {
+    const int at = is_long ? nchunks - 1 - atomicAdd(counts + 1, 1) : atomicAdd(counts, 1);
+    list[at] = make_int4(c, lo, hi, 0);
+  }
+}
+
 // chunk_row[c] = first row r with rowptr[r] >= c*K (lower bound over
 // rowptr[0..m)); chunk_row[nchunks] = m.
 __global__ void chunk_rows_kernel(int m, const int* __restrict__ rowptr, int K,
@@ -96,20 +119,111 @@ __device__ __forceinline__ void split_row_contribute(
   }
 }
 
+// The chunks of short rows: the products go to shared memory in FP64 (exact),
+// element by element with coalesced loads, and every row is then summed by one
+// thread, in column order; no scan.  Persistent CTAs: the loads of a CTA's next
+// chunk are in flight while this one's rows are summed, the descriptor of the
+// one after too.  With `whole` (every chunk of the matrix is short) a chunk also
+// reads the up to kShortRow nonzeros past its end that its last row may have, so
+// no row is split; otherwise split rows meet as in spmv_chunk_kernel.
+//
+// What bounds it: DRAM latency ahead of DRAM bandwidth.  5-point Laplacian 2048^2
+// (21.0M nonzeros, 218 MB): 52 us (4.2 TB/s) against 97 by the segmented scan; one
+// CTA per chunk without the loads ahead 78 us, one thread gathering for each row
+// from staged columns and values 88 to 94 us (300 instructions per row).
+template <int NT, int VT, bool GATED>
+__global__ void __launch_bounds__(NT, 1024 / NT)
+spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __restrict__ col,
+                  const float* __restrict__ val, const float* __restrict__ x, const int* __restrict__ bits,
+                  double alpha, float* __restrict__ y, const int4* __restrict__ list, int count, int whole,
+                  double* carry, unsigned* arrive, int* err) {
+  constexpr int K = NT * VT;
+  extern __shared__ double s_short[];  // two buffers of K + kShortRow products
+  int cc[VT + 1], ra[2], rb[2];        // element VT: past the chunk's end, first warp only
+  float vv[VT + 1];
+  const auto desc = [&](long long i) { return i < count ? __ldg(list + i) : make_int4(-1, 0, 0, 0); };
+  const auto load = [&](const int4& d) {
+    if (d.x < 0) return;
+    const int s = d.x * K, left = nnz - s;
+#pragma unroll
+    for (int j = 0; j <= VT; ++j) {
+      const int q = j * NT + threadIdx.x;
+      const bool in = q < left && (j < VT || (whole && threadIdx.x < kShortRow));
+      cc[j] = in ? __ldcs(col + s + q) : 0;
+      vv[j] = in ? __ldcs(val + s + q) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int r = d.y - 1 + whole + (int)threadIdx.x + q * NT;
+      const bool in = r >= 0 && r < d.z;
+      ra[q] = in ? __ldg(rowptr + r) : 0;
+      rb[q] = in ? __ldg(rowptr + r + 1) : 0;
+    }
+  };
+  int4 d = desc(blockIdx.x), d1 = desc((long long)blockIdx.x + gridDim.x);
+  load(d);
+  int buf = 0;
+  for (long long i = blockIdx.x; i < count; i += gridDim.x) {
+    const int4 d2 = desc(i + 2LL * gridDim.x);
+    double* const s_p = s_short + buf * (K + kShortRow);
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j <= VT; ++j) {
+      if (j == VT && threadIdx.x >= kShortRow) break;
+      bool use = (unsigned)cc[j] < (unsigned)n;
+      bad |= !use;
+      if (GATED) use = use && bit_is_set(bits, cc[j]);
+      const float xv = use ? __ldg(x + cc[j]) : 0.f;
+      s_p[j * NT + threadIdx.x] = use ? (double)vv[j] * (double)xv : 0.0;
+    }
+    if (bad) flag_error(err, kDevErrOob);
+    const int c = d.x, lo = d.y, hi = d.z, s = c * K, e = (int)min((long long)s + K, (long long)nnz);
+    const int a0 = ra[0], b0 = rb[0], a1 = ra[1], b1 = rb[1];
+    load(d1);
+    // the products are there; nobody reads the other buffer (the rows of the
+    // chunk before) any more once this barrier is behind everybody
+    __syncthreads();
+    int q = 0;
+    for (int r = lo - 1 + whole + (int)threadIdx.x; r < hi; r += NT, ++q) {
+      if (r < 0) continue;
+      int a = q == 0 ? a0 : a1, b = q == 0 ? b0 : b1;
+      if (q > 1) {
+        a = __ldg(rowptr + r);
+        b = __ldg(rowptr + r + 1);
+      }
+      const int p1 = (whole ? b : min(b, e)) - s;
+      double sum = 0.0;
+      for (int p = max(a, s) - s; p < p1; ++p) sum += s_p[p];
+      if (r < lo) {
+        if (b > s) split_row_contribute<K>(r, c, 0, sum, rowptr, carry, arrive, alpha, y);
+      } else if (b == a) {
+        y[r] = 0.f;
+      } else if (whole || b <= e) {
+        y[r] = (float)(alpha * sum);
+      } else {
+        split_row_contribute<K>(r, c, 1, sum, rowptr, carry, arrive, alpha, y);
+      }
+    }
+    buf ^= 1;
+    d = d1;
+    d1 = d2;
+  }
+}
+
 template <int NT, int VT, bool GATED>
 __global__ void __launch_bounds__(NT)
 spmv_chunk_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
                   const int* __restrict__ col, const float* __restrict__ val,
                   const float* __restrict__ x, const int* __restrict__ bits,
                   double alpha, float* __restrict__ y,
-                  const int* __restrict__ chunk_row, double* carry,
+                  const int* __restrict__ chunk_row, const int4* __restrict__ list, double* carry,
                   unsigned* arrive, int vec_ok, int* err) {
   constexpr int K = NT * VT;
   __shared__ double sP[K];
   __shared__ double s_wtmp[NT / 32 + 1];
   __shared__ int s_tf[NT / 32 + 1];
   __shared__ unsigned s_flag[K / 32];
-  const int c = blockIdx.x;
+  const int c = list ? __ldg(list + blockIdx.x).x : (int)blockIdx.x;  // no list: every chunk
   const int s = c * K;
   const int e = min(s + K, nnz);
   const int base = s + (int)threadIdx.x * VT;
@@ -239,12 +353,16 @@ int launch_spmv_naive(const SpmvArgs& a, int group, cudaStream_t st) {
 
 int hola_chunk_nnz(int vt) { return 256 * vt; }
 
-int launch_chunk_rows(int m, const int* rowptr, int K, int nchunks,
-                      int* chunk_row, cudaStream_t st) {
+int launch_chunk_rows(int m, int nnz, const int* rowptr, int K, int nchunks, int* chunk_row,
+                      int4* list, int* counts, cudaStream_t st) {
   int threads = nchunks + 1;
   note_launch();
   chunk_rows_kernel<<<(threads + 255) / 256, 256, 0, st>>>(m, rowptr, K, nchunks,
                                                          chunk_row);
+  if (nchunks > 0) {
+    note_launch();
+    chunk_split_kernel<<<(nchunks + 7) / 8, 256, 0, st>>>(rowptr, nnz, K, nchunks, chunk_row, list, counts);
+  }
   return 0;
 }
 
@@ -256,28 +374,41 @@ int launch_spmv_hola(const SpmvArgs& a, const HolaTables& t, cudaStream_t st) {
   }
   const int vec_ok = (((uintptr_t)a.col | (uintptr_t)a.val) & 15u) == 0;
   constexpr int NT = 256;
-#define SPMX_HOLA_CASE(VT)                                                       \
-  case VT:                                                                       \
-    if (a.bits)                                                                  \
-      e = launch_l2_window(spmv_chunk_kernel<NT, VT, true>, dim3(t.nchunks), dim3(NT), 0, st, \
-          a.x, 4 * (size_t)a.n, a.m, a.n, a.nnz, a.rowptr, a.col, a.val, a.x, a.bits, \
-          a.alpha, a.y, (const int*)t.chunk_row, t.carry, t.arrive, vec_ok, a.err); \
-    else                                                                         \
-      e = launch_l2_window(spmv_chunk_kernel<NT, VT, false>, dim3(t.nchunks), dim3(NT), 0, st, \
-          a.x, 4 * (size_t)a.n, a.m, a.n, a.nnz, a.rowptr, a.col, a.val, a.x, a.bits, \
-          a.alpha, a.y, (const int*)t.chunk_row, t.carry, t.arrive, vec_ok, a.err); \
-    break;
+  // the chunks of short rows by their own kernel, the others by the scan; a
+  // matrix with few short chunks goes through the scan whole
+  const int nlong = t.nchunks - t.n_short;
+  const int4* list = t.n_short > 0 ? t.list + t.n_short : nullptr;
   cudaError_t e = cudaSuccess;
-  note_launch();
+#define SPMX_HOLA_CASE(VT)                                                       \
+  case VT: {                                                                     \
+    if (t.n_short > 0) {                                                         \
+      auto kernel = a.bits ? spmv_short_kernel<NT, VT, true> : spmv_short_kernel<NT, VT, false>; \
+      constexpr int smem = 16 * (NT * VT + kShortRow);                           \
+      e = kernel_smem_limit((const void*)kernel, smem);                          \
+      const int cap = 148 * std::min(1024 / NT, (227 << 10) / (smem + 1024));    \
+      const int rounds = (t.n_short + cap - 1) / cap;                            \
+      if (e == cudaSuccess)                                                      \
+        kernel<<<(t.n_short + rounds - 1) / rounds, NT, smem, st>>>(             \
+            a.n, a.nnz, a.rowptr, a.col, a.val, a.x, a.bits, a.alpha, a.y, t.list, t.n_short, nlong == 0, t.carry, \
+            t.arrive, a.err);                                                    \
+    }                                                                            \
+    if (nlong > 0) {                                         \
+      auto kernel = a.bits ? spmv_chunk_kernel<NT, VT, true> : spmv_chunk_kernel<NT, VT, false>; \
+      e = launch_l2_window(kernel, dim3(nlong), dim3(NT), 0, st, a.x, 4 * (size_t)a.n, a.m, a.n, a.nnz, \
+                           a.rowptr, a.col, a.val, a.x, a.bits, a.alpha, a.y, (const int*)t.chunk_row, list, \
+                           t.carry, t.arrive, vec_ok, a.err);                    \
+    }                                                                            \
+    break;                                                                       \
+  }
+  note_launch((t.n_short > 0) + (nlong > 0));
   switch (t.vt) {
     SPMX_HOLA_CASE(4)
     SPMX_HOLA_CASE(8)
     SPMX_HOLA_CASE(16)
     default: return -1;
   }
-  (void)e;
 #undef SPMX_HOLA_CASE
-  return 0;
+  return e == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace spmx
