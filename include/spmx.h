@@ -444,6 +444,12 @@ int spmx_spmv_backward_sparse(spmx_handle_t h, const float* d_x,
                               const int* d_dy_key, const float* d_dy_val,
                               int dy_nnz, float* d_dx, float* d_dvals);
 
+/* the dense-dy adjoint, or the sparse one where dy has fewer than `limit`
+ * nonzeros; decided on the device, nothing is read back.  d_scratch: 8 *
+ * min(limit, m) bytes, 4-byte aligned (unused for limit <= 0) */
+int spmx_spmv_backward_auto(spmx_handle_t h, const float* d_x, const float* d_dy,
+                            int limit, void* d_scratch, float* d_dx, float* d_dvals);
+
 /* ======================= batched SpMSpV (FP32) ============================= */
 /* No reference counterpart (the reference runs one vector per call).  nvec
  * (<= 1024) sparse vectors in one concatenated list: vector v owns entries

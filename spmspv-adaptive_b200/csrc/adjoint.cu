@@ -23,13 +23,18 @@
 
 namespace spmx {
 
+__device__ __forceinline__ bool gate_shut(const DevGate& g) {
+  return g.count && (__ldg(g.count) < g.limit) != g.below;
+}
+
 template <int NT, int VT>
 __global__ void __launch_bounds__(NT)
 spmv_backward_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
                      const int* __restrict__ col, const float* __restrict__ val,
                      const float* __restrict__ x, const float* __restrict__ dy,
                      const int* __restrict__ chunk_row, const int4* __restrict__ list, float* __restrict__ dx,
-                     float* __restrict__ dvals, int* err) {
+                     float* __restrict__ dvals, DevGate gate, int* err) {
+  if (gate_shut(gate)) return;
   constexpr int K = NT * VT;
   __shared__ int s_mark[K];
   __shared__ int s_incl[NT];
@@ -134,7 +139,9 @@ __global__ void __launch_bounds__(NT, 4)
 spmv_backward_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __restrict__ col,
                            const float* __restrict__ val, const float* __restrict__ x,
                            const float* __restrict__ dy, const int4* __restrict__ list, int count,
-                           float* __restrict__ dx, float* __restrict__ dvals, int vec_ok, int* err) {
+                           float* __restrict__ dx, float* __restrict__ dvals, int vec_ok, DevGate gate,
+                           int* err) {
+  if (gate_shut(gate)) return;
   constexpr int K = NT * VT;
   extern __shared__ __align__(16) unsigned char s_raw[];
   BackwardChunk<NT, VT>* const sh = reinterpret_cast<BackwardChunk<NT, VT>*>(s_raw);  // two of them
@@ -207,7 +214,8 @@ adjoint_csc_kernel(int m, int n, const int* __restrict__ rowptr, const int* __re
                    const int* __restrict__ colptr, const int* __restrict__ crow,
                    const float* __restrict__ cval, const float* __restrict__ x,
                    const float* __restrict__ dy, float* __restrict__ dx,
-                   float* __restrict__ dvals, int* err) {
+                   float* __restrict__ dvals, DevGate gate, int* err) {
+  if (gate_shut(gate)) return;
   const long long gid = (long long)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
   if ((blockIdx.x & 1) == 0) {
     if (!dx || gid / G1 >= ((long long)n + 31) / 32 * 32) return;  // whole warps past the end
@@ -248,32 +256,66 @@ adjoint_csc_kernel(int m, int n, const int* __restrict__ rowptr, const int* __re
   }
 }
 
+// G lanes per dy entry; with a gate the entry count is on the device
 template <int G>
 __global__ void __launch_bounds__(256)
 spmv_backward_sparse_kernel(int m, int n, const int* __restrict__ rowptr,
                             const int* __restrict__ col, const float* __restrict__ val,
                             const float* __restrict__ x, int dy_nnz,
                             const int* __restrict__ dy_key, const float* __restrict__ dy_val,
-                            float* __restrict__ dx, float* __restrict__ dvals, int* err) {
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(gid / G), g = (int)(gid % G);
-  if (i >= dy_nnz) return;
-  const int r = __ldg(dy_key + i);
-  if ((unsigned)r >= (unsigned)m) { if (g == 0) flag_error(err, kDevErrOob); return; }
-  const float d = __ldg(dy_val + i);
-  const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
-  for (int k = a + g; k < b; k += G) {
-    const int cc = __ldg(col + k);
-    if ((unsigned)cc >= (unsigned)n) { flag_error(err, kDevErrOob); continue; }
-    if (dvals) dvals[k] = d * __ldg(x + cc);
-    if (dx) atomicAdd(dx + cc, __ldg(val + k) * d);
+                            float* __restrict__ dx, float* __restrict__ dvals, DevGate gate, int* err) {
+  if (gate.count) {
+    dy_nnz = __ldg(gate.count);
+    if ((dy_nnz < gate.limit) != gate.below) return;
   }
+  const long long step = (long long)gridDim.x * blockDim.x / G;
+  const int g = (int)(threadIdx.x % G);
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G; i < dy_nnz; i += step) {
+    const int r = __ldg(dy_key + i);
+    if ((unsigned)r >= (unsigned)m) {
+      if (g == 0) flag_error(err, kDevErrOob);
+      continue;
+    }
+    const float d = __ldg(dy_val + i);
+    const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
+    for (int k = a + g; k < b; k += G) {
+      const int cc = __ldg(col + k);
+      if ((unsigned)cc >= (unsigned)n) { flag_error(err, kDevErrOob); continue; }
+      if (dvals) dvals[k] = d * __ldg(x + cc);
+      if (dx) atomicAdd(dx + cc, __ldg(val + k) * d);
+    }
+  }
+}
+
+__device__ __forceinline__ void clear_floats(float* p, long long len) {
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  const long long head = min(len, (long long)((16 - ((uintptr_t)p & 15)) & 15) / 4);  // up to the 16-byte boundary
+  const long long quads = (len - head) >> 2;
+  float4* p4 = reinterpret_cast<float4*>(p + head);
+  for (long long i = tid; i < quads; i += nt) p4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long long i = tid; i < head; i += nt) p[i] = 0.f;
+  for (long long i = head + 4 * quads + tid; i < len; i += nt) p[i] = 0.f;
+}
+
+__global__ void __launch_bounds__(256)
+backward_clear_kernel(int n, int nnz, float* dx, float* dvals, int dx_always, DevGate gate) {
+  const bool shut = gate_shut(gate);
+  if (dx && (dx_always || !shut)) clear_floats(dx, n);
+  if (dvals && !shut) clear_floats(dvals, nnz);
+}
+
+int launch_backward_clear(int n, int nnz, float* dx, float* dvals, bool dx_always, int num_sms, DevGate gate,
+                          cudaStream_t st) {
+  if (!dx && !dvals) return 0;
+  note_launch();
+  backward_clear_kernel<<<num_sms * 8, 256, 0, st>>>(n, nnz, dx, dvals, dx_always, gate);
+  return 0;
 }
 
 int launch_spmv_backward(int m, int n, int nnz, const int* rowptr, const int* col,
                          const float* val, const float* x, const float* dy,
                          const HolaTables& t, float* dx, float* dvals, int* err,
-                         cudaStream_t st) {
+                         DevGate gate, cudaStream_t st) {
   if (nnz <= 0 || t.nchunks == 0) return 0;
   if (t.K != 2048) return -1;  // the backward pass uses 256 x 8 chunks
   const int nlong = t.nchunks - t.n_short;
@@ -285,29 +327,31 @@ int launch_spmv_backward(int m, int n, int nnz, const int* rowptr, const int* co
     const int rounds = (t.n_short + 148 * 4 - 1) / (148 * 4);
     kernel<<<(t.n_short + rounds - 1) / rounds, 256, smem, st>>>(
         n, nnz, rowptr, col, val, x, dy, t.list, t.n_short, dx, dvals,
-        (((uintptr_t)col | (uintptr_t)val) & 15u) == 0, err);
+        (((uintptr_t)col | (uintptr_t)val) & 15u) == 0, gate, err);
   }
   if (nlong > 0)
     spmv_backward_kernel<256, 8><<<nlong, 256, 0, st>>>(m, n, nnz, rowptr, col, val, x, dy, t.chunk_row,
-                                                        t.n_short > 0 ? t.list + t.n_short : nullptr, dx, dvals, err);
+                                                        t.n_short > 0 ? t.list + t.n_short : nullptr, dx, dvals, gate,
+                                                 err);
   return 0;
 }
 
 template <int G1>
 static void adjoint_csc_g2(int g2, unsigned grid, cudaStream_t st, int m, int n, const int* rowptr,
                            const int* col, const int* colptr, const int* crow, const float* cval,
-                           const float* x, const float* dy, float* dx, float* dvals, int* err) {
+                           const float* x, const float* dy, float* dx, float* dvals, DevGate gate, int* err) {
   switch (g2) {
-    case 1: adjoint_csc_kernel<G1, 1><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 2: adjoint_csc_kernel<G1, 2><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 4: adjoint_csc_kernel<G1, 4><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    default: adjoint_csc_kernel<G1, 8><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
+    case 1: adjoint_csc_kernel<G1, 1><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 2: adjoint_csc_kernel<G1, 2><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 4: adjoint_csc_kernel<G1, 4><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    default: adjoint_csc_kernel<G1, 8><<<grid, 256, 0, st>>>(m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
   }
 }
 
 int launch_spmv_backward_csc(int m, int n, const int* rowptr, const int* col, const int* colptr,
                              const int* crow, const float* cval, const float* x, const float* dy,
-                             int g1, int g2, float* dx, float* dvals, int* err, cudaStream_t st) {
+                             int g1, int g2, float* dx, float* dvals, int* err, DevGate gate,
+                             cudaStream_t st) {
   if ((!dx || n <= 0) && (!dvals || m <= 0)) return 0;
   const long long t1 = dx ? ((long long)n + 31) / 32 * 32 * g1 : 0;
   const long long t2 = dvals ? (long long)m * g2 : 0;
@@ -315,14 +359,31 @@ int launch_spmv_backward_csc(int m, int n, const int* rowptr, const int* col, co
   const unsigned grid = (unsigned)(2 * half);
   note_launch();
   switch (g1) {
-    case 1: adjoint_csc_g2<1>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 2: adjoint_csc_g2<2>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 4: adjoint_csc_g2<4>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 8: adjoint_csc_g2<8>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    case 16: adjoint_csc_g2<16>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
-    default: adjoint_csc_g2<32>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, err); break;
+    case 1: adjoint_csc_g2<1>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 2: adjoint_csc_g2<2>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 4: adjoint_csc_g2<4>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 8: adjoint_csc_g2<8>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    case 16: adjoint_csc_g2<16>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
+    default: adjoint_csc_g2<32>(g2, grid, st, m, n, rowptr, col, colptr, crow, cval, x, dy, dx, dvals, gate, err); break;
   }
   return 0;
+}
+
+static void sparse_backward(int group, unsigned grid, cudaStream_t st, int m, int n, const int* rowptr,
+                            const int* col, const float* val, const float* x, int dy_nnz, const int* dy_key,
+                            const float* dy_val, float* dx, float* dvals, DevGate gate, int* err) {
+#define SPMX_SPARSE_BACKWARD(G) \
+  spmv_backward_sparse_kernel<G><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, gate, err)
+  note_launch();
+  switch (group) {
+    case 1: SPMX_SPARSE_BACKWARD(1); break;
+    case 2: SPMX_SPARSE_BACKWARD(2); break;
+    case 4: SPMX_SPARSE_BACKWARD(4); break;
+    case 8: SPMX_SPARSE_BACKWARD(8); break;
+    case 16: SPMX_SPARSE_BACKWARD(16); break;
+    default: SPMX_SPARSE_BACKWARD(32); break;
+  }
+#undef SPMX_SPARSE_BACKWARD
 }
 
 int launch_spmv_backward_sparse(int m, int n, const int* rowptr, const int* col,
@@ -330,17 +391,17 @@ int launch_spmv_backward_sparse(int m, int n, const int* rowptr, const int* col,
                                 const int* dy_key, const float* dy_val, int group,
                                 float* dx, float* dvals, int* err, cudaStream_t st) {
   if (dy_nnz <= 0) return 0;
-  const long long threads = (long long)dy_nnz * group;
-  const unsigned grid = (unsigned)((threads + 255) / 256);
-  note_launch();
-  switch (group) {
-    case 1: spmv_backward_sparse_kernel<1><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-    case 2: spmv_backward_sparse_kernel<2><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-    case 4: spmv_backward_sparse_kernel<4><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-    case 8: spmv_backward_sparse_kernel<8><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-    case 16: spmv_backward_sparse_kernel<16><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-    default: spmv_backward_sparse_kernel<32><<<grid, 256, 0, st>>>(m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, err); break;
-  }
+  const unsigned grid = (unsigned)(((long long)dy_nnz * group + 255) / 256);
+  sparse_backward(group, grid, st, m, n, rowptr, col, val, x, dy_nnz, dy_key, dy_val, dx, dvals, DevGate{}, err);
+  return 0;
+}
+
+int launch_spmv_backward_gated(int m, int n, const int* rowptr, const int* col, const float* val, const float* x,
+                               const int* dy_key, const float* dy_val, int group, float* dx, float* dvals,
+                               int num_sms, int* err, DevGate gate, cudaStream_t st) {
+  const long long want = ((long long)gate.limit * group + 255) / 256;
+  const unsigned grid = (unsigned)std::max(1LL, std::min<long long>(want, (long long)num_sms * 8));
+  sparse_backward(group, grid, st, m, n, rowptr, col, val, x, 0, dy_key, dy_val, dx, dvals, gate, err);
   return 0;
 }
 

@@ -812,33 +812,75 @@ extern "C" int spmx_spmspv(spmx_handle_t h, float alpha, float* y) {
 // adjoint of y = alpha*A*x: dx = alpha*A^T dy, dvals = alpha*dy[row]*x[col]
 // (alpha folded into dy by the caller's choice of dy; here alpha = 1)
 // ---------------------------------------------------------------------------
-extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* dy, float* dx,
-                                  float* dvals) {
-  SPMX_CHECK_HANDLE(h);
+static int backward_check(spmx_handle_t h, const float* x, const float* dy, float* dvals) {
   if (!h->has_csr || (!h->val && h->nnz > 0))
     return set_error(SPMX_ERR_NOT_READY, "backward needs the CSR input with values");
   if (!dy || (dvals && !x)) return set_error(SPMX_ERR_INVALID_VALUE, "NULL x / dy");
-  if (h->has_csc && (h->csc_val || h->nnz == 0)) {
+  return SPMX_SUCCESS;
+}
+
+static bool backward_by_csc(spmx_handle_t h) { return h->has_csc && (h->csc_val || h->nnz == 0); }
+
+// the dense-dy adjoint; without a CSC the caller has cleared dx
+static int backward_dense(spmx_handle_t h, const float* x, const float* dy, float* dx, float* dvals, DevGate gate) {
+  if (backward_by_csc(h)) {
     // dx = A^T dy as a gather over the CSC and dvals over the CSR, one launch
     const int g1 = h->naive_row_group > 0 ? h->naive_row_group
                                           : stream_group(h->n ? (double)h->nnz / h->n : 1.0);
     const int g2 = std::min(8, stream_group(h->m ? (double)h->nnz / h->m : 1.0));
     launch_spmv_backward_csc(h->m, h->n, h->rowptr, h->col, h->csc_colptr, h->csc_row, h->csc_val, x, dy, g1,
-                             g2, dx, h->nnz > 0 ? dvals : nullptr, h->d_err, h->stream);
+                             g2, dx, h->nnz > 0 ? dvals : nullptr, h->d_err, gate, h->stream);
     return launch_ok("spmv backward");
   }
-  if (!h->hola_ready || h->hola.K != 2048) {
-    const int vt = h->hola_vt;
-    h->hola_vt = 8;
-    const int rc = spmx_hola_preprocess(h);
-    h->hola_vt = vt;
-    SPMX_TRY(rc);
-  }
-  cudaStream_t st = h->stream;
-  if (dx) SPMX_CUDA(cudaMemsetAsync(dx, 0, 4 * (size_t)h->n, st));
   if (launch_spmv_backward(h->m, h->n, h->nnz, h->rowptr, h->col, h->val, x, dy, h->hola, dx,
-                           dvals, h->d_err, st))
+                           dvals, h->d_err, gate, h->stream))
     return set_error(SPMX_ERR_INVALID_VALUE, "backward chunk geometry");
+  return launch_ok("spmv backward");
+}
+
+// the Hola chunk table of the CSR-only adjoint, built on demand
+static int backward_tables(spmx_handle_t h) {
+  if (backward_by_csc(h) || (h->hola_ready && h->hola.K == 2048)) return SPMX_SUCCESS;
+  const int vt = h->hola_vt;
+  h->hola_vt = 8;
+  const int rc = spmx_hola_preprocess(h);
+  h->hola_vt = vt;
+  return rc;
+}
+
+extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* dy, float* dx,
+                                  float* dvals) {
+  SPMX_CHECK_HANDLE(h);
+  SPMX_TRY(backward_check(h, x, dy, dvals));
+  SPMX_TRY(backward_tables(h));
+  if (dx && !backward_by_csc(h)) SPMX_CUDA(cudaMemsetAsync(dx, 0, 4 * (size_t)h->n, h->stream));
+  return backward_dense(h, x, dy, dx, dvals, DevGate{});
+}
+
+// Both adjoints are launched behind the count of dy's nonzeros on the device, so
+// the host neither waits for it nor reads it (a read-back cost 25 us in a step
+// of 177); the one that does not apply returns at once.
+extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const float* dy, int limit, void* scratch,
+                                       float* dx, float* dvals) {
+  SPMX_CHECK_HANDLE(h);
+  SPMX_TRY(backward_check(h, x, dy, dvals));
+  limit = std::min(limit, h->m + 1);
+  if (limit <= 0 || h->m == 0) return spmx_spmv_backward(h, x, dy, dx, dvals);
+  SPMX_TRY(backward_tables(h));
+  if (!scratch) return set_error(SPMX_ERR_INVALID_VALUE, "scratch is NULL");
+  cudaStream_t st = h->stream;
+  int* key = (int*)scratch;
+  float* val = (float*)scratch + std::min(limit, h->m);
+  int* count = h->d_counts + kCntDy;
+  const DevGate sparse{count, limit, true}, dense{count, limit, false};
+  if (launch_compact_nonzero(h->m, dy, key, val, count, h->ls, h->d_err, st, limit))
+    return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
+  if (h->nnz == 0) dvals = nullptr;
+  launch_backward_clear(h->n, h->nnz, dx, dvals, !backward_by_csc(h), h->num_sms, sparse, st);
+  SPMX_TRY(backward_dense(h, x, dy, dx, dvals, dense));
+  const int g = pow2_group((double)h->nnz / h->m);
+  launch_spmv_backward_gated(h->m, h->n, h->rowptr, h->col, h->val, x, key, val, g, dx, dvals,
+                             h->num_sms, h->d_err, sparse, st);
   return launch_ok("spmv backward");
 }
 

@@ -42,18 +42,34 @@ int launch_chunk_rows(int m, int nnz, const int* rowptr, int K, int nchunks, int
                       int4* list, int* counts, cudaStream_t st);
 int hola_chunk_nnz(int vt);
 
+// A kernel that runs or returns at once by a count on the device: with `count`
+// set it runs where (*count < limit) == below.
+struct DevGate {
+  const int* count;
+  int limit;
+  bool below;
+};
+
 // ---- adjoint.cu
 int launch_spmv_backward(int m, int n, int nnz, const int* rowptr, const int* col,
                          const float* val, const float* x, const float* dy,
                          const HolaTables& t, float* dx, float* dvals, int* err,
-                         cudaStream_t st);
+                         DevGate gate, cudaStream_t st);
 int launch_spmv_backward_csc(int m, int n, const int* rowptr, const int* col, const int* colptr,
                              const int* crow, const float* cval, const float* x, const float* dy,
-                             int g1, int g2, float* dx, float* dvals, int* err, cudaStream_t st);
+                             int g1, int g2, float* dx, float* dvals, int* err, DevGate gate,
+                             cudaStream_t st);
 int launch_spmv_backward_sparse(int m, int n, const int* rowptr, const int* col,
                                 const float* val, const float* x, int dy_nnz,
                                 const int* dy_key, const float* dy_val, int group,
                                 float* dx, float* dvals, int* err, cudaStream_t st);
+// the same for a compacted dy of *gate.count entries
+int launch_spmv_backward_gated(int m, int n, const int* rowptr, const int* col, const float* val, const float* x,
+                               const int* dy_key, const float* dy_val, int group, float* dx, float* dvals,
+                               int num_sms, int* err, DevGate gate, cudaStream_t st);
+// dx = 0 and dvals = 0 behind the gate; dx behind no gate where dx_always
+int launch_backward_clear(int n, int nnz, float* dx, float* dvals, bool dx_always, int num_sms, DevGate gate,
+                          cudaStream_t st);
 
 // ---- lookback scratch shared by the single-pass scans
 struct ScanScratch {
@@ -71,6 +87,7 @@ enum CounterSlot : int {
   kCntBlocksTL = 3,
   kCntBlocksMG = 4,
   kCntLong = 5,        // chunks of long columns
+  kCntDy = 6,          // nonzeros of the adjoint's dy
   kCntFeatSum = 8,   // 64-bit (slots 8..9)
   kCntFeatMax = 10,
   kCntFeatMinInv = 11,
@@ -140,9 +157,10 @@ int launch_dense_from_sparse(int nvals, int len, const int* key, const float* va
 int launch_scatter(int nvals, int len, const int* key, const float* val,
                    float* dense, int* bits, int* err, cudaStream_t st);
 int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st);
-// keys/vals of the entries != 0 of dense[0..len), in order; count -> *d_count
+// keys/vals of the entries != 0 of dense[0..len), in order; count -> *d_count.
+// limit > 0: nothing but the count is written where it reaches the limit
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
                            int* d_count, ScanScratch& ls, int* err,
-                           cudaStream_t st);
+                           cudaStream_t st, int limit = 0);
 
 }  // namespace spmx

@@ -100,7 +100,7 @@ template <int NT, int VT>
 __global__ void __launch_bounds__(NT)
 compact_write_kernel(long long len, long long per, const float* __restrict__ dense,
                      const unsigned* __restrict__ counts, int* __restrict__ key,
-                     float* __restrict__ val, int* d_count) {
+                     float* __restrict__ val, int* d_count, unsigned limit) {
   constexpr int NW = NT / 32;
   __shared__ unsigned s_cnt[VT * NW];
   __shared__ unsigned s_wtmp[NW + 1];
@@ -119,9 +119,26 @@ compact_write_kernel(long long len, long long per, const float* __restrict__ den
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
-  // nonzeros before this range
-  unsigned pre = 0;
-  for (int t = tid; t < (int)blockIdx.x; t += NT) pre += __ldcg(counts + t);
+  // nonzeros before this range, and in all
+  unsigned pre = 0, all = 0;
+  for (int t = tid; t < (limit ? (int)gridDim.x : (int)blockIdx.x); t += NT) {
+    const unsigned c = __ldcg(counts + t);
+    all += c;
+    if (t < (int)blockIdx.x) pre += c;
+  }
+  if (limit) {
+    all = warp_sum(all);
+    if (lane == 0) s_red[w] = all;
+    __syncthreads();
+    all = 0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) all += s_red[q];
+    if (all >= limit) {
+      if (blockIdx.x == 0 && tid == 0) *d_count = (int)all;
+      return;
+    }
+    __syncthreads();
+  }
   pre = warp_sum(pre);
   if (lane == 0) s_red[w] = pre;
   __syncthreads();
@@ -209,7 +226,7 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st) {
 
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
                            int* d_count, ScanScratch& ls, int* err,
-                           cudaStream_t st) {
+                           cudaStream_t st, int limit) {
   constexpr int NT = 256, VT = 8;
   (void)err;
   if (len <= 0) { cudaMemsetAsync(d_count, 0, sizeof(int), st); return 0; }
@@ -223,7 +240,7 @@ int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
   if (launch_pdl(compact_count_kernel<NT, VT>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per,
                  dense, ls.counts) != cudaSuccess ||
       launch_pdl(compact_write_kernel<NT, VT>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per,
-                 dense, (const unsigned*)ls.counts, key, val, d_count) != cudaSuccess)
+                 dense, (const unsigned*)ls.counts, key, val, d_count, (unsigned)limit) != cudaSuccess)
     return -2;
   return 0;
 }

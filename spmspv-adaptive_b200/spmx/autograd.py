@@ -10,6 +10,8 @@ in dy's support are touched (the CSC SpMSpV of A^T).
 
 No reference counterpart: the reference has no differentiation.
 """
+import math
+
 import torch
 
 from .handle import SpmspvHandle
@@ -20,8 +22,8 @@ class SparseMatrix:
 
     rowptr: int32 [m+1], col: int32 [nnz] (CUDA tensors).  `sparse_grad`:
     "auto" compacts dy on the device and takes the sparse adjoint when fewer
-    than `sparse_threshold` * m rows are nonzero (this reads one count back to
-    the host); "dense" / "sparse" force a path.
+    than `sparse_threshold` * m rows are nonzero (decided on the device);
+    "dense" / "sparse" force a path.
     """
 
     def __init__(self, m, n, rowptr, col, sparse_grad="auto", sparse_threshold=0.05):
@@ -70,12 +72,13 @@ class SpMVFunction(torch.autograd.Function):
         dvals = torch.empty_like(vals) if need_vals else None
         dx = torch.empty_like(x) if need_x else None
         mode = op.sparse_grad
-        if mode != "dense":
-            key = torch.empty(op.m, dtype=torch.int32, device=dy.device)
-            val = torch.empty(op.m, dtype=torch.float32, device=dy.device)
-            cnt = op.h.dense2sparse_outer(op.m, dy, key, val)
-            if mode == "sparse" or cnt < op.sparse_threshold * op.m:
-                op.h.spmv_backward_sparse(x, key, val, cnt, dx, dvals)
-                return dvals, dx, None
-        op.h.spmv_backward(x, dy, dx, dvals)
+        if mode == "dense":
+            op.h.spmv_backward(x, dy, dx, dvals)
+        else:
+            limit = op.m + 1 if mode == "sparse" else min(math.ceil(op.sparse_threshold * op.m), op.m + 1)
+            # nothing waits for the handle's stream here: a dy that another
+            # stream's allocator may hand out again is kept until it has been read
+            if torch.cuda.current_stream(dy.device) != op.h.stream:
+                dy.record_stream(op.h.stream)
+            op.h.spmv_backward_auto(x, dy, limit, dx, dvals)
         return dvals, dx, None

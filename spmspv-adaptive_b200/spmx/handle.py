@@ -62,6 +62,10 @@ class SpmspvHandle:
         self._stream = stream
         check(lib.spmx_set_stream(self._h, stream.cuda_stream), "set_stream")
 
+    @property
+    def stream(self):
+        return self._stream
+
     def warmup(self):
         check(lib.spmx_warmup(self._h), "warmup")
 
@@ -458,6 +462,17 @@ class SpmspvHandle:
         check(lib.spmx_spmv_backward_sparse(self._h, _f32(x), _i32(dy_key), _f32(dy_val),
                                             int(dy_nnz), _f32(dx), _f32(dvals)),
               "spmv_backward_sparse")
+
+    def spmv_backward_auto(self, x, dy, limit, dx=None, dvals=None):
+        """spmv_backward, or the sparse adjoint where dy has fewer than `limit`
+        nonzeros; decided on the device."""
+        limit = min(int(limit), self.m + 1)
+        tmp = torch.empty(2 * min(limit, self.m), dtype=torch.float32, device=dy.device) if limit > 0 else None
+        if tmp is not None and torch.cuda.current_stream(dy.device) != self._stream:
+            tmp.record_stream(self._stream)
+        check(lib.spmx_spmv_backward_auto(self._h, _f32(x), _f32(dy), limit,
+                                          tmp.data_ptr() if limit > 0 else None, _f32(dx), _f32(dvals)),
+              "spmv_backward_auto")
 
     # -- batched SpMSpV (no reference counterpart) ------------------------------
     def set_batch_options(self, flags):
