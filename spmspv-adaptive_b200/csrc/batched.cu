@@ -51,6 +51,10 @@ constexpr int kBatchMaxVec = 1024;  // nvec limit (shared row accumulators)
 // warp in the first pass of a cyclic assignment.
 constexpr int kBatchChunk = 2048;
 constexpr int kBatchRowCost = 32;
+// Rows above this are taken by whole CTAs before the row walk starts: one warp
+// alone on a hub row (10,000 nonzeros, 300 dependent steps) was the tail of the
+// walk, 0.55 ms of 1.2 ms on a 1M-vertex Chung-Lu graph.
+constexpr int kBatchHubRow = 512;
 
 // sort keys (column) and payloads (entry, vector) of every batch entry
 __global__ void batch_keys_kernel(int n, int nvec, int total, const int* __restrict__ xptr,
@@ -102,6 +106,23 @@ __global__ void batch_chunks_kernel(int m, const int* __restrict__ rowptr, int n
   chunk_row[k] = lo;
 }
 
+// the rows above kBatchHubRow, in any order; *count has their number
+__global__ void batch_hubs_kernel(int m, const int* __restrict__ rowptr, int* __restrict__ hub_row, int* count) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+    if (__ldg(rowptr + i + 1) - __ldg(rowptr + i) > kBatchHubRow) hub_row[atomicAdd(count, 1)] = i;
+}
+
+// the CTA's next hub row (-1: none left); whole CTA
+__device__ __forceinline__ int batch_next_hub(int* ctr, const int* hub_row, const int* nhub, int* s_hub) {
+  __syncthreads();  // the previous hub's shared rows are no longer read
+  if (threadIdx.x == 0) {
+    const int c = atomicAdd(ctr, 1);
+    *s_hub = c < *nhub ? hub_row[c] : -1;
+  }
+  __syncthreads();
+  return *s_hub;
+}
+
 // A warp's rows, chunk by chunk: the next chunk is taken from the counter one
 // chunk ahead (lane 0's atomic, broadcast), so its bounds are in registers by
 // the time the current chunk runs out.  next() returns m once the chunks are
@@ -151,11 +172,8 @@ __global__ void batch_rec_kernel(int total, const unsigned* __restrict__ inv_ent
 // that column's pair range in flight, the head of the row after in flight
 // and the bounds of the third in flight, so only the pair-record loads stay
 // on the critical path of a row's first 32 nonzeros.  The dvals walk takes its
-// rows from the chunks too, one row shallower (the next row's head and dY
-// row, the bounds of the row after).  The dvals walk, which also holds the next row of dY in
-// registers, runs one row shallower (row i + nw's head, row i + 2nw's
-// bounds): the deeper form needs 64 registers there and loses more to the
-// lower occupancy than it gains.
+// rows from the chunks too, one row shallower (the next row's head and dY row,
+// the bounds of the row after).
 struct BatchRowHead {
   int a0, a1;  // row bounds
   int j;       // the lane's first column (a0 + lane), valid if has
@@ -197,17 +215,36 @@ __device__ __forceinline__ void batch_head_pairs(BatchRowHead& h, const int* __r
   }
 }
 
-// acc[v] += a * x over the pairs [p0, p1), two records in flight at a time
+constexpr int kBatchU = 4;  // pair records in flight per lane
+
+// acc[v] += a * x over the pairs [p0, p1)
 __device__ __forceinline__ void batch_add_pairs(float* acc, const int2* __restrict__ rec, int p0, int p1, float a) {
-  int p = p0;
-  for (; p + 1 < p1; p += 2) {
-    const int2 e = __ldg(rec + p), f = __ldg(rec + p + 1);
-    atomicAdd(acc + e.x, a * __int_as_float(e.y));
-    atomicAdd(acc + f.x, a * __int_as_float(f.y));
+  for (int p = p0; p < p1; p += kBatchU) {
+    int2 e[kBatchU];
+#pragma unroll
+    for (int u = 0; u < kBatchU; ++u)
+      if (p + u < p1) e[u] = __ldg(rec + p + u);
+#pragma unroll
+    for (int u = 0; u < kBatchU; ++u)
+      if (p + u < p1) atomicAdd(acc + e[u].x, a * __int_as_float(e[u].y));
   }
-  if (p < p1) {
-    const int2 e = __ldg(rec + p);
-    atomicAdd(acc + e.x, a * __int_as_float(e.y));
+}
+
+// acc += the nonzeros k, k + step, ... < a1 times their pairs, two per lane at a time
+__device__ __forceinline__ void batch_add_row(float* acc, const int* __restrict__ col,
+                                              const float* __restrict__ val,
+                                              const int* __restrict__ invptr, const int2* __restrict__ rec, int n,
+                                              int k, int a1, int step, int* err) {
+  for (; k < a1; k += 2 * step) {
+    const bool two = k + step < a1;
+    const int j0 = __ldg(col + k), j1 = two ? __ldg(col + k + step) : 0;
+    const float v0 = __ldg(val + k), v1 = two ? __ldg(val + k + step) : 0.f;
+    const bool ok0 = (unsigned)j0 < (unsigned)n, ok1 = two && (unsigned)j1 < (unsigned)n;
+    if (!ok0 || (two && !ok1)) flag_error(err, kDevErrOob);
+    const int q00 = ok0 ? __ldg(invptr + j0) : 0, q01 = ok0 ? __ldg(invptr + j0 + 1) : 0;
+    const int q10 = ok1 ? __ldg(invptr + j1) : 0, q11 = ok1 ? __ldg(invptr + j1 + 1) : 0;
+    batch_add_pairs(acc, rec, q00, q01, v0);
+    batch_add_pairs(acc, rec, q10, q11, v1);
   }
 }
 
@@ -216,12 +253,29 @@ __global__ void __launch_bounds__(kBatchWarps * 32)
 batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const int* __restrict__ col,
                      const float* __restrict__ val, const int* __restrict__ invptr,
                      const int2* __restrict__ rec, float alpha, float* __restrict__ Y, int vec4,
-                     const int* __restrict__ chunk_row, int nch, int* ctr, int* err) {
+                     const int* __restrict__ chunk_row, int nch, const int* __restrict__ hub_row,
+                     const int* __restrict__ nhub, int* ctr, int* err) {
   extern __shared__ __align__(16) float s_acc[];  // kBatchWarps rows of nvec
+  __shared__ int s_hub;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* acc = s_acc + warp * nvec;
   for (int v = lane; v < nvec; v += 32) acc[v] = 0.f;
   __syncwarp();
+  // hub rows: the warps share the row's nonzeros, then its accumulators are added up
+  for (int i; (i = batch_next_hub(ctr + 1, hub_row, nhub, &s_hub)) >= 0;) {
+    const int a1 = __ldg(rowptr + i + 1);
+    batch_add_row(acc, col, val, invptr, rec, n, __ldg(rowptr + i) + warp * 32 + lane, a1, kBatchWarps * 32, err);
+    __syncthreads();
+    for (int v = threadIdx.x; v < nvec; v += kBatchWarps * 32) {
+      float t = 0.f;
+#pragma unroll
+      for (int w = 0; w < kBatchWarps; ++w) {
+        t += s_acc[w * nvec + v];
+        s_acc[w * nvec + v] = 0.f;
+      }
+      Y[(size_t)i * nvec + v] = alpha * t;
+    }
+  }
   BatchRowIter it;
   it.init(ctr, nch, chunk_row, m, lane);
   int i = it.next(ctr, nch, chunk_row, m, lane);  // this row, then the next three of the warp
@@ -241,22 +295,15 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
     const int i3 = it.next(ctr, nch, chunk_row, m, lane);
     int c0, c1;
     batch_row_bounds(rowptr, m, i3, c0, c1);
+    const bool hub = cur.a1 - cur.a0 > kBatchHubRow;  // done above (warp-uniform)
+    if (hub) cur.p1 = cur.p0, cur.a1 = cur.a0;
     batch_add_pairs(acc, rec, cur.p0, cur.p1, cur.a);
-    // the row's nonzeros past the first 32, two per lane at a time
-    for (int k = cur.a0 + 32 + lane; k < cur.a1; k += 64) {
-      const bool two = k + 32 < cur.a1;
-      const int j0 = __ldg(col + k), j1 = two ? __ldg(col + k + 32) : 0;
-      const float v0 = __ldg(val + k), v1 = two ? __ldg(val + k + 32) : 0.f;
-      const bool ok0 = (unsigned)j0 < (unsigned)n, ok1 = two && (unsigned)j1 < (unsigned)n;
-      if (!ok0 || (two && !ok1)) flag_error(err, kDevErrOob);
-      const int q00 = ok0 ? __ldg(invptr + j0) : 0, q01 = ok0 ? __ldg(invptr + j0 + 1) : 0;
-      const int q10 = ok1 ? __ldg(invptr + j1) : 0, q11 = ok1 ? __ldg(invptr + j1 + 1) : 0;
-      batch_add_pairs(acc, rec, q00, q01, v0);
-      batch_add_pairs(acc, rec, q10, q11, v1);
-    }
+    // the row's nonzeros past the first 32
+    batch_add_row(acc, col, val, invptr, rec, n, cur.a0 + 32 + lane, cur.a1, 32, err);
     __syncwarp();
     float* yr = Y + (size_t)i * nvec;
-    if (vec4) {  // nvec % 4 == 0 and Y 16-byte aligned (checked on the host): vector stores
+    if (hub) {
+    } else if (vec4) {  // nvec % 4 == 0 and Y 16-byte aligned (checked on the host): vector stores
       float4* y4 = reinterpret_cast<float4*>(yr);
       float4* a4 = reinterpret_cast<float4*>(acc);
       for (int v = lane; v < (nvec >> 2); v += 32) {
@@ -287,15 +334,50 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
 // dxval[e] with an atomic add.  The same pipeline as the forward; for
 // nvec <= 256 with 16-byte rows (pre) each warp has two shared dY rows, and
 // the next row of dY is copied into the other one (cp.async, no registers
-// held) while this row is walked.
-__global__ void __launch_bounds__(kBatchWarps * 32, 5)
+// held) while this row is walked.  Four records in flight per lane at 64
+// registers and 4 CTAs per SM: 1.19 ms on the 1M-vertex Chung-Lu graph with 256
+// vectors; two at 4 CTAs 1.22, two at 5 CTAs (48 registers, spills) 1.37.
+template <bool FUSED>
+__global__ void __launch_bounds__(kBatchWarps * 32, 4)
 batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const int* __restrict__ col,
                    const int* __restrict__ invptr, const int4* __restrict__ rec, float alpha,
                    const float* __restrict__ dY, float* __restrict__ dvals, const float* __restrict__ val,
-                   float* __restrict__ dxval, int vec4, const int* __restrict__ chunk_row, int nch, int* ctr,
-                   int* err) {
+                   float* __restrict__ dxval, int vec4, const int* __restrict__ chunk_row, int nch,
+                   const int* __restrict__ hub_row, const int* __restrict__ nhub, int* ctr, int* err) {
   extern __shared__ __align__(16) float s_dy[];
+  __shared__ int s_hub;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const auto nonzero = [&](int k, int j, float va, const float* g) {
+    float s = 0.f;
+    if ((unsigned)j < (unsigned)n) {
+      const int q1 = __ldg(invptr + j + 1);
+      const float a = FUSED ? alpha * va : 0.f;
+      for (int p = __ldg(invptr + j); p < q1; p += kBatchU) {
+        int4 r[kBatchU];
+#pragma unroll
+        for (int u = 0; u < kBatchU; ++u)
+          if (p + u < q1) r[u] = __ldg(rec + p + u);
+#pragma unroll
+        for (int u = 0; u < kBatchU; ++u) {
+          if (p + u >= q1) continue;
+          const float gv = g[r[u].x];
+          s += __int_as_float(r[u].y) * gv;
+          if (FUSED) atomicAdd(dxval + r[u].z, a * gv);
+        }
+      }
+    } else {
+      flag_error(err, kDevErrOob);
+    }
+    dvals[k] = alpha * s;
+  };
+  // hub rows: the warps share the row's nonzeros and its dY in the first shared row
+  for (int i; (i = batch_next_hub(ctr + 1, hub_row, nhub, &s_hub)) >= 0;) {
+    for (int v = threadIdx.x; v < nvec; v += kBatchWarps * 32) s_dy[v] = __ldg(dY + (size_t)i * nvec + v);
+    __syncthreads();
+    const int a1 = __ldg(rowptr + i + 1);
+    for (int k = __ldg(rowptr + i) + threadIdx.x; k < a1; k += kBatchWarps * 32)
+      nonzero(k, __ldg(col + k), FUSED ? __ldg(val + k) : 0.f, s_dy);
+  }
   const bool pre = vec4 && nvec <= 256;  // two shared dY rows per warp (the host sizes them)
   float* const g0 = s_dy + (size_t)warp * (pre ? 2 : 1) * nvec;
   const int n4 = nvec >> 2;
@@ -315,7 +397,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
   it.init(ctr, nch, chunk_row, m, lane);
   int i = it.next(ctr, nch, chunk_row, m, lane);  // this row and the warp's next
   int i1 = it.next(ctr, nch, chunk_row, m, lane);
-  const float* aval = dxval ? val : nullptr;
+  const float* aval = FUSED ? val : nullptr;
   int b0, b1;
   batch_row_bounds(rowptr, m, i, b0, b1);
   BatchRowHead cur = batch_row_head(col, aval, b0, b1, lane);
@@ -328,7 +410,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     const int i2 = it.next(ctr, nch, chunk_row, m, lane);
     int c0, c1;
     batch_row_bounds(rowptr, m, i2, c0, c1);
-    if (cur.a0 < cur.a1) {  // warp-uniform
+    if (cur.a0 < cur.a1 && cur.a1 - cur.a0 <= kBatchHubRow) {  // warp-uniform
       float* const g = g0 + (pre ? buf * nvec : 0);
       if (pre) {
         cp_async_wait<1>();  // every group but the next row's: this row's dY has landed
@@ -341,21 +423,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
       __syncwarp();
       for (int k = cur.a0 + lane; k < cur.a1; k += 32) {
         const bool first = k == cur.a0 + lane;
-        const int j = first ? cur.j : __ldg(col + k);
-        float s = 0.f;
-        if ((unsigned)j < (unsigned)n) {
-          const int q1 = __ldg(invptr + j + 1);
-          const float a = dxval ? alpha * (first ? cur.a : __ldg(val + k)) : 0.f;
-          for (int p = __ldg(invptr + j); p < q1; ++p) {
-            const int4 r = __ldg(rec + p);
-            const float gv = g[r.x];
-            s += __int_as_float(r.y) * gv;
-            if (dxval) atomicAdd(dxval + r.z, a * gv);
-          }
-        } else {
-          flag_error(err, kDevErrOob);
-        }
-        dvals[k] = alpha * s;
+        nonzero(k, first ? cur.j : __ldg(col + k), first ? cur.a : FUSED ? __ldg(val + k) : 0.f, g);
       }
       __syncwarp();
     }
@@ -509,7 +577,12 @@ static int ensure_batch_chunks(spmx_handle_t h) {
     h->batch_chunk = nullptr;
     SPMX_TRY(dalloc((void**)&h->batch_chunk, 4 * ((size_t)nch + 1), "batch row chunks"));
   }
-  if (!h->batch_ctr) SPMX_TRY(dalloc((void**)&h->batch_ctr, 2 * sizeof(int), "batch chunk counters"));
+  if (!h->batch_ctr) SPMX_TRY(dalloc((void**)&h->batch_ctr, 5 * sizeof(int), "batch chunk counters"));
+  if (!h->batch_hub)
+    SPMX_TRY(dalloc((void**)&h->batch_hub, 4 * ((size_t)h->nnz / (kBatchHubRow + 1) + 1), "batch hub rows"));
+  SPMX_CUDA(cudaMemsetAsync(h->batch_ctr + 4, 0, sizeof(int), h->stream));
+  note_launch();
+  batch_hubs_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->m, h->rowptr, h->batch_hub, h->batch_ctr + 4);
   note_launch();
   batch_chunks_kernel<<<(unsigned)((nch + 1 + 255) / 256), 256, 0, h->stream>>>(h->m, h->rowptr, (int)nch,
                                                                                 h->batch_chunk);
@@ -551,7 +624,7 @@ extern "C" int spmx_spmspv_batched(spmx_handle_t h, int nvec, int x_total, const
   SPMX_TRY(batch_invert(h, nvec, x_total, d_xptr, d_xkey, d_xval, true, &ie, &rec, &rec4));
   if (h->m == 0) return SPMX_SUCCESS;
   SPMX_TRY(ensure_batch_chunks(h));
-  SPMX_CUDA(cudaMemsetAsync(h->batch_ctr, 0, sizeof(int), h->stream));
+  SPMX_CUDA(cudaMemsetAsync(h->batch_ctr, 0, 2 * sizeof(int), h->stream));
   const size_t smem = 4 * (size_t)kBatchWarps * nvec;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(batch_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -559,7 +632,7 @@ extern "C" int spmx_spmspv_batched(spmx_handle_t h, int nvec, int x_total, const
   batch_forward_kernel<<<batch_rows_grid(h, (const void*)batch_forward_kernel, smem), kBatchWarps * 32, smem,
                          h->stream>>>(h->m, h->n, nvec, h->rowptr, h->col, h->val, h->batch_invptr, rec,
                                       alpha, d_Y, (nvec % 4 == 0 && ((uintptr_t)d_Y & 15u) == 0) ? 1 : 0,
-                                      h->batch_chunk, h->batch_nch, h->batch_ctr, h->d_err);
+                                      h->batch_chunk, h->batch_nch, h->batch_hub, h->batch_ctr + 4, h->batch_ctr, h->d_err);
   return launch_ok("batched spmspv");
 }
 
@@ -580,17 +653,16 @@ extern "C" int spmx_spmspv_batched_backward(spmx_handle_t h, int nvec, int x_tot
     const int4* rec4 = nullptr;
     SPMX_TRY(batch_invert(h, nvec, x_total, d_xptr, d_xkey, d_xval, false, &ie, &rec, &rec4));
     SPMX_TRY(ensure_batch_chunks(h));
-    SPMX_CUDA(cudaMemsetAsync(h->batch_ctr + 1, 0, sizeof(int), st));
+    SPMX_CUDA(cudaMemsetAsync(h->batch_ctr + 2, 0, 2 * sizeof(int), st));
     const bool vec4 = nvec % 4 == 0 && ((uintptr_t)d_dY & 15u) == 0;
     // with 16-byte rows of at most 256 entries each warp double-buffers its dY row
     const size_t smem = 4 * (size_t)kBatchWarps * nvec * (vec4 && nvec <= 256 ? 2 : 1);
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(batch_dvals_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = fused ? batch_dvals_kernel<true> : batch_dvals_kernel<false>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     note_launch();
-    batch_dvals_kernel<<<batch_rows_grid(h, (const void*)batch_dvals_kernel, smem), kBatchWarps * 32, smem,
-                         st>>>(h->m, h->n, nvec, h->rowptr, h->col, h->batch_invptr, rec4, alpha,
+    kernel<<<batch_rows_grid(h, (const void*)kernel, smem), kBatchWarps * 32, smem, st>>>(h->m, h->n, nvec, h->rowptr, h->col, h->batch_invptr, rec4, alpha,
                                d_dY, d_dvals, h->val, fused ? d_dxval : nullptr, vec4 ? 1 : 0, h->batch_chunk,
-                               h->batch_nch, h->batch_ctr + 1, h->d_err);
+                               h->batch_nch, h->batch_hub, h->batch_ctr + 4, h->batch_ctr + 2, h->d_err);
   }
   if (d_dxval && x_total > 0 && !fused) {
     if (!h->has_csc || !h->csc_val)

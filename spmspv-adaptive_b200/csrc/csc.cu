@@ -492,7 +492,7 @@ namespace spmx {
 int csc_lb_blocks_per_sm() {
   int b = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &b, csc_lb_kernel<kCscLbNT, kCscLbVT, true>, kCscLbNT, 0) != cudaSuccess) {
+          &b, csc_lb_kernel<kCscLbNT, kCscLbVT, false>, kCscLbNT, 0) != cudaSuccess) {
     cudaGetLastError();
     return 2;
   }

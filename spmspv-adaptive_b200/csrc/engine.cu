@@ -301,7 +301,7 @@ extern "C" int spmx_destroy(spmx_handle_t h) {
   dfree(h->ms_hchunk); dfree(h->ms_hvert); dfree(h->ms_hacc); dfree(h->ms_hcounters);
   for (void* p : h->batch_buf) dfree(p);
   dfree(h->batch_radix); dfree(h->batch_invptr); dfree(h->batch_rec);
-  dfree(h->batch_chunk); dfree(h->batch_ctr);
+  dfree(h->batch_chunk); dfree(h->batch_ctr); dfree(h->batch_hub);
   pool_leave(h->device);
   delete h;
   return SPMX_SUCCESS;

@@ -140,7 +140,10 @@ struct spmx_handle_s {
   int* batch_chunk = nullptr;
   int batch_nch = 0;
   bool batch_chunk_ready = false;
-  int* batch_ctr = nullptr;  // [0] the forward walk's chunk counter, [1] the dvals walk's
+  // [0] the forward walk's chunk counter, [1] its hub counter, [2] [3] the dvals
+  // walk's, [4] number of hub rows
+  int* batch_ctr = nullptr;
+  int* batch_hub = nullptr;  // rows above kBatchHubRow nonzeros
   // hub chunks of the multi-source pull (built once per matrix)
   int4* ms_hchunk = nullptr;
   int* ms_hvert = nullptr;
