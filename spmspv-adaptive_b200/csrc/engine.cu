@@ -223,7 +223,7 @@ extern "C" int spmx_create(int m, int n, int nnz, spmx_handle_t* out) {
   rc = rc ? rc : dalloc((void**)&h->d_iacc, sizeof(int) * 4, "iacc");
   rc = rc ? rc : dalloc((void**)&h->d_u64, sizeof(unsigned long long) * 4, "u64");
   const long long big = std::max<long long>(std::max<long long>(m, n), nnz);
-  h->ls.status_len = (int)(big / 2048 + 4);
+  h->ls.status_len = (int)(std::max<long long>(big / 2048, n / 512) + 4);
   rc = rc ? rc : dalloc((void**)&h->ls.status, sizeof(unsigned long long) * h->ls.status_len,
                         "lookback status");
   rc = rc ? rc : dalloc((void**)&h->ls.ticket, sizeof(unsigned) * 4, "ticket");
@@ -254,6 +254,9 @@ static void free_sort_scratch(spmx_handle_t h) {
   dfree(h->sradix); dfree(h->sslot);
   dfree(h->sy_key); dfree(h->sy_val);
   dfree(h->bk_gcount); dfree(h->bk_boff); dfree(h->bk_cursor);
+  dfree(h->bk_tab);
+  h->bk_tab = nullptr;
+  h->bk_tab_nb = 0;
   h->bk_gcount = h->bk_boff = h->bk_cursor = nullptr;
   h->sk = h->sk_alt = h->sv = h->sv_alt = nullptr;
   h->sradix = nullptr;
@@ -676,10 +679,24 @@ static int ensure_csc_scratch(spmx_handle_t h) {
   return SPMX_SUCCESS;
 }
 
+// the bucket offsets of every block, for at most kBucketTable buckets
+static int ensure_bucket_table(spmx_handle_t h, int nb) {
+  if (nb > kBucketTable || nb <= h->bk_tab_nb) return SPMX_SUCCESS;
+  SPMX_CUDA(cudaStreamSynchronize(h->stream));
+  dfree(h->bk_tab);
+  h->bk_tab = nullptr;
+  h->bk_tab_nb = 0;
+  SPMX_TRY(dalloc((void**)&h->bk_tab, 2 * ((size_t)nb + 1) * h->cs.mg_cap, "bucket table"));
+  h->bk_tab_nb = nb;
+  return SPMX_SUCCESS;
+}
+
 extern "C" int spmx_alloc_pre_buffer(spmx_handle_t h) {
   SPMX_CHECK_HANDLE(h);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
+  int rshift = 0, nb = 0;
+  if (!bucket_geometry(h->m, h->buckets, &rshift, &nb)) SPMX_TRY(ensure_bucket_table(h, nb));
   SPMX_TRY(ensure_dense_x(h));
   SPMX_TRY(ensure_bits(h));
   return SPMX_SUCCESS;
@@ -945,7 +962,7 @@ static int csc_sort(spmx_handle_t h, int variant, float alpha, float* y, int* yk
   const CscArgs a = csc_args(h, alpha);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
-  if (launch_csc_scan(a, h->cs, h->ls, kCscLbNT * kCscLbVT, st))
+  if (launch_csc_scan(a, h->cs, h->ls, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "scan capacity");
   // the pair count sizes the sort launches (the reference reads it back too,
   // DEV/csc_sort_spmspv.cuh:266)
@@ -1063,11 +1080,13 @@ int csc_bucket_impl(spmx_handle_t h, float alpha, float* y, int* ykey, float* yv
   if (bucket_geometry(h->m, buckets > 0 ? buckets : h->buckets, &rshift, &nb))
     return set_error(SPMX_ERR_INVALID_VALUE, "too many rows for the bucket method");
   SPMX_TRY(ensure_scan_tiles(h, nb));
+  SPMX_TRY(ensure_bucket_table(h, nb));
   cudaStream_t st = h->stream;
   const CscArgs a = csc_args(h, alpha);
-  if (launch_csc_scan(a, h->cs, h->ls, kCscLbNT * kCscLbVT, st))
+  if (launch_csc_scan(a, h->cs, h->ls, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "scan capacity");
-  BucketScratch bs{h->bk_gcount, h->bk_boff, h->bk_cursor, (int*)h->sk, (float*)h->sv, h->nnz};
+  BucketScratch bs{h->bk_gcount, h->bk_boff, h->bk_cursor, (int*)h->sk, (float*)h->sv, h->nnz,
+                   h->bk_tab};
   if (launch_bucket_spmspv(a, h->cs, bs, SPMX_CSC_LB_MERGE, rshift, nb, y, ykey, yval,
                            h->d_counts + kCntYnnz, h->ls, h->lb_grid, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "bucket launch capacity");

@@ -129,8 +129,7 @@ constexpr int kFlatChunk = 128;  // this many nonzeros
 constexpr int kCscScanNT = 256, kCscScanVT = 8;   // 2048 x entries per tile
 constexpr int kCscLbNT = 256, kCscLbVT = 8;       // 2048 items per LB block
 
-int launch_csc_scan(const CscArgs& a, const CscScratch& s, ScanScratch& ls,
-                    int block_items, cudaStream_t st);
+int launch_csc_scan(const CscArgs& a, const CscScratch& s, ScanScratch& ls, cudaStream_t st);
 // variant: 1 merge, 2 twolayer.  pairs_row/pairs_val non-NULL: write (row,
 // alpha*val*x) pairs at their scanned position instead of atomics into y.
 int launch_csc_lb(const CscArgs& a, const CscScratch& s, int variant, float* y,

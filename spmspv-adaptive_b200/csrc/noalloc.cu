@@ -164,7 +164,7 @@ extern "C" int spmx_spmspv_csc_noalloc(int m, int n, int nnz, const int* d_csc_r
 
   const CscArgs a{m, n, d_csc_col, d_csc_row, d_csc_val, x_nnz, d_x_key, d_x_val,
                   (double)alpha, err, counts};
-  if (launch_csc_scan(a, s, ls, kNoAllocBlockItems, st))
+  if (launch_csc_scan(a, s, ls, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "noalloc SpMSpV: scan capacity");
   launch_csc_lb(a, s, 1, d_y, nullptr, nullptr, grid, st);
   const cudaError_t e = cudaGetLastError();
