@@ -426,6 +426,87 @@ int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c
              : -2;
 }
 
+// A handful of x entries (one warp's worth) in one launch: every CTA owns a slice
+// of y in shared memory, reads all the products (kSliceItems at most, from L2
+// but for the first CTA), adds those of its rows and stores the whole slice, so
+// y needs no fill before.
+//
+// What it saves is a launch: x of 11 entries on 1M rows 5.3 us per call from
+// Python against 7.7 with the zero fill and the scatter, each of whose launches
+// takes the host 2.2 us.  On the device alone the pair is faster (2.5 us per call
+// enqueued ahead, against 3.0, and 3.5 for 32 entries), because the scatter
+// reads x and its columns while y is being cleared, so a capture, which pays no
+// launches, keeps the pair.
+constexpr int kSliceNT = 256, kSliceRows = 4096, kSliceItems = 2048;
+constexpr int kSliceMaxRows = 148 * 8 * kSliceRows;  // one wave of CTAs
+
+__global__ void __launch_bounds__(kSliceNT)
+csc_slice_kernel(CscArgs a, float* __restrict__ y) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ __align__(16) float s_acc[kSliceRows];
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < kSliceRows / 4; i += kSliceNT)
+    reinterpret_cast<float4*>(s_acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  // every warp for itself: the entries' columns and a prefix of their lengths
+  const int key = lane < a.x_nnz ? a.x_key[lane] : -1;
+  float xv = lane < a.x_nnz ? a.x_val[lane] : 0.f;
+  const bool ok = (unsigned)key < (unsigned)a.n;
+  if (lane < a.x_nnz && !ok) flag_error(a.err, kDevErrOob);
+  int cs = 0, len = 0;
+  if (ok) {
+    cs = a.colptr[key];
+    len = a.colptr[key + 1] - cs;
+  }
+  xv = (float)(a.alpha * (double)xv);
+  const int incl = warp_inclusive_sum(len);
+  const int base = cs - (incl - len);
+  const int total = __shfl_sync(FULL, incl, 31);
+  const int row0 = blockIdx.x * kSliceRows;
+  __syncthreads();  // the slice is clear
+  for (int q0 = tid & ~31; q0 < total; q0 += kSliceNT) {
+    const int q = q0 + lane;
+    int o = 0;  // the entry that owns item q
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(FULL, incl, o + step - 1) <= q) o += step;
+    const int p = __shfl_sync(FULL, base, o) + q;
+    const float x = __shfl_sync(FULL, xv, o);
+    if (q < total) {
+      const int r = a.row[p];
+      if ((unsigned)r >= (unsigned)a.m) flag_error(a.err, kDevErrOob);
+      else if ((unsigned)(r - row0) < (unsigned)kSliceRows) atomicAdd(&s_acc[r - row0], a.val[p] * x);
+    }
+  }
+  __syncthreads();
+  const int rows = min(kSliceRows, a.m - row0);
+  float* const out = y + row0;
+  if ((((uintptr_t)out) & 15u) == 0) {
+    for (int i = tid; i < rows >> 2; i += kSliceNT)
+      reinterpret_cast<float4*>(out)[i] = reinterpret_cast<const float4*>(s_acc)[i];
+    for (int i = (rows & ~3) + tid; i < rows; i += kSliceNT) out[i] = s_acc[i];
+  } else {
+    for (int i = tid; i < rows; i += kSliceNT) out[i] = s_acc[i];
+  }
+}
+
+bool csc_slice_fits(const CscArgs& a, long long col_max, cudaStream_t st) {
+  if (a.x_nnz > 32 || a.m > kSliceMaxRows || col_max < 0 || a.x_nnz * col_max > kSliceItems) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap == cudaStreamCaptureStatusNone;
+}
+
+int launch_csc_slice(const CscArgs& a, float* y, cudaStream_t st) {
+  if (a.m <= 0) return 0;
+  note_launch();
+  return launch_pdl(csc_slice_kernel, dim3((unsigned)((a.m + kSliceRows - 1) / kSliceRows)), dim3(kSliceNT), 0, st, a,
+                    y) == cudaSuccess
+             ? 0
+             : -2;
+}
+
 // zero y, then the naive CSC SpMSpV as a programmatic dependent launch
 int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, cudaStream_t st) {
   if (a.m > 0 && launch_zero_fill(y, a.m, num_sms, st)) return -2;

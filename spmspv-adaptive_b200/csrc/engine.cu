@@ -942,7 +942,9 @@ static int csc_atomic(spmx_handle_t h, int variant, float alpha, float* y, int* 
                       float* yval, int* ynnz) {
   cudaStream_t st = h->stream;
   const CscArgs a = csc_args(h, alpha);
-  if (variant == SPMX_CSC_NAIVE) {
+  if (variant == SPMX_CSC_NAIVE && csc_slice_fits(a, h->col_max, st)) {
+    if (launch_csc_slice(a, y, st)) return set_error(SPMX_ERR_CUDA, "csc spmspv launch");
+  } else if (variant == SPMX_CSC_NAIVE) {
     // zero-fill and SpMSpV overlap through a programmatic dependent launch
     if (launch_csc_naive_zeroed(a, col_group(h), y, h->num_sms, st))
       return set_error(SPMX_ERR_INVALID_VALUE, "bad column group");

@@ -140,6 +140,10 @@ int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st);
 // counts[kCntBinlen].
 int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
                     cudaStream_t st);
+// the naive CSC SpMSpV of a handful of x entries in one launch, and whether it
+// applies (col_max: the longest column, -1 where it is not known)
+bool csc_slice_fits(const CscArgs& a, long long col_max, cudaStream_t st);
+int launch_csc_slice(const CscArgs& a, float* y, cudaStream_t st);
 // y = 0 then the naive CSC SpMSpV, as a programmatic dependent launch pair
 int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, cudaStream_t st);
 int launch_csc_naive_pairs(const CscArgs& a, const CscScratch& s, int group,
