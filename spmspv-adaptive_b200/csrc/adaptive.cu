@@ -295,8 +295,8 @@ static int ensure_bfs(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&h->bfs_front, 4 * words, "bfs front"));
   SPMX_TRY(dalloc((void**)&h->bfs_fb1, 4 * words, "bfs front 1"));
   SPMX_TRY(dalloc((void**)&h->bfs_fb2, 4 * words, "bfs front 2"));
-  SPMX_TRY(dalloc((void**)&h->bfs_q[0], 4 * (size_t)std::max(h->n, 1), "bfs queue 0"));
-  SPMX_TRY(dalloc((void**)&h->bfs_q[1], 4 * (size_t)std::max(h->n, 1), "bfs queue 1"));
+  SPMX_TRY(dalloc((void**)&h->bfs_q[0], 8 * (size_t)std::max(h->n, 1), "bfs queue 0"));
+  SPMX_TRY(dalloc((void**)&h->bfs_q[1], 8 * (size_t)std::max(h->n, 1), "bfs queue 1"));
   SPMX_TRY(dalloc((void**)&h->bfs_cnt, 4 * 4, "bfs counts"));
   SPMX_TRY(dalloc((void**)&h->bfs_edges, 8 * 4, "bfs edges"));
   SPMX_TRY(dalloc((void**)&h->bfs_ctrl, sizeof(BfsCtrl), "bfs ctrl"));
@@ -322,7 +322,7 @@ static int bfs_persistent(spmx_handle_t h, int source, int* levels, int* depth) 
   const int n = h->n;
   // the kernel initialises levels, the visited set and the frontier bitmaps
   BfsPersistentArgs a{n, source, h->num_sms, (long long)h->nnz, h->rowptr, h->col, levels,
-                      h->bfs_visited, h->bfs_front, h->bfs_fb1, h->bfs_fb2, h->bfs_q[0], h->bfs_q[1],
+                      h->bfs_visited, h->bfs_front, h->bfs_fb1, h->bfs_fb2, (int2*)h->bfs_q[0], (int2*)h->bfs_q[1],
                       (BfsCtrl*)h->bfs_ctrl, h->bfs_alpha, h->bfs_beta, h->d_err};
   const int rc = launch_bfs_persistent(a, st);
   if (rc) return set_error(SPMX_ERR_CUDA, std::string("cooperative BFS launch: ") +

@@ -6,11 +6,12 @@ namespace spmx {
 
 // device control block of the persistent BFS kernels (zeroed before a launch)
 struct BfsCtrl {
-  int cnt[3];                    // next-frontier sizes, by level % 3
-  int depth;                     // number of levels, written at the end
-  unsigned long long edges[3];   // sum of degrees of the next frontier (multi-source: size << 32 | sum)
-  unsigned bar_count, bar_gen;   // grid barrier
+  unsigned long long edges[3];   // next frontier by level % 3: size << 32 | sum of the degrees
+  // grid barrier: arrivals on one line, what the waiting CTAs poll on another
+  unsigned bar_count, gap0[31];
+  unsigned bar_gen, gap1[31];
   int abort_flag;
+  int depth;                     // number of levels, written at the end
   int pad;                       // multi-source: levels already expanded
 };
 
@@ -24,8 +25,8 @@ struct BfsPersistentArgs {
   unsigned* fb0;
   unsigned* fb1;
   unsigned* fb2;
-  int* q0;
-  int* q1;
+  int2* q0;  // [n] ranges of columns
+  int2* q1;
   BfsCtrl* ctrl;
   double alpha, beta;  // direction switch: push->pull when m_f > m_u/alpha,
                        // pull->push when n_f < n/beta

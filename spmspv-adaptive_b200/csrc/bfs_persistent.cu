@@ -27,26 +27,59 @@ __device__ __forceinline__ bool tbit(const unsigned* bits, int v) {
   return (bits[v >> 5] >> (v & 31)) & 1u;
 }
 
-__device__ __forceinline__ void warp_append2(bool want, int v, int deg, int* q, int* q_count,
-                                             unsigned long long* edge_count) {
-  const unsigned mask = __ballot_sync(0xffffffffu, want);
-  if (!mask) return;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(mask) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(q_count, __popc(mask));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (want) q[base + __popc(mask & lanemask_lt())] = v;
-  unsigned long long d = want ? (unsigned long long)deg : 0ull;
-  d = warp_sum(d);
-  if (lane == leader) atomicAdd(edge_count, d);
-}
+// A warp's way into the next queue: entries collect in shared memory and are
+// appended about a hundred at a time, because every append adds to one counter
+// (queue length in the high word, sum of the degrees, at most nnz, in the low
+// word) and atomics on one address take about 2 ns each.
+constexpr int kOutFlush = 96, kOutCap = kOutFlush + 32;
+template <class T>
+struct WarpOut {
+  T* buf;         // kOutCap entries of this warp
+  int cnt;        // warp-uniform
+  unsigned deg;   // the lane's share of their degrees
+  T* q;
+  unsigned long long* counter;
 
+  __device__ __forceinline__ void flush() {
+    if (!cnt) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned d = __reduce_add_sync(0xffffffffu, deg);
+    unsigned base = 0;
+    if (lane == 0) base = (unsigned)(atomicAdd(counter, ((unsigned long long)cnt << 32) | d) >> 32);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int i = lane; i < cnt; i += 32) q[base + i] = buf[i];
+    __syncwarp();
+    cnt = 0;
+    deg = 0;
+  }
+  __device__ __forceinline__ void add(bool want, T e, int d) {
+    const unsigned mask = __ballot_sync(0xffffffffu, want);
+    if (!mask) return;
+    if (want) {
+      buf[cnt + __popc(mask & lanemask_lt())] = e;
+      deg += (unsigned)d;
+    }
+    cnt += __popc(mask);
+    __syncwarp();
+    if (cnt >= kOutFlush) flush();
+  }
+};
+
+// What bounds it: L2 round trips and the grid barrier of every level.  A queue
+// entry is a vertex's range of columns, looked up when it is found, beside the
+// atomic that finds it, so a push level is queue -> columns -> visited bit ->
+// append.  R-MAT 14 (16,384 vertices, 0.43M edges, 6 levels) 39 us, 16 44, 18 61,
+// 20 (31M edges) 116, against 42, 50, 133 and 242 us with vertices in the queue
+// (row bounds a round trip later on both sides), an append of two atomics per 32
+// edges, and the barrier's two words on one line (which alone took 95 and 188 at
+// 18 and 20).  Two edges in flight per lane instead of one, with the early exits
+// after both: 41, 46, 63 and 128 us; four: 47, 52, 70 and 178.
 __global__ void __launch_bounds__(256)
 bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowptr,
                       const int* __restrict__ col, int* __restrict__ levels,
-                      unsigned* visited, unsigned* fb0, unsigned* fb1, unsigned* fb2, int* q0, int* q1,
+                      unsigned* visited, unsigned* fb0, unsigned* fb1, unsigned* fb2, int2* q0, int2* q1,
                       BfsCtrl* ctrl, double alpha_b, double beta_b, int src, int* err) {
+  __shared__ int2 s_out[8][kOutCap];
   const GridBarrier bar{&ctrl->bar_count, &ctrl->bar_gen, &ctrl->abort_flag};
   const int lane = threadIdx.x & 31;
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,11 +96,8 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
     fb2[w] = 0u;
   }
   if (gtid == 0) {
-    q0[0] = src;
-    for (int k = 0; k < 3; ++k) {
-      ctrl->cnt[k] = 0;
-      ctrl->edges[k] = 0ull;
-    }
+    q0[0] = make_int2(__ldg(rowptr + src), __ldg(rowptr + src + 1));
+    for (int k = 0; k < 3; ++k) ctrl->edges[k] = 0ull;
   }
   if (!grid_sync(bar, err)) return;
   const int src_deg = __ldg(rowptr + src + 1) - __ldg(rowptr + src);
@@ -80,8 +110,8 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
     else if (pull && (double)nf < (double)n / beta_b) pull = false;
     const int nxt = cur ^ 1;
     const int slot = (L + 1) % 3;
-    int* qn = nxt ? q1 : q0;
-    const int* qc = cur ? q1 : q0;
+    const int2* qc = cur ? q1 : q0;
+    WarpOut<int2> out{s_out[threadIdx.x >> 5], 0, 0u, nxt ? q1 : q0, &ctrl->edges[slot]};
     // frontier bitmaps rotate over three buffers: this level reads fbs[L % 3],
     // writes fbs[(L + 1) % 3], and clears fbs[(L + 2) % 3] (the frontier of
     // the previous level, read by nobody now) for the next level; the counter
@@ -91,10 +121,7 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
     unsigned* fbr = fbs[(L + 2) % 3];
     if (L > 0)
       for (long long w = gtid; w < words; w += nthreads) fbr[w] = 0u;
-    if (gtid == 0) {
-      ctrl->cnt[(L + 2) % 3] = 0;
-      ctrl->edges[(L + 2) % 3] = 0ull;
-    }
+    if (gtid == 0) ctrl->edges[(L + 2) % 3] = 0ull;
     if (pull) {
       for (long long vb = gwarp * 32; vb < n; vb += nwarps * 32) {
         const int v = (int)(vb + lane);
@@ -108,10 +135,10 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
         }
         const bool heavy = open && deg > 32;
         if (open && !heavy) {
-          for (int k = a; k < b; ++k) {
+          for (int k = a; k < b && !found; ++k) {
             const int u = __ldg(col + k);
-            if ((unsigned)u >= (unsigned)n) { flag_error(err, kDevErrOob); continue; }
-            if (tbit(fbc, u)) { found = true; break; }
+            if ((unsigned)u >= (unsigned)n) flag_error(err, kDevErrOob);
+            else found = tbit(fbc, u);
           }
         }
         // vertices of degree > 32: the whole warp looks for a frontier neighbour
@@ -138,7 +165,7 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
           atomicOr(visited + (v >> 5), 1u << (v & 31));
           atomicOr(fbn + (v >> 5), 1u << (v & 31));
         }
-        warp_append2(found, v, deg, qn, &ctrl->cnt[slot], &ctrl->edges[slot]);
+        out.add(found, make_int2(a, b), deg);
       }
     } else {
       // a small frontier gets several warps per vertex (equal slices of its
@@ -147,38 +174,38 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
       for (long long wi = gwarp; wi < nf * g; wi += nwarps) {
         const long long f = wi / g;
         const long long part = wi - f * g;
-        const int u = qc[f];
-        const int a0 = __ldg(rowptr + u), b0 = __ldg(rowptr + u + 1);
-        const int a = a0 + (int)(((long long)(b0 - a0) * part) / g);
-        const int b = a0 + (int)(((long long)(b0 - a0) * (part + 1)) / g);
+        const int2 e = qc[f];
+        const int a = e.x + (int)(((long long)(e.y - e.x) * part) / g);
+        const int b = e.x + (int)(((long long)(e.y - e.x) * (part + 1)) / g);
         for (int kb = a; kb < b; kb += 32) {
           const int k = kb + lane;
           bool win = false;
-          int v = 0, deg = 0;
+          int v = 0, va = 0, vb = 0;
           if (k < b) {
             v = __ldg(col + k);
             if ((unsigned)v >= (unsigned)n) {
               flag_error(err, kDevErrOob);
             } else if (!tbit(visited, v)) {
               const unsigned bit = 1u << (v & 31);
-              const unsigned old = atomicOr(visited + (v >> 5), bit);
-              if (!(old & bit)) {
-                win = true;
+              win = !(atomicOr(visited + (v >> 5), bit) & bit);
+              va = __ldg(rowptr + v);  // beside the atomic, whether it wins or not
+              vb = __ldg(rowptr + v + 1);
+              if (win) {
                 levels[v] = L + 1;
                 atomicOr(fbn + (v >> 5), bit);
-                deg = __ldg(rowptr + v + 1) - __ldg(rowptr + v);
               }
             }
           }
-          warp_append2(win, v, deg, qn, &ctrl->cnt[slot], &ctrl->edges[slot]);
+          out.add(win, make_int2(va, vb), vb - va);
         }
       }
     }
+    out.flush();
     if (!grid_sync(bar, err)) return;
-    nf = *(volatile int*)&ctrl->cnt[slot];
-    const long long me = (long long)*(volatile unsigned long long*)&ctrl->edges[slot];
-    mf = me;
-    mu -= me;
+    const unsigned long long packed = *(volatile unsigned long long*)&ctrl->edges[slot];
+    nf = (long long)(packed >> 32);
+    mf = (long long)(packed & 0xffffffffull);
+    mu -= mf;
     if (nf == 0) break;
     cur = nxt;
     ++L;
@@ -272,51 +299,16 @@ __device__ __forceinline__ void ms_expand(const MsBfsState& t, long long gwarp, 
   }
 }
 
-// A warp's way into the next queue: vertices collect in shared memory and are
-// appended about a hundred at a time, because every append adds to one counter
-// (queue length in the high word, sum of the degrees, at most nnz, in the low
-// word) and atomics on one address take about 2 ns each.
-constexpr int kMsFlush = 96, kMsOut = kMsFlush + 32;
-struct MsOut {
-  int* buf;       // kMsOut vertices of this warp
-  int cnt;        // warp-uniform
-  unsigned deg;   // the lane's share of their degrees
-  int* q;
-  unsigned long long* counter;
-
-  __device__ __forceinline__ void flush() {
-    if (!cnt) return;
-    const int lane = threadIdx.x & 31;
-    const unsigned d = __reduce_add_sync(0xffffffffu, deg);
-    unsigned base = 0;
-    if (lane == 0) base = (unsigned)(atomicAdd(counter, ((unsigned long long)cnt << 32) | d) >> 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int i = lane; i < cnt; i += 32) q[base + i] = buf[i];
-    __syncwarp();
-    cnt = 0;
-    deg = 0;
-  }
-  __device__ __forceinline__ void add(bool want, int v, int d) {
-    const unsigned mask = __ballot_sync(0xffffffffu, want);
-    if (!mask) return;
-    if (want) {
-      buf[cnt + __popc(mask & lanemask_lt())] = v;
-      deg += (unsigned)d;
-    }
-    cnt += __popc(mask);
-    __syncwarp();
-    if (cnt >= kMsFlush) flush();
-  }
-};
-
-constexpr int kMsU = 4;    // edges in flight per lane
-constexpr int kMsLane = 8;   // a single lane pushes at most this many edges
-constexpr int kMsHubU = 8; // of a hub chunk: 256 edges, one round trip
+// edges in flight per lane: pushes and mid-degree vertices, then light vertices
+// and hub chunks; a single lane pushes at most kMsLane.  Early exits are tested
+// after each group, so more is not better: R-MAT 22 / 20 (20 sources), us: 2 and
+// 4 1688 / 503, 2 and 2 1697 / 503, 4 and 8 1875 / 607, 1 and 1 1981 / 605
+constexpr int kMsU = 2, kMsHubU = 4, kMsLane = 8;
 
 // pushes the word fu over the edges [a, b) (whole warp)
 __device__ __forceinline__ void ms_push(const MsBfsState& t, const int* __restrict__ rowptr,
                                         const int* __restrict__ col, int a, int b, unsigned long long fu,
-                                        MsOut& out, int* err) {
+                                        WarpOut<int>& out, int* err) {
   const int lane = threadIdx.x & 31;
   for (int kb = a; kb < b; kb += 32 * kMsU) {
     int v[kMsU];
@@ -385,8 +377,8 @@ __device__ __forceinline__ unsigned long long ms_pull(const unsigned long long* 
 
 // What bounds it: the gathers of the frontier words in the two heavy pull levels
 // (one 32-byte L2 sector per edge) and their latency.  64 sources on R-MAT 22
-// (4.2M vertices, 128M edges), expansion included: 1.9 ms (pull levels 0.80 and
-// 0.54 ms, the first push 0.18, expansion 0.23), against 15.7 ms with level
+// (4.2M vertices, 128M edges), expansion included: 1.7 ms (the two pull levels
+// 1.2, the first push 0.18, expansion 0.23), against 15.7 ms with level
 // stores per vertex and a strided transposition (1.7 + 5.0 ms), hubs of up to
 // 10^5 edges on four warps each (one push level 8.8 ms) and one dependent
 // chain per 32 edges (first pull level 3.2 ms).
@@ -394,7 +386,7 @@ __global__ void __launch_bounds__(256)
 msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, const int* __restrict__ rowptr,
                         const int* __restrict__ col, int* q0, int* q1, BfsCtrl* ctrl, HubChunks hub, int* err) {
   const GridBarrier bar{&ctrl->bar_count, &ctrl->bar_gen, &ctrl->abort_flag};
-  __shared__ int s_out[8][kMsOut];
+  __shared__ int s_out[8][kOutCap];
   const unsigned long long FULL = t.ns >= 64 ? ~0ull : ((1ull << t.ns) - 1ull);
   const int n = t.n;
   const int lane = threadIdx.x & 31;
@@ -418,7 +410,7 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
     unsigned long long* counter = &ctrl->edges[(L + 1) % 3];
     int* qn = nxt ? q1 : q0;
     const int* qc = cur ? q1 : q0;
-    MsOut out{s_out[threadIdx.x >> 5], 0, 0u, qn, counter};
+    WarpOut<int> out{s_out[threadIdx.x >> 5], 0, 0u, qn, counter};
     const unsigned long long* fc = cur ? t.front1 : t.front0;
     unsigned long long* fn = nxt ? t.front1 : t.front0;
     if (pull) {
@@ -684,8 +676,8 @@ int launch_bfs_persistent(const BfsPersistentArgs& a, cudaStream_t st) {
   unsigned* f0 = a.fb0;
   unsigned* f1 = a.fb1;
   unsigned* f2 = a.fb2;
-  int* q0 = a.q0;
-  int* q1 = a.q1;
+  int2* q0 = a.q0;
+  int2* q1 = a.q1;
   BfsCtrl* ctrl = a.ctrl;
   double al = a.alpha, be = a.beta;
   int src = a.src;

@@ -388,6 +388,7 @@ __device__ __forceinline__ unsigned lb_warp_lookback(const LookbackState& st,
 // CTA that waits too long records kDevErrTimeout, raises the abort word and
 // returns false; callers then leave the kernel.
 // ---------------------------------------------------------------------------
+constexpr int kBarSleep = 20;
 struct GridBarrier {
   unsigned* count;
   unsigned* generation;
@@ -416,7 +417,7 @@ __device__ __forceinline__ bool grid_sync(const GridBarrier& b, int* err) {
           ok = 0;
           break;
         }
-        __nanosleep(64);
+        __nanosleep(kBarSleep);
       }
     }
     __threadfence();
