@@ -300,6 +300,8 @@ static int ensure_bfs(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&h->bfs_cnt, 4 * 4, "bfs counts"));
   SPMX_TRY(dalloc((void**)&h->bfs_edges, 8 * 4, "bfs edges"));
   SPMX_TRY(dalloc((void**)&h->bfs_ctrl, sizeof(BfsCtrl), "bfs ctrl"));
+  SPMX_CUDA(cudaMemsetAsync(h->bfs_ctrl, 0, sizeof(BfsCtrl), h->stream));
+  SPMX_CUDA(cudaStreamSynchronize(h->stream));
   h->bfs_n = h->n;
   return SPMX_SUCCESS;
 }
@@ -357,6 +359,8 @@ static int ensure_msbfs(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&h->ms_q1, 4 * n, "msbfs queue 1"));
   SPMX_TRY(dalloc(&h->ms_planes, 32 * n, "msbfs level planes"));
   SPMX_TRY(dalloc(&h->ms_ctrl, sizeof(BfsCtrl), "msbfs ctrl"));
+  SPMX_CUDA(cudaMemsetAsync(h->ms_ctrl, 0, sizeof(BfsCtrl), h->stream));
+  SPMX_CUDA(cudaStreamSynchronize(h->stream));
   SPMX_TRY(dalloc((void**)&h->ms_visit, 32 * n, "msbfs words"));
   h->ms_front0 = h->ms_visit + n;
   h->ms_front1 = h->ms_visit + 2 * n;

@@ -4,13 +4,14 @@
 
 namespace spmx {
 
-// device control block of the persistent BFS kernels (zeroed before a launch)
+// device control block of the persistent BFS kernels (zeroed once)
 struct BfsCtrl {
   unsigned long long edges[3];   // next frontier by level % 3: size << 32 | sum of the degrees
   // grid barrier: arrivals on one line, what the waiting CTAs poll on another
   unsigned bar_count, gap0[31];
   unsigned bar_gen, gap1[31];
   int abort_flag;
+  unsigned left;                 // CTAs that have left the kernel
   int depth;                     // number of levels, written at the end
   int pad;                       // multi-source: levels already expanded
 };

@@ -65,10 +65,22 @@ struct WarpOut {
   }
 };
 
+// Every CTA leaves through here; the last one puts the barrier back for the next
+// launch (also after a barrier that gave up), so no launch clears it first.
+__device__ __forceinline__ void bfs_leave(BfsCtrl* ctrl) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&ctrl->left, 1u) != gridDim.x - 1) return;
+  ctrl->bar_count = 0u;
+  ctrl->abort_flag = 0;
+  ctrl->left = 0u;
+}
+
 // What bounds it: L2 round trips and the grid barrier of every level.  A queue
 // entry is a vertex's range of columns, looked up when it is found, beside the
 // atomic that finds it, so a push level is queue -> columns -> visited bit ->
-// append.  R-MAT 14 (16,384 vertices, 0.43M edges, 6 levels) 39 us, 16 44, 18 61,
+// append.  R-MAT 14 (16,384 vertices, 0.43M edges, 6 levels) 38 us, 16 43, 18 61,
 // 20 (31M edges) 116, against 42, 50, 133 and 242 us with vertices in the queue
 // (row bounds a round trip later on both sides), an append of two atomics per 32
 // edges, and the barrier's two words on one line (which alone took 95 and 188 at
@@ -99,7 +111,10 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
     q0[0] = make_int2(__ldg(rowptr + src), __ldg(rowptr + src + 1));
     for (int k = 0; k < 3; ++k) ctrl->edges[k] = 0ull;
   }
-  if (!grid_sync(bar, err)) return;
+  if (!grid_sync(bar, err)) {
+      bfs_leave(ctrl);
+      return;
+    }
   const int src_deg = __ldg(rowptr + src + 1) - __ldg(rowptr + src);
   long long nf = 1, mf = src_deg, mu = total_edges - src_deg;
   bool pull = false;
@@ -201,7 +216,10 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
       }
     }
     out.flush();
-    if (!grid_sync(bar, err)) return;
+    if (!grid_sync(bar, err)) {
+      bfs_leave(ctrl);
+      return;
+    }
     const unsigned long long packed = *(volatile unsigned long long*)&ctrl->edges[slot];
     nf = (long long)(packed >> 32);
     mf = (long long)(packed & 0xffffffffull);
@@ -211,6 +229,7 @@ bfs_persistent_kernel(int n, long long total_edges, const int* __restrict__ rowp
     ++L;
   }
   if (gtid == 0) ctrl->depth = L + 1;
+  bfs_leave(ctrl);
 }
 
 
@@ -402,7 +421,10 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
     if (L + 1 == kMsPlaneLevels) {  // the next level does not fit the planes
       ms_expand(t, gwarp, nwarps);
       if (gtid == 0) ctrl->pad = 1;
-      if (!grid_sync(bar, err)) return;
+      if (!grid_sync(bar, err)) {
+      bfs_leave(ctrl);
+      return;
+    }
       direct = true;
     }
     const bool pull = (double)mf > (double)total_edges / alpha_ms;
@@ -548,7 +570,10 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
       }
     }
     out.flush();
-    if (!grid_sync(bar, err)) return;
+    if (!grid_sync(bar, err)) {
+      bfs_leave(ctrl);
+      return;
+    }
     // retire the current frontier
     for (long long f = gtid; f < nq; f += nthreads) ((unsigned long long*)fc)[qc[f]] = 0ull;
     const long long nn = (long long)(*(volatile unsigned long long*)counter >> 32);  // before the pulled hubs
@@ -592,7 +617,10 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
       }
     }
     if (gtid == 0) ctrl->edges[(L + 2) % 3] = 0ull;
-    if (!grid_sync(bar, err)) return;
+    if (!grid_sync(bar, err)) {
+      bfs_leave(ctrl);
+      return;
+    }
     packed = *(volatile unsigned long long*)counter;
     nq = (long long)(packed >> 32);
     mf = (long long)(packed & 0xffffffffull);
@@ -601,6 +629,7 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
     ++L;
   }
   if (gtid == 0) ctrl->depth = L + 1;
+  bfs_leave(ctrl);
 }
 
 __global__ void __launch_bounds__(256) msbfs_expand_kernel(MsBfsState t, const BfsCtrl* ctrl) {
@@ -617,6 +646,8 @@ msbfs_init_kernel(MsBfsState t, MsSources srcs, const int* __restrict__ rowptr, 
   const int v = s < t.ns ? srcs.v[s] : -1;
   const bool ok = (unsigned)v < (unsigned)t.n;
   s_v[s] = ok ? v : -1;
+  if (s < 3) ctrl->edges[s] = 0ull;
+  if (s == 3) ctrl->pad = 0;
   __syncthreads();
   unsigned long long bits = 0ull;
   bool first = ok;
@@ -665,7 +696,6 @@ int launch_bfs_persistent(const BfsPersistentArgs& a, cudaStream_t st) {
   // small graphs get few CTAs: the level barriers then cost less
   const int grid = coop_grid(bfs_persistent_kernel, a.num_sms, 16, a.n);
   if (grid <= 0) return -1;
-  cudaMemsetAsync(a.ctrl, 0, sizeof(BfsCtrl), st);
   note_launch();
   int n = a.n;
   long long te = a.total_edges;
@@ -715,7 +745,6 @@ int launch_hub_chunks(int n, const int* rowptr, int deg_cut, int4* chunk, int* v
 int launch_msbfs(const MsBfsArgs& a, cudaStream_t st) {
   const int grid = coop_grid(msbfs_persistent_kernel, a.num_sms, a.num_sms, a.n);
   if (grid <= 0) return -1;
-  cudaMemsetAsync(a.ctrl, 0, sizeof(BfsCtrl), st);
   MsBfsState t{a.n, a.ns, a.layout, a.levels, a.visit, a.front0, a.front1, a.next, a.planes};
   note_launch(3);
   msbfs_init_kernel<<<1, 64, 0, st>>>(t, a.srcs, a.rowptr, a.q0, a.ctrl);
