@@ -10,10 +10,10 @@
 //   DEV/csc_sort_load_balance.cuh:295) whose look-back spins without bound on
 //   `sum[gid-1]==0` (scan_kernel.cuh:99).
 //
-// The dense-y (atomic) write-back of a handle needs no global scan:
-// csc_flat_kernel.
+// The dense-y (atomic) write-back of a handle, and its sorted (key, value)
+// write-back up to a number of rows, need no global scan: csc_flat_kernel.
 //
-// Stage 2 of the sort write-back and of the allocation-free entry point (the
+// Stage 2 of the sort write-back above that, and of the allocation-free entry point (the
 //   bucket kernels share the block mapping), csc_lb_kernel: persistent CTAs take blocks of 2048 work items.
 //   "twolayer" blocks hold 2048 nonzeros (DEV/csc_two_layer_load_balance_
 //   fuse_reduction_modify.cuh:155); "merge" blocks hold 2048 merge-path items
@@ -187,6 +187,13 @@ csc_naive_kernel(CscArgs a, float* __restrict__ y) {
   }
 }
 
+template <class T>
+__device__ __forceinline__ void row_add(T* y, float v) {
+  // v + 0.0 is never -0.0, nor is a sum that it entered
+  if (sizeof(T) == 8) atomicAdd(y, (T)v + (T)0);
+  else atomicAdd(y, (T)v);
+}
+
 // Load-balanced SpMSpV with atomic write-back, without a scan: a warp takes E
 // consecutive x entries (E = 2^elog <= 32), scans their column lengths with
 // shuffles and spreads the nonzeros over its lanes, U per lane in flight; a
@@ -204,9 +211,11 @@ csc_naive_kernel(CscArgs a, float* __restrict__ y) {
 // entries): 512 and 256 16.7 / 141 us, 256 and 256 14.7 / 106, 128 and 128 13.4 /
 // 96, 64 and 64 13.6 / 85.  Two nonzeros in flight per lane instead of four 14.2 /
 // 108, eight 15.6 / 122.
-template <int U>
+//
+// T = double: y starts at -0.0 (row_add), so that it tells the rows reached.
+template <int U, class T>
 __global__ void __launch_bounds__(256)
-csc_flat_kernel(CscArgs a, int elog, float* __restrict__ y, CscLong* queue, int qcap, int defer) {
+csc_flat_kernel(CscArgs a, int elog, T* __restrict__ y, CscLong* queue, int qcap, int defer) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ unsigned s_bin[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -258,7 +267,7 @@ csc_flat_kernel(CscArgs a, int elog, float* __restrict__ y, CscLong* queue, int 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (q0 + u * 32 + lane >= total) continue;
-      if ((unsigned)r[u] < (unsigned)a.m) atomicAdd(y + r[u], v[u]);
+      if ((unsigned)r[u] < (unsigned)a.m) row_add(y + r[u], v[u]);
       else flag_error(a.err, kDevErrOob);
     }
     q0 += 32 * U;
@@ -281,7 +290,7 @@ csc_flat_kernel(CscArgs a, int elog, float* __restrict__ y, CscLong* queue, int 
       } else {  // only with repeated x keys: this lane's chunk on the spot
         for (int k = s0; k < s1; ++k) {
           const int rr = __ldg(a.row + k);
-          if ((unsigned)rr < (unsigned)a.m) atomicAdd(y + rr, __ldg(a.val + k) * x);
+          if ((unsigned)rr < (unsigned)a.m) row_add(y + rr, __ldg(a.val + k) * x);
           else flag_error(a.err, kDevErrOob);
         }
       }
@@ -297,8 +306,9 @@ csc_flat_kernel(CscArgs a, int elog, float* __restrict__ y, CscLong* queue, int 
 }
 
 // the chunks of the long columns, one warp each
+template <class T>
 __global__ void __launch_bounds__(256)
-csc_flat_long_kernel(CscArgs a, float* __restrict__ y, const CscLong* queue, int qcap) {
+csc_flat_long_kernel(CscArgs a, T* __restrict__ y, const CscLong* queue, int qcap) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   constexpr int U = 8;
@@ -319,7 +329,7 @@ csc_flat_long_kernel(CscArgs a, float* __restrict__ y, const CscLong* queue, int
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (kb + u * 32 + lane >= ch.k1) continue;
-        if ((unsigned)r[u] < (unsigned)a.m) atomicAdd(y + r[u], v[u]);
+        if ((unsigned)r[u] < (unsigned)a.m) row_add(y + r[u], v[u]);
         else flag_error(a.err, kDevErrOob);
       }
     }
@@ -393,6 +403,8 @@ int launch_csc_lb(const CscArgs& a, const CscScratch& s, int variant, float* y,
 // wait (x keys, column bounds) therefore never starts while a grid that
 // writes them is still running.
 // c0 / c1 (optional) are cleared too: counters of the grid that follows.
+// NEG: y holds m / 2 doubles (16-byte aligned), which become -0.0.
+template <bool NEG>
 __global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, int* c1) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
@@ -400,15 +412,16 @@ __global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, in
     if (c0) *c0 = 0;
     if (c1) *c1 = 0;
   }
+  constexpr float hi = NEG ? -0.0f : 0.0f;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nt = (long long)gridDim.x * blockDim.x;
   if ((((uintptr_t)y) & 15u) == 0) {
     float4* y4 = reinterpret_cast<float4*>(y);
     const long long m4 = m >> 2;
-    for (long long i = tid; i < m4; i += nt) y4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (long long i = (m4 << 2) + tid; i < m; i += nt) y[i] = 0.f;
+    for (long long i = tid; i < m4; i += nt) y4[i] = make_float4(0.f, hi, 0.f, hi);
+    for (long long i = (m4 << 2) + tid; i < m; i += nt) y[i] = (i & 1) ? hi : 0.f;
   } else {
-    for (long long i = tid; i < m; i += nt) y[i] = 0.f;
+    for (long long i = tid; i < m; i += nt) y[i] = (i & 1) ? hi : 0.f;
   }
 }
 
@@ -420,7 +433,7 @@ int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c
   if (m <= 0 && !c0 && !c1) return 0;
   const long long blocks = std::min<long long>((m + 1023) / 1024, (long long)num_sms * 4);
   note_launch();
-  return launch_pdl(zero_fill_kernel, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st, y, m, c0, c1) ==
+  return launch_pdl(zero_fill_kernel<false>, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st, y, m, c0, c1) ==
                  cudaSuccess
              ? 0
              : -2;
@@ -537,9 +550,15 @@ int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, 
   return e == cudaSuccess ? 0 : -2;
 }
 
-int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
-                    cudaStream_t st) {
-  if (launch_zero_fill(y, a.m, num_sms, st, a.counts + kCntBinlen, a.counts + kCntLong)) return -2;
+template <class T>
+static int launch_flat(const CscArgs& a, const CscScratch& s, T* y, long long col_max, int num_sms, cudaStream_t st) {
+  constexpr bool NEG = sizeof(T) == 8;
+  const long long words = (long long)a.m * (sizeof(T) / 4);
+  const long long blocks = std::min<long long>((words + 1023) / 1024, (long long)num_sms * 4);
+  note_launch();
+  if (launch_pdl(zero_fill_kernel<NEG>, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st,
+                 reinterpret_cast<float*>(y), words, a.counts + kCntBinlen, a.counts + kCntLong) != cudaSuccess)
+    return -2;
   if (a.x_nnz <= 0) return 0;
   // entries per warp: enough that the grid is about one wave of warps
   const long long resident = (long long)num_sms * 64;
@@ -548,12 +567,22 @@ int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long c
   const long long warps = ((long long)a.x_nnz + (1 << elog) - 1) >> elog;
   const int defer = col_max < 0 || col_max > kFlatCut;  // the longest column, where it is known
   note_launch(1 + defer);
-  cudaError_t e = launch_pdl(csc_flat_kernel<4>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, a, elog, y,
+  cudaError_t e = launch_pdl(csc_flat_kernel<4, T>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, a, elog, y,
                              s.longq, s.long_cap, defer);
   if (e == cudaSuccess && defer)
-    e = launch_pdl(csc_flat_long_kernel, dim3((unsigned)num_sms * 4), dim3(256), 0, st, a, y,
+    e = launch_pdl(csc_flat_long_kernel<T>, dim3((unsigned)num_sms * 4), dim3(256), 0, st, a, y,
                    (const CscLong*)s.longq, s.long_cap);
   return e == cudaSuccess ? 0 : -2;
+}
+
+int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
+                    cudaStream_t st) {
+  return launch_flat(a, s, y, col_max, num_sms, st);
+}
+
+int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, int num_sms,
+                         cudaStream_t st) {
+  return launch_flat(a, s, acc, col_max, num_sms, st);
 }
 
 int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st) {

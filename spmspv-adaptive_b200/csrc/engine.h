@@ -67,8 +67,7 @@ struct spmx_handle_s {
   unsigned* sv_alt = nullptr;
   void* sradix = nullptr;     // radix_scratch_bytes
   int* sslot = nullptr;
-  int* sy_key = nullptr;      // internal sparse y (adaptive path)
-  float* sy_val = nullptr;
+  double* srow = nullptr;     // y in double (csc_row_scan); or an internal sparse y, keys before values
   bool sort_ready = false;
   int* bk_gcount = nullptr;   // bucket histogram / offsets / cursors
   int* bk_boff = nullptr;

@@ -140,6 +140,9 @@ int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st);
 // counts[kCntBinlen].
 int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
                     cudaStream_t st);
+// the same into acc, whose rows that no nonzero reaches stay -0.0 (no other is)
+int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, int num_sms,
+                         cudaStream_t st);
 // the naive CSC SpMSpV of a handful of x entries in one launch, and whether it
 // applies (col_max: the longest column, -1 where it is not known)
 bool csc_slice_fits(const CscArgs& a, long long col_max, cudaStream_t st);
@@ -163,7 +166,10 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st);
 // keys/vals of the entries != 0 of dense[0..len), in order; count -> *d_count.
 // limit > 0: nothing but the count is written where it reaches the limit
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
-                           int* d_count, ScanScratch& ls, int* err,
-                           cudaStream_t st, int limit = 0);
+                           int* d_count, ScanScratch& ls, cudaStream_t st, int limit = 0);
+// keys/vals (each optional) of the entries of acc[0..len) other than -0.0, in
+// order; dense (optional): all of them, rounded, the others 0; count -> *d_count
+int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
+                        ScanScratch& ls, cudaStream_t st);
 
 }  // namespace spmx

@@ -78,10 +78,13 @@ __global__ void dense2bits_kernel(int len, const float* __restrict__ dense,
 // on another CTA.
 constexpr int kCompactMaxRanges = 1024;
 
-template <int NT, int VT>
+// T = double: the entries kept are those other than -0.0 (launch_compact_rows).
+__device__ __forceinline__ bool compact_keep(float v) { return v != 0.0f; }
+__device__ __forceinline__ bool compact_keep(double v) { return __double_as_longlong(v) != (long long)(1ULL << 63); }
+
+template <int NT, int VT, class T>
 __global__ void __launch_bounds__(NT)
-compact_count_kernel(long long len, long long per, const float* __restrict__ dense,
-                     unsigned* __restrict__ counts) {
+compact_count_kernel(long long len, long long per, const T* __restrict__ in, unsigned* __restrict__ counts) {
   constexpr int NW = NT / 32;
   __shared__ unsigned s_w[NW];
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -92,7 +95,7 @@ compact_count_kernel(long long len, long long per, const float* __restrict__ den
 #pragma unroll
     for (int j = 0; j < VT; ++j) {
       const long long i = b + j * NT + threadIdx.x;
-      c += (i < r1 && __ldg(dense + i) != 0.0f) ? 1u : 0u;
+      c += (i < r1 && compact_keep(__ldg(in + i))) ? 1u : 0u;
     }
   }
   c = warp_sum(c);
@@ -105,11 +108,12 @@ compact_count_kernel(long long len, long long per, const float* __restrict__ den
   }
 }
 
-template <int NT, int VT>
+template <int NT, int VT, class T>
 __global__ void __launch_bounds__(NT)
-compact_write_kernel(long long len, long long per, const float* __restrict__ dense,
-                     const unsigned* __restrict__ counts, int* __restrict__ key,
-                     float* __restrict__ val, int* d_count, unsigned limit) {
+compact_write_kernel(long long len, long long per, const T* __restrict__ in, const unsigned* __restrict__ counts,
+                     float* __restrict__ dense, int* __restrict__ key, float* __restrict__ val, int* d_count,
+                     unsigned limit) {
+  constexpr bool ROWS = sizeof(T) == 8;
   constexpr int NW = NT / 32;
   __shared__ unsigned s_cnt[VT * NW];
   __shared__ unsigned s_wtmp[NW + 1];
@@ -118,14 +122,17 @@ compact_write_kernel(long long len, long long per, const float* __restrict__ den
   __shared__ float s_val[NT * VT];
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const long long r0 = (long long)blockIdx.x * per, r1 = min(len, r0 + per);
-  // the first sub-tile's values: dense was written before pass 1 waited, so
-  // it is complete once this grid starts
-  float v[VT];
+  // the first sub-tile's values: they were written before pass 1 waited, so
+  // they are complete once this grid starts
+  T v[VT];
+  const auto load = [&](long long b) {
 #pragma unroll
-  for (int j = 0; j < VT; ++j) {
-    const long long i = r0 + j * NT + tid;
-    v[j] = (i < r1) ? __ldg(dense + i) : 0.0f;
-  }
+    for (int j = 0; j < VT; ++j) {
+      const long long i = b + j * NT + tid;
+      v[j] = (i < r1) ? __ldg(in + i) : ROWS ? (T)-0.0 : (T)0;
+    }
+  };
+  load(r0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   // nonzeros before this range, and in all
@@ -155,17 +162,11 @@ compact_write_kernel(long long len, long long per, const float* __restrict__ den
 #pragma unroll
   for (int q = 0; q < NW; ++q) run += s_red[q];
   for (long long b = r0; b < r1; b += (long long)NT * VT) {
-    if (b != r0) {
-#pragma unroll
-      for (int j = 0; j < VT; ++j) {
-        const long long i = b + j * NT + tid;
-        v[j] = (i < r1) ? __ldg(dense + i) : 0.0f;
-      }
-    }
+    if (b != r0) load(b);
     unsigned mask[VT];
 #pragma unroll
     for (int j = 0; j < VT; ++j) {
-      mask[j] = __ballot_sync(0xffffffffu, v[j] != 0.0f);
+      mask[j] = __ballot_sync(0xffffffffu, compact_keep(v[j]));
       if (lane == 0) s_cnt[j * NW + w] = __popc(mask[j]);
     }
     __syncthreads();
@@ -179,16 +180,23 @@ compact_write_kernel(long long len, long long per, const float* __restrict__ den
     // stores are contiguous (full PCIe write packets for pinned host memory)
 #pragma unroll
     for (int j = 0; j < VT; ++j) {
-      if (v[j] != 0.0f) {
+      if (compact_keep(v[j])) {
         const unsigned pos = s_cnt[j * NW + w] + __popc(mask[j] & lanemask_lt());
         s_key[pos] = (int)(b + j * NT + tid);
-        s_val[pos] = v[j];
+        s_val[pos] = (float)v[j];
+      }
+    }
+    if (ROWS && dense) {
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        const long long i = b + j * NT + tid;
+        if (i < r1) dense[i] = (float)(v[j] + (T)0);  // -0.0 + 0 = 0
       }
     }
     __syncthreads();
     for (unsigned t = tid; t < total; t += NT) {
-      key[run + t] = s_key[t];
-      val[run + t] = s_val[t];
+      if (!ROWS || key) key[run + t] = s_key[t];
+      if (!ROWS || val) val[run + t] = s_val[t];
     }
     run += total;
     __syncthreads();
@@ -230,11 +238,10 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st) {
   return 0;
 }
 
-int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
-                           int* d_count, ScanScratch& ls, int* err,
-                           cudaStream_t st, int limit) {
+template <class T>
+static int launch_compact(int len, const T* in, float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
+                          cudaStream_t st, int limit) {
   constexpr int NT = 256, VT = 8;
-  (void)err;
   if (len <= 0) { cudaMemsetAsync(d_count, 0, sizeof(int), st); return 0; }
   // ranges of whole sub-tiles, at most kCompactMaxRanges of them
   const long long sub = NT * VT;
@@ -243,12 +250,22 @@ int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
   const long long ranges = (len + per - 1) / per;
   if (ranges > ls.status_len || !ls.counts) return -1;
   note_launch(2);
-  if (launch_pdl(compact_count_kernel<NT, VT>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per,
-                 dense, ls.counts) != cudaSuccess ||
-      launch_pdl(compact_write_kernel<NT, VT>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per,
-                 dense, (const unsigned*)ls.counts, key, val, d_count, (unsigned)limit) != cudaSuccess)
+  if (launch_pdl(compact_count_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
+                 ls.counts) != cudaSuccess ||
+      launch_pdl(compact_write_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
+                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit) != cudaSuccess)
     return -2;
   return 0;
+}
+
+int launch_compact_nonzero(int len, const float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
+                           cudaStream_t st, int limit) {
+  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit);
+}
+
+int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
+                        ScanScratch& ls, cudaStream_t st) {
+  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0);
 }
 
 }  // namespace spmx
