@@ -194,6 +194,26 @@ __device__ __forceinline__ void row_add(T* y, float v) {
   else atomicAdd(y, (T)v);
 }
 
+// The warp's products r, v (r = -1: none) into y, those of one row as one.  A row
+// that holds most columns otherwise takes one reduction after the other at 1.5 ns
+// each: 9 nonzeros a column, one row full, x of 1M 1,570 us against 484 so; but
+// without such a row 78 against 118, match_any being a loop over the distinct rows.
+template <class T>
+__device__ __forceinline__ void row_add_warp(T* y, int r, float v) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned same = __match_any_sync(FULL, r);
+  double d = (double)v + 0.0;
+  for (unsigned left = __ballot_sync(FULL, r >= 0 && (same & (same - 1))); left;) {
+    const int src = __ffs(left) - 1;
+    const unsigned grp = __shfl_sync(FULL, same, src);
+    const double t = warp_sum((grp >> lane) & 1u ? d : 0.0);
+    if (lane == src) d = t;
+    left &= ~grp;
+  }
+  if (r >= 0 && lane == __ffs(same) - 1) atomicAdd(y + r, (T)d);
+}
+
 // Load-balanced SpMSpV with atomic write-back, without a scan: a warp takes E
 // consecutive x entries (E = 2^elog <= 32), scans their column lengths with
 // shuffles and spreads the nonzeros over its lanes, U per lane in flight; a
@@ -213,7 +233,7 @@ __device__ __forceinline__ void row_add(T* y, float v) {
 // 108, eight 15.6 / 122.
 //
 // T = double: y starts at -0.0 (row_add), so that it tells the rows reached.
-template <int U, class T>
+template <int U, class T, bool COMBINE>
 __global__ void __launch_bounds__(256)
 csc_flat_kernel(CscArgs a, int elog, T* __restrict__ y, CscLong* queue, int qcap, int defer) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -266,6 +286,12 @@ csc_flat_kernel(CscArgs a, int elog, T* __restrict__ y, CscLong* queue, int qcap
   for (int q0 = 0;;) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      if (COMBINE) {
+        const bool in = (unsigned)r[u] < (unsigned)a.m;
+        if (!in && q0 + u * 32 + lane < total) flag_error(a.err, kDevErrOob);
+        row_add_warp(y, in ? r[u] : -1, v[u]);
+        continue;
+      }
       if (q0 + u * 32 + lane >= total) continue;
       if ((unsigned)r[u] < (unsigned)a.m) row_add(y + r[u], v[u]);
       else flag_error(a.err, kDevErrOob);
@@ -550,7 +576,7 @@ int launch_csc_naive_zeroed(const CscArgs& a, int group, float* y, int num_sms, 
   return e == cudaSuccess ? 0 : -2;
 }
 
-template <class T>
+template <class T, bool COMBINE>
 static int launch_flat(const CscArgs& a, const CscScratch& s, T* y, long long col_max, int num_sms, cudaStream_t st) {
   constexpr bool NEG = sizeof(T) == 8;
   const long long words = (long long)a.m * (sizeof(T) / 4);
@@ -567,7 +593,7 @@ static int launch_flat(const CscArgs& a, const CscScratch& s, T* y, long long co
   const long long warps = ((long long)a.x_nnz + (1 << elog) - 1) >> elog;
   const int defer = col_max < 0 || col_max > kFlatCut;  // the longest column, where it is known
   note_launch(1 + defer);
-  cudaError_t e = launch_pdl(csc_flat_kernel<4, T>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, a, elog, y,
+  cudaError_t e = launch_pdl(csc_flat_kernel<4, T, COMBINE>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, a, elog, y,
                              s.longq, s.long_cap, defer);
   if (e == cudaSuccess && defer)
     e = launch_pdl(csc_flat_long_kernel<T>, dim3((unsigned)num_sms * 4), dim3(256), 0, st, a, y,
@@ -577,12 +603,18 @@ static int launch_flat(const CscArgs& a, const CscScratch& s, T* y, long long co
 
 int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
                     cudaStream_t st) {
-  return launch_flat(a, s, y, col_max, num_sms, st);
+  return launch_flat<float, false>(a, s, y, col_max, num_sms, st);
 }
 
-int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, int num_sms,
-                         cudaStream_t st) {
-  return launch_flat(a, s, acc, col_max, num_sms, st);
+// products that one row may get before those of a warp are combined: they take 50
+// us one by one (x of 100,000, a row of 73,000: 50 us a call either way)
+constexpr int kHubProducts = 32768;
+
+int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, long long row_max,
+                         int num_sms, cudaStream_t st) {
+  const bool combine = a.x_nnz > kHubProducts && (row_max < 0 || row_max > kHubProducts);
+  return combine ? launch_flat<double, true>(a, s, acc, col_max, num_sms, st)
+                 : launch_flat<double, false>(a, s, acc, col_max, num_sms, st);
 }
 
 int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st) {

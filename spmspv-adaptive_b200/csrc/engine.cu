@@ -380,6 +380,7 @@ extern "C" int spmx_input_csc(spmx_handle_t h, int nnz, const int* csc_row,
   h->csc_val = csc_val;
   h->has_csc = true;
   h->col_max = -1;
+  h->row_max = -1;
   return SPMX_SUCCESS;
 }
 
@@ -462,7 +463,10 @@ extern "C" int spmx_to_csc(spmx_handle_t h) {
     SPMX_CUDA(cudaMemsetAsync(h->own_colptr, 0, 4 * (size_t)(n + 1), st));
   }
   if (rc) return rc;
+  launch_max_degree(m, h->rowptr, h->d_iacc, st);
+  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned, h->d_iacc, sizeof(int), cudaMemcpyDeviceToHost, st));
   SPMX_CUDA(cudaStreamSynchronize(st));
+  h->row_max = h->h_pinned[0];
   h->csc_colptr = h->own_colptr;
   h->csc_row = h->own_row;
   h->csc_val = h->own_cval;
@@ -984,7 +988,7 @@ static int csc_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float
   const CscArgs a = csc_args(h, alpha);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
-  if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->num_sms, st) ||
+  if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->row_max, h->num_sms, st) ||
       launch_compact_rows(h->m, h->srow, y, ykey, yval, h->d_counts + kCntYnnz, h->ls, st))
     return set_error(SPMX_ERR_CUDA, "csc sorted spmspv launch");
   SPMX_TRY(launch_ok("csc sorted spmspv"));

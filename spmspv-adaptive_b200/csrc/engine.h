@@ -99,6 +99,7 @@ struct spmx_handle_s {
   double mat_feat[10] = {0};
   bool std_row_ready = false;
   long long col_max = -1;     // longest CSC column (-1 = not computed)
+  long long row_max = -1;     // longest row of the CSC matrix (-1 = not known)
   float std_row = 0.f;
   long long bin_len = -1;
   long long vec_max = 0, vec_min = 0;

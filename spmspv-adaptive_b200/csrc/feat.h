@@ -4,6 +4,8 @@
 
 namespace spmx {
 
+// the longest row -> *out
+int launch_max_degree(int m, const int* rowptr, int* out, cudaStream_t st);
 int launch_mat_features(int m, const int* rowptr, int nnz, double avg,
                         double avg_int, double* acc, int* iacc,
                         cudaStream_t st);

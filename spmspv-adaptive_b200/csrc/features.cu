@@ -201,6 +201,31 @@ int launch_mat_features(int m, const int* rowptr, int nnz, double avg,
   return 0;
 }
 
+// longest row: one atomic per CTA (mat_features_kernel's six per warp take 70 us
+// for 1M rows, this 4)
+__global__ void __launch_bounds__(256)
+max_degree_kernel(int m, const int* __restrict__ rowptr, int* out) {
+  __shared__ int s_w[8];
+  int mx = 0;
+  for (long long r = (long long)blockIdx.x * 256 + threadIdx.x; r < m; r += (long long)gridDim.x * 256)
+    mx = max(mx, __ldg(rowptr + r + 1) - __ldg(rowptr + r));
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < 8; ++q) mx = max(mx, s_w[q]);
+    atomicMax(out, mx);
+  }
+}
+
+int launch_max_degree(int m, const int* rowptr, int* out, cudaStream_t st) {
+  cudaMemsetAsync(out, 0, sizeof(int), st);
+  if (m <= 0) return 0;
+  note_launch();
+  max_degree_kernel<<<grid_for(m, 256, 148 * 4), 256, 0, st>>>(m, rowptr, out);
+  return 0;
+}
+
 int launch_degree_hist(int m, const int* rowptr, int* hist, cudaStream_t st) {
   if (m <= 0) return 0;
   note_launch();

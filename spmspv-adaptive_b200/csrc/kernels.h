@@ -140,9 +140,10 @@ int launch_csc_naive(const CscArgs& a, int group, float* y, cudaStream_t st);
 // counts[kCntBinlen].
 int launch_csc_flat(const CscArgs& a, const CscScratch& s, float* y, long long col_max, int num_sms,
                     cudaStream_t st);
-// the same into acc, whose rows that no nonzero reaches stay -0.0 (no other is)
-int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, int num_sms,
-                         cudaStream_t st);
+// the same into acc, whose rows that no nonzero reaches stay -0.0 (no other is);
+// row_max: the longest row, -1 where it is not known
+int launch_csc_flat_rows(const CscArgs& a, const CscScratch& s, double* acc, long long col_max, long long row_max,
+                         int num_sms, cudaStream_t st);
 // the naive CSC SpMSpV of a handful of x entries in one launch, and whether it
 // applies (col_max: the longest column, -1 where it is not known)
 bool csc_slice_fits(const CscArgs& a, long long col_max, cudaStream_t st);

@@ -88,3 +88,30 @@ def test_many_rows(torch_cuda, m, k):
     h = make_handle(A, torch, hola=False)
     key = np.sort(rng.choice(64, k, replace=False)).astype(np.int32)
     _check(torch, A, h, 1, key, rng.uniform(-1, 1, k).astype(np.float32), "keyval")
+
+
+@pytest.mark.parametrize("csr", [True, False])
+@pytest.mark.parametrize("k", [32768, 32769, 40000])
+def test_full_rows(torch_cuda, k, csr):
+    """Rows of every column, with and without the row lengths being known: from
+    32,769 products of a row on, those of a warp are combined."""
+    from gpu_util import dev
+    from spmx import SpmspvHandle
+    from spmx.gen import Csr
+    torch = torch_cuda
+    m, n = 300, 40000
+    rng = np.random.default_rng(k)
+    full = np.zeros((m, n), bool)
+    full[[0, 17, 299]] = True
+    full[rng.integers(0, m, 2 * n), rng.integers(0, n, 2 * n)] = True
+    r, c = np.nonzero(full)
+    rowptr = np.r_[0, np.cumsum(full.sum(1))].astype(np.int32)
+    A = Csr(m, n, rowptr, c.astype(np.int32), rng.uniform(-1, 1, len(c)).astype(np.float32))
+    if csr:
+        h = make_handle(A, torch, hola=False)
+    else:
+        colptr, row, cval = (dev(t, torch) for t in A.to_csc())
+        h = SpmspvHandle(m, n, A.nnz)
+        h.InputCSC(A.nnz, row, colptr, cval)
+    key = np.sort(rng.choice(n, k, replace=False)).astype(np.int32)
+    _check(torch, A, h, 2, key, rng.uniform(-1, 1, k).astype(np.float32))
