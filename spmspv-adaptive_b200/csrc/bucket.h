@@ -5,7 +5,6 @@
 namespace spmx {
 
 constexpr int kBucketMax = 16384;  // buckets per call (shared-memory histogram)
-constexpr int kBucketTable = 1024; // at most this many: pairs sorted per block, with a table
 
 struct BucketScratch {
   int* gcount;   // [kBucketMax]
@@ -14,7 +13,6 @@ struct BucketScratch {
   int* prow;     // pair rows   [cap]
   float* pval;   // pair values [cap]
   int cap;
-  unsigned short* tab;  // [(nb + 1) * mg_cap] bucket offsets of the blocks (nb <= kBucketTable)
 };
 
 // rows per bucket = 1 << rshift (256 .. 8192); returns -1 if m needs more

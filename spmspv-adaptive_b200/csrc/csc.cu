@@ -381,16 +381,16 @@ csc_naive_pairs_kernel(CscArgs a, CscScratch s, int* __restrict__ prow,
 }
 
 // --------------------------------------------------------------------------
-// tiles of 512 entries, four times as many CTAs, while the status array holds
-// their look-back words: 105,000 entries 9 us against 14 in tiles of 2,048 (the
-// block tables divide by a constant now), 35,000 6 against 10.7
+// tiles of 512 entries, four times as many CTAs, while these are one wave (8 per
+// SM) and the status array holds their look-back words: 105,000 entries 9 us
+// against 14 in tiles of 2,048, 35,000 6 against 10.7; 1M entries 15 us more
 int launch_csc_scan(const CscArgs& a, const CscScratch& s, ScanScratch& ls, cudaStream_t st) {
   constexpr int NT = kCscScanNT, VT = kCscScanVT, VS = 2;
   if (a.x_nnz <= 0) return 0;
   LookbackState lbs{ls.status, ls.ticket};
   const int small = (int)(((long long)a.x_nnz + NT * VS - 1) / (NT * VS));
   note_launch();
-  if (small <= ls.status_len) {
+  if (small <= 148 * 8 && small <= ls.status_len) {
     csc_scan_kernel<NT, VS><<<small, NT, 0, st>>>(a, s, lbs, small);
     return 0;
   }

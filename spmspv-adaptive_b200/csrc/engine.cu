@@ -254,9 +254,6 @@ static void free_sort_scratch(spmx_handle_t h) {
   dfree(h->sradix); dfree(h->sslot);
   dfree(h->srow);
   dfree(h->bk_gcount); dfree(h->bk_boff); dfree(h->bk_cursor);
-  dfree(h->bk_tab);
-  h->bk_tab = nullptr;
-  h->bk_tab_nb = 0;
   h->bk_gcount = h->bk_boff = h->bk_cursor = nullptr;
   h->sk = h->sk_alt = h->sv = h->sv_alt = nullptr;
   h->sradix = nullptr;
@@ -384,13 +381,18 @@ extern "C" int spmx_input_csc(spmx_handle_t h, int nnz, const int* csc_row,
   return SPMX_SUCCESS;
 }
 
-// The sorted (key, value) write-back up to this many rows accumulates in dense
-// rows and compacts those reached (csc_row_scan), above it where a quarter as many
-// products as rows are to be expected; else the products are sorted by row.
+// The sorted (key, value) write-back and the bucket method up to this many rows
+// accumulate in dense rows and compact those reached (launch_row_scan), above it
+// where a quarter as many products as rows are to be expected; else the products
+// are sorted by row, or into buckets.
 // 8M rows, x of 10 / 10,000 / 100,000 / 1M of 1M columns with four nonzeros each:
 // 58 / 63 / 72 / 108 us against 69 / 82 / 111 / 305 sorted; 1M rows 41 / 41 / 41 / 57
 // against 76 / 88 / 113 / 285; 16M rows 101 / 106 / 120 / 212 against 67 / 84 / 111 /
-// 313; 32M rows and 4M products 338 against 333.
+// 313; 32M rows and 4M products 338 against 333.  Against the buckets: 1M rows 30 /
+// 32 / 36 / 56 against 57 / 71 / 83 / 209, 8M rows 51 / 56 / 66 / 100 against 71 / 82 /
+// 97 / 248, 16M 98 / 101 / 123 / 209 against 83 / 92 / 108 / 266, 32M 171 / 184 / 206 /
+// 334 against 107 / 122 / 140 / 330.  And a row that many columns meet, on which the
+// buckets' shared-memory additions queue: one full row, x of 1M 489 us against 29,000.
 constexpr int kRowScanMax = 1 << 23;
 
 static bool row_scan_fits(spmx_handle_t h) {
@@ -399,20 +401,19 @@ static bool row_scan_fits(spmx_handle_t h) {
 
 static int ensure_sort_scratch(spmx_handle_t h) {
   if (h->sort_ready) return SPMX_SUCCESS;
-  const size_t cap = (size_t)std::max(h->nnz, 1);
-  const size_t ycap = (size_t)std::max(h->m, 1);
-  SPMX_TRY(dalloc((void**)&h->sk, 4 * cap, "sort keys"));
-  SPMX_TRY(dalloc((void**)&h->sv, 4 * cap, "sort vals"));
-  SPMX_TRY(dalloc((void**)&h->srow, 8 * ycap, "row sums"));
+  SPMX_TRY(dalloc((void**)&h->srow, 8 * (size_t)std::max(h->m, 1), "row sums"));
   if (h->m > kRowScanMax) {
+    const size_t cap = (size_t)std::max(h->nnz, 1);
+    SPMX_TRY(dalloc((void**)&h->sk, 4 * cap, "sort keys"));
     SPMX_TRY(dalloc((void**)&h->sk_alt, 4 * cap, "sort keys alt"));
+    SPMX_TRY(dalloc((void**)&h->sv, 4 * cap, "sort vals"));
     SPMX_TRY(dalloc((void**)&h->sv_alt, 4 * cap, "sort vals alt"));
     SPMX_TRY(dalloc((void**)&h->sslot, 4 * cap, "sort slots"));
     SPMX_TRY(dalloc(&h->sradix, radix_scratch_bytes((int)cap), "radix scratch"));
+    SPMX_TRY(dalloc((void**)&h->bk_gcount, 4 * (size_t)kBucketMax, "bucket counts"));
+    SPMX_TRY(dalloc((void**)&h->bk_boff, 4 * (size_t)(kBucketMax + 1), "bucket offsets"));
+    SPMX_TRY(dalloc((void**)&h->bk_cursor, 4 * (size_t)kBucketMax, "bucket cursors"));
   }
-  SPMX_TRY(dalloc((void**)&h->bk_gcount, 4 * (size_t)kBucketMax, "bucket counts"));
-  SPMX_TRY(dalloc((void**)&h->bk_boff, 4 * (size_t)(kBucketMax + 1), "bucket offsets"));
-  SPMX_TRY(dalloc((void**)&h->bk_cursor, 4 * (size_t)kBucketMax, "bucket cursors"));
   h->sort_ready = true;
   return SPMX_SUCCESS;
 }
@@ -696,24 +697,10 @@ static int ensure_csc_scratch(spmx_handle_t h) {
   return SPMX_SUCCESS;
 }
 
-// the bucket offsets of every block, for at most kBucketTable buckets
-static int ensure_bucket_table(spmx_handle_t h, int nb) {
-  if (nb > kBucketTable || nb <= h->bk_tab_nb) return SPMX_SUCCESS;
-  SPMX_CUDA(cudaStreamSynchronize(h->stream));
-  dfree(h->bk_tab);
-  h->bk_tab = nullptr;
-  h->bk_tab_nb = 0;
-  SPMX_TRY(dalloc((void**)&h->bk_tab, 2 * ((size_t)nb + 1) * h->cs.mg_cap, "bucket table"));
-  h->bk_tab_nb = nb;
-  return SPMX_SUCCESS;
-}
-
 extern "C" int spmx_alloc_pre_buffer(spmx_handle_t h) {
   SPMX_CHECK_HANDLE(h);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
-  int rshift = 0, nb = 0;
-  if (!bucket_geometry(h->m, h->buckets, &rshift, &nb)) SPMX_TRY(ensure_bucket_table(h, nb));
   SPMX_TRY(ensure_dense_x(h));
   SPMX_TRY(ensure_bits(h));
   return SPMX_SUCCESS;
@@ -976,22 +963,29 @@ static int csc_atomic(spmx_handle_t h, int variant, float alpha, float* y, int* 
 }
 
 // y's rows are accumulated in double, from -0.0: a row that a nonzero reaches is
-// listed whatever its sum, and the sums lose less to rounding than in the sort
-// (3.5e-8 of the largest against 6.2e-8).
+// listed whatever its sum, and the sums lose less to rounding than in the sort or
+// the buckets (3.5e-8 of the largest against 6.2e-8 and 1.6e-7).
 // What bounds it: the chain of five grids and the read-back of the counts.  Zipf
-// 700,001 rows, x of 35,000 (0.4M products): 40 us a call against 115 for the scan
+// 700,001 rows, x of 35,000 (0.4M products): 39 us a call against 115 for the scan
 // of the columns, the products in column order, their radix sort and a reduction
-// by key, with a read-back after the scan; 21 of the 40 are the grids (fill 2,
-// columns 7, long columns 4, count 3, write 4).
-static int csc_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int* ynnz) {
-  cudaStream_t st = h->stream;
+// by key, with a read-back after the scan; 21 of the 39 are the grids (fill 2,
+// columns 7, long columns 4, count 3, write 4).  Zipf 1M, x of 105,000 (1.7M
+// products) 49 us against 87 in buckets.
+// cap: the products above which the device error flag is raised, -1 for none
+static int launch_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int cap) {
   const CscArgs a = csc_args(h, alpha);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
-  if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->row_max, h->num_sms, st) ||
-      launch_compact_rows(h->m, h->srow, y, ykey, yval, h->d_counts + kCntYnnz, h->ls, st))
-    return set_error(SPMX_ERR_CUDA, "csc sorted spmspv launch");
-  SPMX_TRY(launch_ok("csc sorted spmspv"));
+  if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->row_max, h->num_sms, h->stream) ||
+      launch_compact_rows(h->m, h->srow, y, ykey, yval, h->d_counts + kCntYnnz,
+                          cap < 0 ? nullptr : h->d_counts + kCntBinlen, cap, h->d_err, h->ls, h->stream))
+    return set_error(SPMX_ERR_CUDA, "csc spmspv launch");
+  return launch_ok("csc row scan");
+}
+
+static int csc_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int* ynnz) {
+  cudaStream_t st = h->stream;
+  SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, -1));
   SPMX_CUDA(cudaMemcpyAsync(h->h_pinned, h->d_counts + kCntYnnz, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   SPMX_CUDA(cudaStreamSynchronize(st));
   static_assert(kCntBinlen == kCntYnnz + 1, "read together");
@@ -1125,14 +1119,17 @@ int csc_bucket_impl(spmx_handle_t h, float alpha, float* y, int* ykey, float* yv
   int rshift = 0, nb = 0;
   if (bucket_geometry(h->m, buckets > 0 ? buckets : h->buckets, &rshift, &nb))
     return set_error(SPMX_ERR_INVALID_VALUE, "too many rows for the bucket method");
+  if (row_scan_fits(h)) {
+    SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, h->nnz));
+    if (ynnz) SPMX_TRY(read_counter(h, kCntYnnz, ynnz));
+    return SPMX_SUCCESS;
+  }
   SPMX_TRY(ensure_scan_tiles(h, nb));
-  SPMX_TRY(ensure_bucket_table(h, nb));
   cudaStream_t st = h->stream;
   const CscArgs a = csc_args(h, alpha);
   if (launch_csc_scan(a, h->cs, h->ls, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "scan capacity");
-  BucketScratch bs{h->bk_gcount, h->bk_boff, h->bk_cursor, (int*)h->sk, (float*)h->sv, h->nnz,
-                   h->bk_tab};
+  BucketScratch bs{h->bk_gcount, h->bk_boff, h->bk_cursor, (int*)h->sk, (float*)h->sv, h->nnz};
   if (launch_bucket_spmspv(a, h->cs, bs, SPMX_CSC_LB_MERGE, rshift, nb, y, ykey, yval,
                            h->d_counts + kCntYnnz, h->ls, h->lb_grid, st))
     return set_error(SPMX_ERR_INVALID_VALUE, "bucket launch capacity");

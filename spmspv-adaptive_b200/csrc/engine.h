@@ -73,8 +73,6 @@ struct spmx_handle_s {
   int* bk_boff = nullptr;
   int* bk_cursor = nullptr;
   int buckets = 0;            // 0 = default (256)
-  unsigned short* bk_tab = nullptr;  // bucket offsets per block, bk_tab_nb + 1 rows of cs.mg_cap
-  int bk_tab_nb = 0;
 
   // CSR5 tile tables (csr5.cu) and tiled-SpMV tables (tiled.cu)
   void* csr5 = nullptr;

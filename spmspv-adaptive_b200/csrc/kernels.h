@@ -169,8 +169,9 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st);
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
                            int* d_count, ScanScratch& ls, cudaStream_t st, int limit = 0);
 // keys/vals (each optional) of the entries of acc[0..len) other than -0.0, in
-// order; dense (optional): all of them, rounded, the others 0; count -> *d_count
+// order; dense (optional): all of them, rounded, the others 0; count -> *d_count.
+// *total (optional) above cap: kDevErrCapacity
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        ScanScratch& ls, cudaStream_t st);
+                        const int* total, int cap, int* err, ScanScratch& ls, cudaStream_t st);
 
 }  // namespace spmx

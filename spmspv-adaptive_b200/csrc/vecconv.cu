@@ -112,7 +112,7 @@ template <int NT, int VT, class T>
 __global__ void __launch_bounds__(NT)
 compact_write_kernel(long long len, long long per, const T* __restrict__ in, const unsigned* __restrict__ counts,
                      float* __restrict__ dense, int* __restrict__ key, float* __restrict__ val, int* d_count,
-                     unsigned limit) {
+                     unsigned limit, const int* __restrict__ total, int cap, int* err) {
   constexpr bool ROWS = sizeof(T) == 8;
   constexpr int NW = NT / 32;
   __shared__ unsigned s_cnt[VT * NW];
@@ -201,7 +201,10 @@ compact_write_kernel(long long len, long long per, const T* __restrict__ in, con
     run += total;
     __syncthreads();
   }
-  if (blockIdx.x == gridDim.x - 1 && tid == 0) *d_count = (int)run;
+  if (blockIdx.x == gridDim.x - 1 && tid == 0) {
+    *d_count = (int)run;
+    if (ROWS && total && *(const volatile int*)total > cap) flag_error(err, kDevErrCapacity);
+  }
 }
 
 int launch_scatter(int nvals, int len, const int* key, const float* val,
@@ -240,7 +243,7 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st) {
 
 template <class T>
 static int launch_compact(int len, const T* in, float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
-                          cudaStream_t st, int limit) {
+                          cudaStream_t st, int limit, const int* total, int cap, int* err) {
   constexpr int NT = 256, VT = 8;
   if (len <= 0) { cudaMemsetAsync(d_count, 0, sizeof(int), st); return 0; }
   // ranges of whole sub-tiles, at most kCompactMaxRanges of them
@@ -253,19 +256,19 @@ static int launch_compact(int len, const T* in, float* dense, int* key, float* v
   if (launch_pdl(compact_count_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
                  ls.counts) != cudaSuccess ||
       launch_pdl(compact_write_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
-                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit) != cudaSuccess)
+                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit, total, cap, err) != cudaSuccess)
     return -2;
   return 0;
 }
 
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
                            cudaStream_t st, int limit) {
-  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit);
+  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit, nullptr, 0, nullptr);
 }
 
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        ScanScratch& ls, cudaStream_t st) {
-  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0);
+                        const int* total, int cap, int* err, ScanScratch& ls, cudaStream_t st) {
+  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0, total, cap, err);
 }
 
 }  // namespace spmx

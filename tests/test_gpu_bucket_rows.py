@@ -1,7 +1,6 @@
-"""The bucket SpMSpV that sorts pairs per block: bucket counts around the table's
-limit (1,024), more buckets than threads, one bucket, blocks with no pair in most
-buckets, rows of many pairs, x sizes around the tiles of the column scan (512
-entries), a row out of range, and its outputs in every combination."""
+"""The bucket SpMSpV: bucket counts asked for from 1 to 4,000, rows of many pairs, x
+sizes around 512 and 4,096 entries, a row out of range, and its outputs in every
+combination."""
 import numpy as np
 import pytest
 

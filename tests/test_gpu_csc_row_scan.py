@@ -76,7 +76,8 @@ def test_repeated_keys_beyond_the_nonzeros(torch_cuda, variant):
 
 @pytest.mark.parametrize("m", [1 << 23, (1 << 23) + 1])
 @pytest.mark.parametrize("k", [3, 64])
-def test_many_rows(torch_cuda, m, k):
+@pytest.mark.parametrize("variant", [1, 3])
+def test_many_rows(torch_cuda, m, k, variant):
     from spmx.gen import Csr
     torch = torch_cuda
     rng = np.random.default_rng(k)
@@ -87,7 +88,8 @@ def test_many_rows(torch_cuda, m, k):
     A = Csr(m, 64, rowptr, rng.integers(0, 64, nnz).astype(np.int32), rng.uniform(-1, 1, nnz).astype(np.float32))
     h = make_handle(A, torch, hola=False)
     key = np.sort(rng.choice(64, k, replace=False)).astype(np.int32)
-    _check(torch, A, h, 1, key, rng.uniform(-1, 1, k).astype(np.float32), "keyval")
+    _check(torch, A, h, variant, key, rng.uniform(-1, 1, k).astype(np.float32), "keyval")
+    _check(torch, A, h, variant, key, rng.uniform(-1, 1, k).astype(np.float32), "all")
 
 
 @pytest.mark.parametrize("csr", [True, False])
