@@ -578,10 +578,14 @@ extern "C" int spmx_sparse2bitarray(spmx_handle_t h) {
 
 static int dense_to_sparse(spmx_handle_t h, int len, const float* dense, int* key,
                            float* val, int slot, int* host_count) {
-  if (launch_compact_nonzero(len, dense, key, val, h->d_counts + slot, h->ls, h->stream))
+  if (launch_compact_nonzero(len, dense, key, val, h->d_counts + slot, h->ls, h->stream, 0,
+                             host_count ? h->h_pinned : nullptr))
     return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
   SPMX_TRY(launch_ok("dense2sparse"));
-  if (host_count) SPMX_TRY(read_counter(h, slot, host_count));
+  if (host_count) {
+    SPMX_CUDA(cudaStreamSynchronize(h->stream));
+    *host_count = h->h_pinned[0];
+  }
   return SPMX_SUCCESS;
 }
 
@@ -966,29 +970,29 @@ static int csc_atomic(spmx_handle_t h, int variant, float alpha, float* y, int* 
 // listed whatever its sum, and the sums lose less to rounding than in the sort or
 // the buckets (3.5e-8 of the largest against 6.2e-8 and 1.6e-7).
 // What bounds it: the chain of five grids and the read-back of the counts.  Zipf
-// 700,001 rows, x of 35,000 (0.4M products): 39 us a call against 115 for the scan
+// 700,001 rows, x of 35,000 (0.4M products): 33 us a call against 115 for the scan
 // of the columns, the products in column order, their radix sort and a reduction
-// by key, with a read-back after the scan; 21 of the 39 are the grids (fill 2,
+// by key, with a read-back after the scan; 21 of the 33 are the grids (fill 2,
 // columns 7, long columns 4, count 3, write 4).  Zipf 1M, x of 105,000 (1.7M
-// products) 49 us against 87 in buckets.
-// cap: the products above which the device error flag is raised, -1 for none
-static int launch_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int cap) {
+// products) 42 us against 87 in buckets.
+// cap: the products above which the device error flag is raised, -1 for none;
+// h_counts: rows listed and products, written by the last grid (a copy behind it
+// costs 7 us more)
+static int launch_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int cap, int* h_counts) {
   const CscArgs a = csc_args(h, alpha);
   SPMX_TRY(ensure_csc_scratch(h));
   SPMX_TRY(ensure_sort_scratch(h));
   if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->row_max, h->num_sms, h->stream) ||
       launch_compact_rows(h->m, h->srow, y, ykey, yval, h->d_counts + kCntYnnz,
-                          cap < 0 ? nullptr : h->d_counts + kCntBinlen, cap, h->d_err, h->ls, h->stream))
+                          h->d_counts + kCntBinlen, cap, h->d_err, h_counts, h->ls, h->stream))
     return set_error(SPMX_ERR_CUDA, "csc spmspv launch");
   return launch_ok("csc row scan");
 }
 
 static int csc_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, float* yval, int* ynnz) {
   cudaStream_t st = h->stream;
-  SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, -1));
-  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned, h->d_counts + kCntYnnz, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, -1, h->h_pinned));
   SPMX_CUDA(cudaStreamSynchronize(st));
-  static_assert(kCntBinlen == kCntYnnz + 1, "read together");
   h->bin_len = h->h_pinned[1];
   if (h->bin_len > h->nnz) return set_error(SPMX_ERR_INVALID_VALUE, "bin_len exceeds nnz: duplicate x keys");
   if (ynnz) *ynnz = h->h_pinned[0];
@@ -1120,8 +1124,11 @@ int csc_bucket_impl(spmx_handle_t h, float alpha, float* y, int* ykey, float* yv
   if (bucket_geometry(h->m, buckets > 0 ? buckets : h->buckets, &rshift, &nb))
     return set_error(SPMX_ERR_INVALID_VALUE, "too many rows for the bucket method");
   if (row_scan_fits(h)) {
-    SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, h->nnz));
-    if (ynnz) SPMX_TRY(read_counter(h, kCntYnnz, ynnz));
+    SPMX_TRY(launch_row_scan(h, alpha, y, ykey, yval, h->nnz, ynnz ? h->h_pinned : nullptr));
+    if (ynnz) {
+      SPMX_CUDA(cudaStreamSynchronize(h->stream));
+      *ynnz = h->h_pinned[0];
+    }
     return SPMX_SUCCESS;
   }
   SPMX_TRY(ensure_scan_tiles(h, nb));

@@ -165,13 +165,17 @@ int launch_scatter(int nvals, int len, const int* key, const float* val,
                    float* dense, int* bits, int* err, cudaStream_t st);
 int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st);
 // keys/vals of the entries != 0 of dense[0..len), in order; count -> *d_count.
-// limit > 0: nothing but the count is written where it reaches the limit
+// limit > 0: nothing but the count is written where it reaches the limit.
+// h_counts (optional, two ints of page-locked host memory; without a limit): the
+// count once the grid is done
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
-                           int* d_count, ScanScratch& ls, cudaStream_t st, int limit = 0);
+                           int* d_count, ScanScratch& ls, cudaStream_t st, int limit = 0,
+                           int* h_counts = nullptr);
 // keys/vals (each optional) of the entries of acc[0..len) other than -0.0, in
 // order; dense (optional): all of them, rounded, the others 0; count -> *d_count.
-// *total (optional) above cap: kDevErrCapacity
+// *total above cap >= 0: kDevErrCapacity.  h_counts (optional, page-locked host
+// memory): the count and *total once the grid is done
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        const int* total, int cap, int* err, ScanScratch& ls, cudaStream_t st);
+                        const int* total, int cap, int* err, int* h_counts, ScanScratch& ls, cudaStream_t st);
 
 }  // namespace spmx

@@ -112,7 +112,7 @@ template <int NT, int VT, class T>
 __global__ void __launch_bounds__(NT)
 compact_write_kernel(long long len, long long per, const T* __restrict__ in, const unsigned* __restrict__ counts,
                      float* __restrict__ dense, int* __restrict__ key, float* __restrict__ val, int* d_count,
-                     unsigned limit, const int* __restrict__ total, int cap, int* err) {
+                     unsigned limit, const int* __restrict__ total, int cap, int* err, int* h_counts) {
   constexpr bool ROWS = sizeof(T) == 8;
   constexpr int NW = NT / 32;
   __shared__ unsigned s_cnt[VT * NW];
@@ -203,7 +203,12 @@ compact_write_kernel(long long len, long long per, const T* __restrict__ in, con
   }
   if (blockIdx.x == gridDim.x - 1 && tid == 0) {
     *d_count = (int)run;
-    if (ROWS && total && *(const volatile int*)total > cap) flag_error(err, kDevErrCapacity);
+    if (h_counts) h_counts[0] = (int)run;
+    if (ROWS) {
+      const int products = *(const volatile int*)total;
+      if (cap >= 0 && products > cap) flag_error(err, kDevErrCapacity);
+      if (h_counts) h_counts[1] = products;
+    }
   }
 }
 
@@ -243,9 +248,13 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st) {
 
 template <class T>
 static int launch_compact(int len, const T* in, float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
-                          cudaStream_t st, int limit, const int* total, int cap, int* err) {
+                          cudaStream_t st, int limit, const int* total, int cap, int* err, int* h_counts) {
   constexpr int NT = 256, VT = 8;
-  if (len <= 0) { cudaMemsetAsync(d_count, 0, sizeof(int), st); return 0; }
+  if (len <= 0) {
+    cudaMemsetAsync(d_count, 0, sizeof(int), st);
+    if (h_counts) h_counts[0] = h_counts[1] = 0;
+    return 0;
+  }
   // ranges of whole sub-tiles, at most kCompactMaxRanges of them
   const long long sub = NT * VT;
   const long long subs = (len + sub - 1) / sub;
@@ -256,19 +265,20 @@ static int launch_compact(int len, const T* in, float* dense, int* key, float* v
   if (launch_pdl(compact_count_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
                  ls.counts) != cudaSuccess ||
       launch_pdl(compact_write_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
-                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit, total, cap, err) != cudaSuccess)
+                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit, total, cap, err,
+                 h_counts) != cudaSuccess)
     return -2;
   return 0;
 }
 
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
-                           cudaStream_t st, int limit) {
-  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit, nullptr, 0, nullptr);
+                           cudaStream_t st, int limit, int* h_counts) {
+  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit, nullptr, -1, nullptr, h_counts);
 }
 
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        const int* total, int cap, int* err, ScanScratch& ls, cudaStream_t st) {
-  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0, total, cap, err);
+                        const int* total, int cap, int* err, int* h_counts, ScanScratch& ls, cudaStream_t st) {
+  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0, total, cap, err, h_counts);
 }
 
 }  // namespace spmx
