@@ -94,10 +94,12 @@ spmv_backward_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
 // (cp.async), and the bounds and dy of its rows are on their way into registers.
 //
 // What bounds it: the 21M reductions into dx, then DRAM (340 MB).  5-point
-// Laplacian 2048^2 (21.0M nonzeros): 82 us against 136 with the rows found by a
+// Laplacian 2048^2 (21.0M nonzeros): 80 us against 136 with the rows found by a
 // scan of marks; one thread walking each row, so that the reductions of
 // neighbouring lanes fall on neighbouring entries, took 89 (chunk by chunk) and
-// 92 us (persistent).
+// 92 us (persistent).  512 threads per chunk in three CTAs 80 us, in four 83, 256 in
+// four 84 (86 with a range check per element); dvals alone 57, 48 and 53 us, so
+// four there.
 template <int NT, int VT>
 struct BackwardChunk {
   static constexpr int K = NT * VT;
@@ -107,13 +109,34 @@ struct BackwardChunk {
 };
 
 // every nonzero of a staged chunk: its dvals entry and its share of dx
-template <int NT, int VT, bool FULL>
+template <int NT, int VT, bool FULL, bool DX, bool DV>
 __device__ __forceinline__ void backward_elements(const BackwardChunk<NT, VT>& t, int n, int cnt,
                                                   const float* __restrict__ x, float* __restrict__ dx,
                                                   float* __restrict__ dvals, int* err) {
   const int e0 = threadIdx.x;
   int c[VT];
   float xv[VT];
+  if (FULL) {  // every column in range: no check per element
+    unsigned top = 0;
+#pragma unroll
+    for (int j = 0; j < VT; ++j) {
+      c[j] = t.col[e0 + j * NT];
+      top = max(top, (unsigned)c[j]);
+    }
+    if (top < (unsigned)n) {
+      if (DV) {
+#pragma unroll
+        for (int j = 0; j < VT; ++j) xv[j] = __ldg(x + c[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < VT; ++j) {
+        const float g = t.g[e0 + j * NT];
+        if (DX && g != 0.0f) atomicAdd(dx + c[j], t.val[e0 + j * NT] * g);
+        if (DV) __stcs(dvals + e0 + j * NT, g * xv[j]);
+      }
+      return;
+    }
+  }
   bool bad = false;
 #pragma unroll
   for (int j = 0; j < VT; ++j) {
@@ -122,20 +145,20 @@ __device__ __forceinline__ void backward_elements(const BackwardChunk<NT, VT>& t
     const bool ok = (unsigned)c[j] < (unsigned)n;
     bad |= !ok;
     if (!ok || !in) c[j] = -1;
-    xv[j] = dvals && c[j] >= 0 ? __ldg(x + c[j]) : 0.f;
+    xv[j] = DV && c[j] >= 0 ? __ldg(x + c[j]) : 0.f;
   }
 #pragma unroll
   for (int j = 0; j < VT; ++j) {
     if (c[j] < 0) continue;
     const float g = t.g[e0 + j * NT];
-    if (dx && g != 0.0f) atomicAdd(dx + c[j], t.val[e0 + j * NT] * g);
-    if (dvals) __stcs(dvals + e0 + j * NT, g * xv[j]);
+    if (DX && g != 0.0f) atomicAdd(dx + c[j], t.val[e0 + j * NT] * g);
+    if (DV) __stcs(dvals + e0 + j * NT, g * xv[j]);
   }
   if (bad) flag_error(err, kDevErrOob);
 }
 
-template <int NT, int VT>
-__global__ void __launch_bounds__(NT, 4)
+template <int NT, int VT, int CTAS, bool DX, bool DV>
+__global__ void __launch_bounds__(NT, CTAS)
 spmv_backward_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __restrict__ col,
                            const float* __restrict__ val, const float* __restrict__ x,
                            const float* __restrict__ dy, const int4* __restrict__ list, int count,
@@ -154,12 +177,12 @@ spmv_backward_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const
       if (vec_ok && cnt == K) {
         for (int q = threadIdx.x; q < K / 4; q += NT) {
           cp_async16(sh[into].col + 4 * q, col + s + 4 * q);
-          if (dx) cp_async16(sh[into].val + 4 * q, val + s + 4 * q);
+          if (DX) cp_async16(sh[into].val + 4 * q, val + s + 4 * q);
         }
       } else {
         for (int q = threadIdx.x; q < cnt; q += NT) {
           cp_async4(sh[into].col + q, col + s + q);
-          if (dx) cp_async4(sh[into].val + q, val + s + q);
+          if (DX) cp_async4(sh[into].val + q, val + s + q);
         }
       }
 #pragma unroll
@@ -196,8 +219,8 @@ spmv_backward_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const
     cp_async_wait<0>();
     __syncthreads();  // the chunk is complete, and nobody reads the other one any more
     load(d1, buf ^ 1);
-    if (cnt == K) backward_elements<NT, VT, true>(t, n, K, x, dx, dvals ? dvals + s : nullptr, err);
-    else backward_elements<NT, VT, false>(t, n, cnt, x, dx, dvals ? dvals + s : nullptr, err);
+    if (cnt == K) backward_elements<NT, VT, true, DX, DV>(t, n, K, x, dx, DV ? dvals + s : nullptr, err);
+    else backward_elements<NT, VT, false, DX, DV>(t, n, cnt, x, dx, DV ? dvals + s : nullptr, err);
     buf ^= 1;
     d = d1;
     d1 = d2;
@@ -321,11 +344,15 @@ int launch_spmv_backward(int m, int n, int nnz, const int* rowptr, const int* co
   const int nlong = t.nchunks - t.n_short;
   note_launch((t.n_short > 0) + (nlong > 0));
   if (t.n_short > 0) {
-    constexpr int smem = 2 * sizeof(BackwardChunk<256, 8>);
-    const auto kernel = spmv_backward_short_kernel<256, 8>;
+    constexpr int NT = 512, VT = 4;
+    constexpr int smem = 2 * sizeof(BackwardChunk<NT, VT>);
+    const auto kernel = !dvals ? spmv_backward_short_kernel<NT, VT, 3, true, false>
+                        : dx   ? spmv_backward_short_kernel<NT, VT, 3, true, true>
+                               : spmv_backward_short_kernel<NT, VT, 4, false, true>;
     if (kernel_smem_limit((const void*)kernel, smem) != cudaSuccess) return -2;
-    const int rounds = (t.n_short + 148 * 4 - 1) / (148 * 4);
-    kernel<<<(t.n_short + rounds - 1) / rounds, 256, smem, st>>>(
+    const int cap = 148 * (dx ? 3 : 4);
+    const int rounds = (t.n_short + cap - 1) / cap;
+    kernel<<<(t.n_short + rounds - 1) / rounds, NT, smem, st>>>(
         n, nnz, rowptr, col, val, x, dy, t.list, t.n_short, dx, dvals,
         (((uintptr_t)col | (uintptr_t)val) & 15u) == 0, gate, err);
   }

@@ -123,19 +123,23 @@ __device__ __forceinline__ void split_row_contribute(
 // element by element with coalesced loads, and every row is then summed by one
 // thread, in column order; no scan.  Persistent CTAs: the loads of a CTA's next
 // chunk are in flight while this one's rows are summed, the descriptor of the
-// one after too.  With `whole` (every chunk of the matrix is short) a chunk also
-// reads the up to kShortRow nonzeros past its end that its last row may have, so
-// no row is split; otherwise split rows meet as in spmv_chunk_kernel.
+// one after too.  WHOLE (every chunk of the matrix is short): a chunk also reads
+// the up to kShortRow nonzeros past its end that its last row may have, so no row
+// is split; otherwise split rows meet as in spmv_chunk_kernel.
 //
-// What bounds it: DRAM latency ahead of DRAM bandwidth.  5-point Laplacian 2048^2
-// (21.0M nonzeros, 218 MB): 52 us (4.2 TB/s) against 97 by the segmented scan; one
-// CTA per chunk without the loads ahead 78 us, one thread gathering for each row
-// from staged columns and values 88 to 94 us (300 instructions per row).
-template <int NT, int VT, bool GATED>
+// What bounds it: instruction issue, then DRAM latency.  5-point Laplacian 2048^2
+// (21.0M nonzeros, 218 MB): 43 us (5.1 TB/s) with no check per element where the
+// chunk is inside the matrix and its largest column in range, 49 with them (47
+// warp instructions per 32 nonzeros), 97 by the segmented scan; one CTA per chunk
+// without the loads ahead 78 us, one thread gathering for each row from staged
+// columns and values 88 to 94 us.  Row sums in predicated blocks of two, four and
+// eight 45 to 47 us, 512 threads per chunk 51 us, conversions to FP64 by integer
+// operations 57.
+template <int NT, int VT, bool GATED, bool WHOLE>
 __global__ void __launch_bounds__(NT, 1024 / NT)
 spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __restrict__ col,
                   const float* __restrict__ val, const float* __restrict__ x, const int* __restrict__ bits,
-                  double alpha, float* __restrict__ y, const int4* __restrict__ list, int count, int whole,
+                  double alpha, float* __restrict__ y, const int4* __restrict__ list, int count,
                   double* carry, unsigned* arrive, int* err) {
   constexpr int K = NT * VT;
   extern __shared__ double s_short[];  // two buffers of K + kShortRow products
@@ -145,16 +149,32 @@ spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __r
   const auto load = [&](const int4& d) {
     if (d.x < 0) return;
     const int s = d.x * K, left = nnz - s;
+    const int* const cp = col + s + threadIdx.x;
+    const float* const vp = val + s + threadIdx.x;
+    cc[VT] = 0;
+    vv[VT] = 0.f;
+    if (left >= K + kShortRow) {
 #pragma unroll
-    for (int j = 0; j <= VT; ++j) {
-      const int q = j * NT + threadIdx.x;
-      const bool in = q < left && (j < VT || (whole && threadIdx.x < kShortRow));
-      cc[j] = in ? __ldcs(col + s + q) : 0;
-      vv[j] = in ? __ldcs(val + s + q) : 0.f;
+      for (int j = 0; j < VT; ++j) {
+        cc[j] = __ldcs(cp + j * NT);
+        vv[j] = __ldcs(vp + j * NT);
+      }
+      if (WHOLE && threadIdx.x < kShortRow) {
+        cc[VT] = __ldcs(cp + K);
+        vv[VT] = __ldcs(vp + K);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j <= VT; ++j) {
+        const int q = j * NT + threadIdx.x;
+        const bool in = q < left && (j < VT || (WHOLE && threadIdx.x < kShortRow));
+        cc[j] = in ? __ldcs(cp + j * NT) : 0;
+        vv[j] = in ? __ldcs(vp + j * NT) : 0.f;
+      }
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const int r = d.y - 1 + whole + (int)threadIdx.x + q * NT;
+      const int r = d.y - 1 + WHOLE + (int)threadIdx.x + q * NT;
       const bool in = r >= 0 && r < d.z;
       ra[q] = in ? __ldg(rowptr + r) : 0;
       rb[q] = in ? __ldg(rowptr + r + 1) : 0;
@@ -166,17 +186,29 @@ spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __r
   for (long long i = blockIdx.x; i < count; i += gridDim.x) {
     const int4 d2 = desc(i + 2LL * gridDim.x);
     double* const s_p = s_short + buf * (K + kShortRow);
-    bool bad = false;
+    unsigned top = 0;
 #pragma unroll
-    for (int j = 0; j <= VT; ++j) {
-      if (j == VT && threadIdx.x >= kShortRow) break;
-      bool use = (unsigned)cc[j] < (unsigned)n;
-      bad |= !use;
-      if (GATED) use = use && bit_is_set(bits, cc[j]);
-      const float xv = use ? __ldg(x + cc[j]) : 0.f;
-      s_p[j * NT + threadIdx.x] = use ? (double)vv[j] * (double)xv : 0.0;
+    for (int j = 0; j <= VT; ++j) top = max(top, (unsigned)cc[j]);
+    if (!GATED && top < (unsigned)n) {
+      float xv[VT];
+#pragma unroll
+      for (int j = 0; j < VT; ++j) xv[j] = __ldg(x + cc[j]);
+#pragma unroll
+      for (int j = 0; j < VT; ++j) s_p[j * NT + threadIdx.x] = (double)vv[j] * (double)xv[j];
+      if (WHOLE && threadIdx.x < kShortRow) s_p[K + threadIdx.x] = (double)vv[VT] * (double)__ldg(x + cc[VT]);
+    } else {
+      bool bad = false;
+#pragma unroll
+      for (int j = 0; j <= VT; ++j) {
+        if (j == VT && threadIdx.x >= kShortRow) break;
+        bool use = (unsigned)cc[j] < (unsigned)n;
+        bad |= !use;
+        if (GATED) use = use && bit_is_set(bits, cc[j]);
+        const float xv = use ? __ldg(x + cc[j]) : 0.f;
+        s_p[j * NT + threadIdx.x] = use ? (double)vv[j] * (double)xv : 0.0;
+      }
+      if (bad) flag_error(err, kDevErrOob);
     }
-    if (bad) flag_error(err, kDevErrOob);
     const int c = d.x, lo = d.y, hi = d.z, s = c * K, e = (int)min((long long)s + K, (long long)nnz);
     const int a0 = ra[0], b0 = rb[0], a1 = ra[1], b1 = rb[1];
     load(d1);
@@ -184,21 +216,21 @@ spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __r
     // chunk before) any more once this barrier is behind everybody
     __syncthreads();
     int q = 0;
-    for (int r = lo - 1 + whole + (int)threadIdx.x; r < hi; r += NT, ++q) {
+    for (int r = lo - 1 + WHOLE + (int)threadIdx.x; r < hi; r += NT, ++q) {
       if (r < 0) continue;
       int a = q == 0 ? a0 : a1, b = q == 0 ? b0 : b1;
       if (q > 1) {
         a = __ldg(rowptr + r);
         b = __ldg(rowptr + r + 1);
       }
-      const int p1 = (whole ? b : min(b, e)) - s;
+      const int p1 = (WHOLE ? b : min(b, e)) - s;
       double sum = 0.0;
       for (int p = max(a, s) - s; p < p1; ++p) sum += s_p[p];
       if (r < lo) {
         if (b > s) split_row_contribute<K>(r, c, 0, sum, rowptr, carry, arrive, alpha, y);
       } else if (b == a) {
         y[r] = 0.f;
-      } else if (whole || b <= e) {
+      } else if (WHOLE || b <= e) {
         y[r] = (float)(alpha * sum);
       } else {
         split_row_contribute<K>(r, c, 1, sum, rowptr, carry, arrive, alpha, y);
@@ -382,14 +414,15 @@ int launch_spmv_hola(const SpmvArgs& a, const HolaTables& t, cudaStream_t st) {
 #define SPMX_HOLA_CASE(VT)                                                       \
   case VT: {                                                                     \
     if (t.n_short > 0) {                                                         \
-      auto kernel = a.bits ? spmv_short_kernel<NT, VT, true> : spmv_short_kernel<NT, VT, false>; \
+      auto kernel = nlong == 0 ? (a.bits ? spmv_short_kernel<NT, VT, true, true> : spmv_short_kernel<NT, VT, false, true>) \
+                               : (a.bits ? spmv_short_kernel<NT, VT, true, false> : spmv_short_kernel<NT, VT, false, false>); \
       constexpr int smem = 16 * (NT * VT + kShortRow);                           \
       e = kernel_smem_limit((const void*)kernel, smem);                          \
       const int cap = 148 * std::min(1024 / NT, (227 << 10) / (smem + 1024));    \
       const int rounds = (t.n_short + cap - 1) / cap;                            \
       if (e == cudaSuccess)                                                      \
         kernel<<<(t.n_short + rounds - 1) / rounds, NT, smem, st>>>(             \
-            a.n, a.nnz, a.rowptr, a.col, a.val, a.x, a.bits, a.alpha, a.y, t.list, t.n_short, nlong == 0, t.carry, \
+            a.n, a.nnz, a.rowptr, a.col, a.val, a.x, a.bits, a.alpha, a.y, t.list, t.n_short, t.carry, \
             t.arrive, a.err);                                                    \
     }                                                                            \
     if (nlong > 0) {                                         \
