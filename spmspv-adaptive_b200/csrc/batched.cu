@@ -45,11 +45,16 @@ constexpr int kBatchMaxVec = 1024;  // nvec limit (shared row accumulators)
 // Row chunks of the row walks: a row weighs its nonzeros plus kBatchRowCost
 // (the fixed cost of a row: its Y row store and its latency chain); chunk k
 // holds the rows whose prefix weight rowptr[i] + kBatchRowCost * i starts in
-// [k * kBatchChunk, (k + 1) * kBatchChunk).  Warps take chunks in order from
+// [k, k + 1) times the chunk's weight.  Warps take chunks in order from
 // a device counter, so the heavy rows (of a power-law matrix numbered by
 // weight, the first ones) spread over the warps instead of landing one per
 // warp in the first pass of a cyclic assignment.
-constexpr int kBatchChunk = 2048;
+// Chunks of 2,048, or smaller ones in a matrix of fewer than 32,768 such: with two
+// chunks per warp the last ones to finish held half of the chip idle (262,144
+// vertices x 256: 8,192 chunks 440 + 537 us forward and backward, 16,384 361 + 496,
+// 32,768 315 + 414; 65,536 301 + 393, but 300,001 x 16 180 + 182 against 174 + 178:
+// a chunk costs an atomic on one address, about 2 ns).
+constexpr int kBatchChunk = 2048, kBatchChunkMin = 128, kBatchChunks = 32768;
 constexpr int kBatchRowCost = 32;
 // Rows above this are taken by whole CTAs before the row walk starts: one warp
 // alone on a hub row (10,000 nonzeros, 300 dependent steps) was the tail of the
@@ -87,16 +92,17 @@ __global__ void batch_bounds_kernel(int total, const unsigned* __restrict__ skey
   }
 }
 
-// chunk_row[k] = first row i with rowptr[i] + kBatchRowCost * i >= k * kBatchChunk
+// chunk_row[k] = first row i with rowptr[i] + kBatchRowCost * i >= k * chunk
 // (chunk_row[nch] = m)
-__global__ void batch_chunks_kernel(int m, const int* __restrict__ rowptr, int nch, int* __restrict__ chunk_row) {
+__global__ void batch_chunks_kernel(int m, const int* __restrict__ rowptr, int nch, long long chunk,
+                                    int* __restrict__ chunk_row) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k > nch) return;
   if (k == nch) {
     chunk_row[k] = m;
     return;
   }
-  const long long target = (long long)k * kBatchChunk;
+  const long long target = k * chunk;
   int lo = 0, hi = m;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
@@ -570,7 +576,8 @@ static int batch_invert(spmx_handle_t h, int nvec, int total, const int* xptr, c
 static int ensure_batch_chunks(spmx_handle_t h) {
   if (h->batch_chunk_ready) return SPMX_SUCCESS;
   const long long w = (long long)h->nnz + (long long)kBatchRowCost * h->m;
-  const long long nch = w / kBatchChunk + 1;
+  const long long chunk = std::min<long long>(kBatchChunk, std::max<long long>(w / kBatchChunks, kBatchChunkMin));
+  const long long nch = w / chunk + 1;
   if (nch >= INT32_MAX) return set_error(SPMX_ERR_INVALID_VALUE, "batched SpMSpV: too many row chunks");
   if (!h->batch_chunk || h->batch_nch != (int)nch) {
     dfree(h->batch_chunk);
@@ -584,7 +591,7 @@ static int ensure_batch_chunks(spmx_handle_t h) {
   note_launch();
   batch_hubs_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->m, h->rowptr, h->batch_hub, h->batch_ctr + 4);
   note_launch();
-  batch_chunks_kernel<<<(unsigned)((nch + 1 + 255) / 256), 256, 0, h->stream>>>(h->m, h->rowptr, (int)nch,
+  batch_chunks_kernel<<<(unsigned)((nch + 1 + 255) / 256), 256, 0, h->stream>>>(h->m, h->rowptr, (int)nch, chunk,
                                                                                 h->batch_chunk);
   h->batch_nch = (int)nch;
   h->batch_chunk_ready = true;

@@ -49,3 +49,35 @@ def test_hub_rows(torch_cuda, nvec, hubs, options):
     assert orc.within_tol(dvals.cpu().numpy(), e, mag, RTOL)[0]
     g, gm = 0.5 * (D.T @ dY)[xkey, vec], 0.5 * (abs(D.T) @ abs(dY))[xkey, vec]
     assert orc.within_tol(dxval.cpu().numpy(), g, gm, RTOL)[0]
+
+
+@pytest.mark.parametrize("m", [130_000, 131_073, 200_001])
+def test_row_chunk_sizes(torch_cuda, m):
+    """Row chunks between the smallest (128) and the largest weight: row counts
+    on both sides of the first size above 128 (a row weighs its nonzeros + 32)."""
+    torch = torch_cuda
+    lens = np.random.default_rng(m).integers(0, 3, m)
+    rowptr = np.r_[0, np.cumsum(lens)].astype(np.int32)
+    from spmx.gen import Csr
+    rng = np.random.default_rng(7)
+    A = Csr(m, 50, rowptr, rng.integers(0, 50, rowptr[-1]).astype(np.int32),
+            rng.standard_normal(rowptr[-1]).astype(np.float32))
+    h = make_handle(A, torch, csc=False, hola=False)
+    nvec = 3
+    X = rng.standard_normal((50, nvec)).astype(np.float32)
+    xptr = np.arange(nvec + 1, dtype=np.int32) * 50
+    xkey, xval = np.tile(np.arange(50, dtype=np.int32), nvec), np.ascontiguousarray(X.T).ravel()
+    xp, xk, xv = (dev(a, torch) for a in (xptr, xkey, xval))
+    dY = rng.standard_normal((m, nvec)).astype(np.float32)
+    Y, dvals = torch.full((m, nvec), 9.0, device="cuda"), torch.full((A.nnz,), 9.0, device="cuda")
+    h.spmspv_batched(xp, xk, xv, 1.0, Y)
+    h.spmspv_batched_backward(xp, xk, xv, 1.0, dev(dY, torch), None, dvals)
+    h.check_device_error()
+    row = np.repeat(np.arange(m), lens)
+    prod = A.val[:, None].astype(np.float64) * X[A.col]
+    want, mag = np.zeros((m, nvec)), np.zeros((m, nvec))
+    np.add.at(want, row, prod)
+    np.add.at(mag, row, np.abs(prod))
+    assert orc.within_tol(Y.cpu().numpy(), want, mag, RTOL)[0]
+    each = dY[row].astype(np.float64) * X[A.col]
+    assert orc.within_tol(dvals.cpu().numpy(), each.sum(1), np.abs(each).sum(1), RTOL)[0]
