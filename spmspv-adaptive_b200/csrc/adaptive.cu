@@ -288,18 +288,24 @@ static int bfs_stepped(spmx_handle_t h, int source, int* levels, int* depth);
 
 static int ensure_bfs(spmx_handle_t h) {
   if (h->bfs_n == h->n && h->bfs_visited) return SPMX_SUCCESS;
-  dfree(h->bfs_visited); dfree(h->bfs_front); dfree(h->bfs_q[0]); dfree(h->bfs_q[1]);
-  dfree(h->bfs_cnt); dfree(h->bfs_edges); dfree(h->bfs_fb1); dfree(h->bfs_fb2); dfree(h->bfs_ctrl);
-  const size_t words = (size_t)std::max((h->n + 31) / 32, 1);
-  SPMX_TRY(dalloc((void**)&h->bfs_visited, 4 * words, "bfs visited"));
-  SPMX_TRY(dalloc((void**)&h->bfs_front, 4 * words, "bfs front"));
-  SPMX_TRY(dalloc((void**)&h->bfs_fb1, 4 * words, "bfs front 1"));
-  SPMX_TRY(dalloc((void**)&h->bfs_fb2, 4 * words, "bfs front 2"));
-  SPMX_TRY(dalloc((void**)&h->bfs_q[0], 8 * (size_t)std::max(h->n, 1), "bfs queue 0"));
-  SPMX_TRY(dalloc((void**)&h->bfs_q[1], 8 * (size_t)std::max(h->n, 1), "bfs queue 1"));
-  SPMX_TRY(dalloc((void**)&h->bfs_cnt, 4 * 4, "bfs counts"));
-  SPMX_TRY(dalloc((void**)&h->bfs_edges, 8 * 4, "bfs edges"));
-  SPMX_TRY(dalloc((void**)&h->bfs_ctrl, sizeof(BfsCtrl), "bfs ctrl"));
+  // one allocation (nine took 20 us more of the first traversal)
+  dfree(h->bfs_visited);
+  h->bfs_visited = nullptr;
+  const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t words = up(4 * (size_t)std::max((h->n + 31) / 32, 1)), queue = up(8 * (size_t)std::max(h->n, 1));
+  char* p = nullptr;
+  SPMX_TRY(dalloc((void**)&p, 4 * words + 2 * queue + 512 + up(sizeof(BfsCtrl)), "bfs bitmaps and queues"));
+  h->bfs_visited = (unsigned*)p;
+  h->bfs_front = (unsigned*)(p + words);
+  h->bfs_fb1 = (unsigned*)(p + 2 * words);
+  h->bfs_fb2 = (unsigned*)(p + 3 * words);
+  p += 4 * words;
+  h->bfs_q[0] = (int*)p;
+  h->bfs_q[1] = (int*)(p + queue);
+  p += 2 * queue;
+  h->bfs_cnt = (int*)p;
+  h->bfs_edges = (decltype(h->bfs_edges))(p + 256);
+  h->bfs_ctrl = p + 512;
   SPMX_CUDA(cudaMemsetAsync(h->bfs_ctrl, 0, sizeof(BfsCtrl), h->stream));
   SPMX_CUDA(cudaStreamSynchronize(h->stream));
   h->bfs_n = h->n;

@@ -293,8 +293,7 @@ extern "C" int spmx_destroy(spmx_handle_t h) {
   spmx_tiled_postprocess(h);
   spmx_round_postprocess(h);
   spmx_hybrid_postprocess(h);
-  dfree(h->bfs_visited); dfree(h->bfs_front); dfree(h->bfs_q[0]); dfree(h->bfs_q[1]);
-  dfree(h->bfs_cnt); dfree(h->bfs_edges); dfree(h->bfs_fb1); dfree(h->bfs_fb2); dfree(h->bfs_ctrl);
+  dfree(h->bfs_visited);  // and all of the traversal's scratch behind it
   dfree(h->ms_visit); dfree(h->ms_planes);
   dfree(h->ms_q0); dfree(h->ms_q1); dfree(h->ms_ctrl);
   dfree(h->ms_hchunk); dfree(h->ms_hvert); dfree(h->ms_hacc); dfree(h->ms_hcounters);

@@ -154,7 +154,7 @@ struct spmx_handle_s {
   const int* ms_hub_rowptr = nullptr;
   int ms_hub_nnz = -1;
   double bfs_alpha = 14.0, bfs_beta = 24.0, msbfs_alpha = 12.0;
-  unsigned* bfs_visited = nullptr;
+  unsigned* bfs_visited = nullptr;         // the allocation that holds this and the rest (ensure_bfs)
   unsigned* bfs_front = nullptr;
   unsigned* bfs_fb2 = nullptr;
   int* bfs_q[2] = {nullptr, nullptr};
