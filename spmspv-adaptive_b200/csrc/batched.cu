@@ -56,10 +56,13 @@ constexpr int kBatchMaxVec = 1024;  // nvec limit (shared row accumulators)
 // a chunk costs an atomic on one address, about 2 ns).
 constexpr int kBatchChunk = 2048, kBatchChunkMin = 128, kBatchChunks = 32768;
 constexpr int kBatchRowCost = 32;
-// Rows above this are taken by whole CTAs before the row walk starts: one warp
-// alone on a hub row (10,000 nonzeros, 300 dependent steps) was the tail of the
-// walk, 0.55 ms of 1.2 ms on a 1M-vertex Chung-Lu graph.
-constexpr int kBatchHubRow = 512;
+// Rows above kBatchHubRow nonzeros and above 1 / kBatchHubShare of the matrix's are
+// taken by whole CTAs before the row walk starts: one warp alone on a hub row
+// (10,000 nonzeros, 300 dependent steps) was the tail of the walk, 0.55 ms of 1.2 ms
+// on a 1M-vertex Chung-Lu graph.  A CTA is slower per nonzero, so not more rows
+// than the tail asks for: 4M vertices, 134M nonzeros, forward 2.10 ms with 512, 2.03
+// with 2,048; 65,536 vertices, 2M nonzeros, 179 us with 512, 150 with 384.
+constexpr int kBatchHubRow = 384, kBatchHubShare = 65536;
 
 // sort keys (column) and payloads (entry, vector) of every batch entry
 __global__ void batch_keys_kernel(int n, int nvec, int total, const int* __restrict__ xptr,
@@ -112,10 +115,11 @@ __global__ void batch_chunks_kernel(int m, const int* __restrict__ rowptr, int n
   chunk_row[k] = lo;
 }
 
-// the rows above kBatchHubRow, in any order; *count has their number
-__global__ void batch_hubs_kernel(int m, const int* __restrict__ rowptr, int* __restrict__ hub_row, int* count) {
+// the rows above hub_min, in any order; *count has their number
+__global__ void batch_hubs_kernel(int m, const int* __restrict__ rowptr, int hub_min, int* __restrict__ hub_row,
+                                  int* count) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-    if (__ldg(rowptr + i + 1) - __ldg(rowptr + i) > kBatchHubRow) hub_row[atomicAdd(count, 1)] = i;
+    if (__ldg(rowptr + i + 1) - __ldg(rowptr + i) > hub_min) hub_row[atomicAdd(count, 1)] = i;
 }
 
 // the CTA's next hub row (-1: none left); whole CTA
@@ -221,22 +225,28 @@ __device__ __forceinline__ void batch_head_pairs(BatchRowHead& h, const int* __r
   }
 }
 
-constexpr int kBatchU = 4;  // pair records in flight per lane
+// Pair records in flight per lane; one where columns have fewer than one pair on
+// average (batch_sparse), where more only cost registers: 4M vertices, 2.7M entries,
+// forward 2.42 ms with four, 2.16 with two, 2.09 with one, the fused dvals walk 2.88,
+// 2.91 and 2.81 (at 5 CTAs per SM; at 4 3.36).
+constexpr int kBatchU = 4, kBatchSparseU = 1;
 
 // acc[v] += a * x over the pairs [p0, p1)
+template <int U>
 __device__ __forceinline__ void batch_add_pairs(float* acc, const int2* __restrict__ rec, int p0, int p1, float a) {
-  for (int p = p0; p < p1; p += kBatchU) {
-    int2 e[kBatchU];
+  for (int p = p0; p < p1; p += U) {
+    int2 e[U];
 #pragma unroll
-    for (int u = 0; u < kBatchU; ++u)
+    for (int u = 0; u < U; ++u)
       if (p + u < p1) e[u] = __ldg(rec + p + u);
 #pragma unroll
-    for (int u = 0; u < kBatchU; ++u)
+    for (int u = 0; u < U; ++u)
       if (p + u < p1) atomicAdd(acc + e[u].x, a * __int_as_float(e[u].y));
   }
 }
 
 // acc += the nonzeros k, k + step, ... < a1 times their pairs, two per lane at a time
+template <int U>
 __device__ __forceinline__ void batch_add_row(float* acc, const int* __restrict__ col,
                                               const float* __restrict__ val,
                                               const int* __restrict__ invptr, const int2* __restrict__ rec, int n,
@@ -249,17 +259,18 @@ __device__ __forceinline__ void batch_add_row(float* acc, const int* __restrict_
     if (!ok0 || (two && !ok1)) flag_error(err, kDevErrOob);
     const int q00 = ok0 ? __ldg(invptr + j0) : 0, q01 = ok0 ? __ldg(invptr + j0 + 1) : 0;
     const int q10 = ok1 ? __ldg(invptr + j1) : 0, q11 = ok1 ? __ldg(invptr + j1 + 1) : 0;
-    batch_add_pairs(acc, rec, q00, q01, v0);
-    batch_add_pairs(acc, rec, q10, q11, v1);
+    batch_add_pairs<U>(acc, rec, q00, q01, v0);
+    batch_add_pairs<U>(acc, rec, q10, q11, v1);
   }
 }
 
 // Y[i][:] = alpha * sum_k A[i][k] * X[col_k][:], one warp per row
+template <int U>
 __global__ void __launch_bounds__(kBatchWarps * 32)
 batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const int* __restrict__ col,
                      const float* __restrict__ val, const int* __restrict__ invptr,
                      const int2* __restrict__ rec, float alpha, float* __restrict__ Y, int vec4,
-                     const int* __restrict__ chunk_row, int nch, const int* __restrict__ hub_row,
+                     const int* __restrict__ chunk_row, int nch, int hub_min, const int* __restrict__ hub_row,
                      const int* __restrict__ nhub, int* ctr, int* err) {
   extern __shared__ __align__(16) float s_acc[];  // kBatchWarps rows of nvec
   __shared__ int s_hub;
@@ -270,7 +281,7 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
   // hub rows: the warps share the row's nonzeros, then its accumulators are added up
   for (int i; (i = batch_next_hub(ctr + 1, hub_row, nhub, &s_hub)) >= 0;) {
     const int a1 = __ldg(rowptr + i + 1);
-    batch_add_row(acc, col, val, invptr, rec, n, __ldg(rowptr + i) + warp * 32 + lane, a1, kBatchWarps * 32, err);
+    batch_add_row<U>(acc, col, val, invptr, rec, n, __ldg(rowptr + i) + warp * 32 + lane, a1, kBatchWarps * 32, err);
     __syncthreads();
     for (int v = threadIdx.x; v < nvec; v += kBatchWarps * 32) {
       float t = 0.f;
@@ -301,11 +312,11 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
     const int i3 = it.next(ctr, nch, chunk_row, m, lane);
     int c0, c1;
     batch_row_bounds(rowptr, m, i3, c0, c1);
-    const bool hub = cur.a1 - cur.a0 > kBatchHubRow;  // done above (warp-uniform)
+    const bool hub = cur.a1 - cur.a0 > hub_min;  // done above (warp-uniform)
     if (hub) cur.p1 = cur.p0, cur.a1 = cur.a0;
-    batch_add_pairs(acc, rec, cur.p0, cur.p1, cur.a);
+    batch_add_pairs<U>(acc, rec, cur.p0, cur.p1, cur.a);
     // the row's nonzeros past the first 32
-    batch_add_row(acc, col, val, invptr, rec, n, cur.a0 + 32 + lane, cur.a1, 32, err);
+    batch_add_row<U>(acc, col, val, invptr, rec, n, cur.a0 + 32 + lane, cur.a1, 32, err);
     __syncwarp();
     float* yr = Y + (size_t)i * nvec;
     if (hub) {
@@ -343,12 +354,12 @@ batch_forward_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, con
 // held) while this row is walked.  Four records in flight per lane at 64
 // registers and 4 CTAs per SM: 1.19 ms on the 1M-vertex Chung-Lu graph with 256
 // vectors; two at 4 CTAs 1.22, two at 5 CTAs (48 registers, spills) 1.37.
-template <bool FUSED>
-__global__ void __launch_bounds__(kBatchWarps * 32, 4)
+template <bool FUSED, int U>
+__global__ void __launch_bounds__(kBatchWarps * 32, U == kBatchU ? 4 : 5)
 batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const int* __restrict__ col,
                    const int* __restrict__ invptr, const int4* __restrict__ rec, float alpha,
                    const float* __restrict__ dY, float* __restrict__ dvals, const float* __restrict__ val,
-                   float* __restrict__ dxval, int vec4, const int* __restrict__ chunk_row, int nch,
+                   float* __restrict__ dxval, int vec4, const int* __restrict__ chunk_row, int nch, int hub_min,
                    const int* __restrict__ hub_row, const int* __restrict__ nhub, int* ctr, int* err) {
   extern __shared__ __align__(16) float s_dy[];
   __shared__ int s_hub;
@@ -358,13 +369,13 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     if ((unsigned)j < (unsigned)n) {
       const int q1 = __ldg(invptr + j + 1);
       const float a = FUSED ? alpha * va : 0.f;
-      for (int p = __ldg(invptr + j); p < q1; p += kBatchU) {
-        int4 r[kBatchU];
+      for (int p = __ldg(invptr + j); p < q1; p += U) {
+        int4 r[U];
 #pragma unroll
-        for (int u = 0; u < kBatchU; ++u)
+        for (int u = 0; u < U; ++u)
           if (p + u < q1) r[u] = __ldg(rec + p + u);
 #pragma unroll
-        for (int u = 0; u < kBatchU; ++u) {
+        for (int u = 0; u < U; ++u) {
           if (p + u >= q1) continue;
           const float gv = g[r[u].x];
           s += __int_as_float(r[u].y) * gv;
@@ -416,7 +427,7 @@ batch_dvals_kernel(int m, int n, int nvec, const int* __restrict__ rowptr, const
     const int i2 = it.next(ctr, nch, chunk_row, m, lane);
     int c0, c1;
     batch_row_bounds(rowptr, m, i2, c0, c1);
-    if (cur.a0 < cur.a1 && cur.a1 - cur.a0 <= kBatchHubRow) {  // warp-uniform
+    if (cur.a0 < cur.a1 && cur.a1 - cur.a0 <= hub_min) {  // warp-uniform
       float* const g = g0 + (pre ? buf * nvec : 0);
       if (pre) {
         cp_async_wait<1>();  // every group but the next row's: this row's dY has landed
@@ -571,6 +582,8 @@ static int batch_invert(spmx_handle_t h, int nvec, int total, const int* xptr, c
   return SPMX_SUCCESS;
 }
 
+static int batch_hub_min(spmx_handle_t h) { return std::max(kBatchHubRow, h->nnz / kBatchHubShare); }
+
 // the row chunks of the matrix (built once per CSR input; the counters they
 // are taken from are zeroed before every launch)
 static int ensure_batch_chunks(spmx_handle_t h) {
@@ -589,7 +602,8 @@ static int ensure_batch_chunks(spmx_handle_t h) {
     SPMX_TRY(dalloc((void**)&h->batch_hub, 4 * ((size_t)h->nnz / (kBatchHubRow + 1) + 1), "batch hub rows"));
   SPMX_CUDA(cudaMemsetAsync(h->batch_ctr + 4, 0, sizeof(int), h->stream));
   note_launch();
-  batch_hubs_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->m, h->rowptr, h->batch_hub, h->batch_ctr + 4);
+  batch_hubs_kernel<<<h->num_sms * 8, 256, 0, h->stream>>>(h->m, h->rowptr, batch_hub_min(h), h->batch_hub,
+                                                                   h->batch_ctr + 4);
   note_launch();
   batch_chunks_kernel<<<(unsigned)((nch + 1 + 255) / 256), 256, 0, h->stream>>>(h->m, h->rowptr, (int)nch, chunk,
                                                                                 h->batch_chunk);
@@ -619,6 +633,9 @@ static int batch_rows_grid(spmx_handle_t h, const void* kernel, size_t smem) {
   return (int)std::max(1LL, std::min<long long>(want, (long long)per * h->num_sms));
 }
 
+// fewer than one pair per column: most columns have none or one
+static bool batch_sparse(spmx_handle_t h, int x_total) { return x_total < h->n; }
+
 extern "C" int spmx_spmspv_batched(spmx_handle_t h, int nvec, int x_total, const int* d_xptr,
                                    const int* d_xkey, const float* d_xval, float alpha, float* d_Y) {
   SPMX_CHECK_HANDLE(h);
@@ -633,13 +650,14 @@ extern "C" int spmx_spmspv_batched(spmx_handle_t h, int nvec, int x_total, const
   SPMX_TRY(ensure_batch_chunks(h));
   SPMX_CUDA(cudaMemsetAsync(h->batch_ctr, 0, 2 * sizeof(int), h->stream));
   const size_t smem = 4 * (size_t)kBatchWarps * nvec;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(batch_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto kernel = batch_sparse(h, x_total) ? batch_forward_kernel<kBatchSparseU> : batch_forward_kernel<kBatchU>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   note_launch();
-  batch_forward_kernel<<<batch_rows_grid(h, (const void*)batch_forward_kernel, smem), kBatchWarps * 32, smem,
-                         h->stream>>>(h->m, h->n, nvec, h->rowptr, h->col, h->val, h->batch_invptr, rec,
+  kernel<<<batch_rows_grid(h, (const void*)kernel, smem), kBatchWarps * 32, smem, h->stream>>>(
+                                      h->m, h->n, nvec, h->rowptr, h->col, h->val, h->batch_invptr, rec,
                                       alpha, d_Y, (nvec % 4 == 0 && ((uintptr_t)d_Y & 15u) == 0) ? 1 : 0,
-                                      h->batch_chunk, h->batch_nch, h->batch_hub, h->batch_ctr + 4, h->batch_ctr, h->d_err);
+                                      h->batch_chunk, h->batch_nch, batch_hub_min(h), h->batch_hub, h->batch_ctr + 4,
+                                      h->batch_ctr, h->d_err);
   return launch_ok("batched spmspv");
 }
 
@@ -664,12 +682,15 @@ extern "C" int spmx_spmspv_batched_backward(spmx_handle_t h, int nvec, int x_tot
     const bool vec4 = nvec % 4 == 0 && ((uintptr_t)d_dY & 15u) == 0;
     // with 16-byte rows of at most 256 entries each warp double-buffers its dY row
     const size_t smem = 4 * (size_t)kBatchWarps * nvec * (vec4 && nvec <= 256 ? 2 : 1);
-    const auto kernel = fused ? batch_dvals_kernel<true> : batch_dvals_kernel<false>;
+    const auto kernel =
+        batch_sparse(h, x_total)
+            ? (fused ? batch_dvals_kernel<true, kBatchSparseU> : batch_dvals_kernel<false, kBatchSparseU>)
+            : (fused ? batch_dvals_kernel<true, kBatchU> : batch_dvals_kernel<false, kBatchU>);
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     note_launch();
     kernel<<<batch_rows_grid(h, (const void*)kernel, smem), kBatchWarps * 32, smem, st>>>(h->m, h->n, nvec, h->rowptr, h->col, h->batch_invptr, rec4, alpha,
                                d_dY, d_dvals, h->val, fused ? d_dxval : nullptr, vec4 ? 1 : 0, h->batch_chunk,
-                               h->batch_nch, h->batch_hub, h->batch_ctr + 4, h->batch_ctr + 2, h->d_err);
+                               h->batch_nch, batch_hub_min(h), h->batch_hub, h->batch_ctr + 4, h->batch_ctr + 2, h->d_err);
   }
   if (d_dxval && x_total > 0 && !fused) {
     if (!h->has_csc || !h->csc_val)

@@ -1,6 +1,7 @@
-"""Batched SpMSpV rows around the hub limit (512 nonzeros), which whole CTAs
-take: 511, 512, 513 and more rows above it than there are CTAs, with vector
-counts that are and are not multiples of 4 and above 256; against FP64."""
+"""Batched SpMSpV rows around the hub limit (384 nonzeros), which whole CTAs
+take: 384, 385 and more rows above it than there are CTAs, with vector counts
+that are and are not multiples of 4 and above 256, fewer and more batch entries
+than columns; against FP64."""
 import numpy as np
 import pytest
 
@@ -19,7 +20,7 @@ def test_hub_rows(torch_cuda, nvec, hubs, options):
     torch = torch_cuda
     rng = np.random.default_rng(nvec + hubs)
     lens = rng.integers(0, 12, 1500)
-    lens[100:103] = (511, 512, 40)
+    lens[100:105] = (511, 512, 40, 384, 385)
     lens[200:200 + hubs] = 513 + rng.integers(0, 60, hubs)
     A = rand_csr(1500, 1600, lens=lens, seed=6)
     h = make_handle(A, torch, hola=False)
