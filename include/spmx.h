@@ -68,9 +68,9 @@ extern "C" {
 #define SPMX_CSC_NAIVE     0  /* group of threads per x nonzero            */
 #define SPMX_CSC_LB_MERGE  1  /* merge-path partition over (x entries, nnz) */
 #define SPMX_CSC_LB_TWOLAYER 2/* fixed nnz per CTA, block-start table      */
-#define SPMX_CSC_BUCKET    3  /* row-block buckets, no global atomics      */
+#define SPMX_CSC_BUCKET    3  /* dense rows; above 8M rows row-block buckets */
 #define SPMX_WB_ATOMIC     0  /* dense y via atomics (+ optional compaction)*/
-#define SPMX_WB_SORT       1  /* (row,val) pairs -> sort -> reduce_by_key   */
+#define SPMX_WB_SORT       1  /* sorted (row,val) of every row reached      */
 
 /* ---- the eight adaptive kernels, in the reference's three-stage tree order
  *      (TEST/new_test_app.cu:406-456): solution x workload x write-back      */
@@ -298,7 +298,9 @@ int spmx_spmspv(spmx_handle_t h, float alpha, float* d_y);
  *    nonzeros of y (entries != 0) are also compacted into them, in row order.
  *  - sort:   d_y_key/d_y_val receive the rows touched by x's columns, sorted,
  *    with their sums (zeros kept — reduce_by_key semantics); d_y may be NULL,
- *    otherwise it is also written densely.
+ *    otherwise it is also written densely.  Sums are accumulated in double up
+ *    to 8M rows.  Refused where x's repeated keys select more nonzeros than
+ *    the matrix has (the outputs are then undefined).
  *  - bucket: as sort for the sparse output, plus dense d_y if non-NULL.
  * ynnz (host, may be NULL) receives the output count (synchronises). */
 int spmx_spmspv_csc(spmx_handle_t h, int variant, int writeback, float alpha,
@@ -397,8 +399,8 @@ int spmx_run_adaptive(spmx_handle_t h, float alpha, float* d_y, int* kernel_used
 /* Per-matrix autotuner (no reference counterpart beyond the reference's
  * Hola-vs-CSR5 timing, TEST/generate_model_data.cu:487-516): times the
  * load-balanced SpMV back-ends (Hola 4/8/16 nonzeros per thread, CSR5, tiled
- * geometries), the naive kernels' lanes per row / column, merge-path vs
- * fixed-nonzero CSC blocks and the bucket count, and keeps the fastest.
+ * geometries), the naive kernels' lanes per row / column and the bucket count,
+ * and keeps the fastest.
  * cache_path (may be NULL): a text file of tuned parameters keyed by a matrix
  * fingerprint; a hit applies them without timing.  spmv_type_out (may be NULL)
  * receives the chosen SpMV back-end. */
