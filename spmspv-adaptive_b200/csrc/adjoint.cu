@@ -339,7 +339,8 @@ int launch_spmv_backward(int m, int n, int nnz, const int* rowptr, const int* co
                          const float* val, const float* x, const float* dy,
                          const HolaTables& t, float* dx, float* dvals, int* err,
                          DevGate gate, cudaStream_t st) {
-  if (nnz <= 0 || t.nchunks == 0) return 0;
+  // the kernels of short rows have a form for dx, for dvals and for both
+  if (nnz <= 0 || t.nchunks == 0 || (!dx && !dvals)) return 0;
   if (t.K != 2048) return -1;  // the backward pass uses 256 x 8 chunks
   const int nlong = t.nchunks - t.n_short;
   note_launch((t.n_short > 0) + (nlong > 0));

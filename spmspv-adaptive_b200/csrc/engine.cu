@@ -876,6 +876,7 @@ extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* 
                                   float* dvals) {
   SPMX_CHECK_HANDLE(h);
   SPMX_TRY(backward_check(h, x, dy, dvals));
+  if (!dx && !dvals) return SPMX_SUCCESS;
   SPMX_TRY(backward_tables(h));
   if (dx && !backward_by_csc(h)) SPMX_CUDA(cudaMemsetAsync(dx, 0, 4 * (size_t)h->n, h->stream));
   return backward_dense(h, x, dy, dx, dvals, DevGate{});
@@ -890,6 +891,7 @@ extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const fl
   SPMX_TRY(backward_check(h, x, dy, dvals));
   limit = std::min(limit, h->m + 1);
   if (limit <= 0 || h->m == 0) return spmx_spmv_backward(h, x, dy, dx, dvals);
+  if (!dx && !dvals) return SPMX_SUCCESS;
   SPMX_TRY(backward_tables(h));
   if (!scratch) return set_error(SPMX_ERR_INVALID_VALUE, "scratch is NULL");
   cudaStream_t st = h->stream;
