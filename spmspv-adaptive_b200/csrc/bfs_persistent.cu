@@ -497,7 +497,11 @@ msbfs_persistent_kernel(MsBfsState t, long long total_edges, double alpha_ms, co
       for (long long c = gwarp; c < hub.nchunks; c += nwarps) {
         int4 nch = ch;
         if (c + nwarps < hub.nchunks) nch = hub.chunk[c + nwarps];
-        const unsigned long long got = have | *(volatile unsigned long long*)(hub.acc + ch.w);
+        // other warps add to the accumulator meanwhile: one lane's reading of it
+        // decides for the warp, which goes through full-mask reductions below
+        unsigned long long got = 0ull;
+        if (lane == 0) got = have | *(volatile unsigned long long*)(hub.acc + ch.w);
+        got = __shfl_sync(0xffffffffu, got, 0);
         if (got != FULL) {
           const unsigned long long acc = ms_pull<kMsHubU>(fc, col, n, ch.y, ch.z, have, FULL, err);
           if (lane == 0 && (acc & ~got)) atomicOr(hub.acc + ch.w, acc);
