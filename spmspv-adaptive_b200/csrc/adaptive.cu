@@ -378,32 +378,44 @@ static int ensure_msbfs(spmx_handle_t h) {
 // vertices of degree above this are pulled in chunks of this many edges
 constexpr int kHubDegree = 256;
 
-// hub chunk list of the multi-source pull, built once per matrix
-static int ensure_hubs(spmx_handle_t h) {
-  if (h->ms_hub_rowptr == h->rowptr && h->ms_hub_nnz == h->nnz && h->ms_hcounters) return SPMX_SUCCESS;
+// Hub chunk list of the multi-source BFS, built once per matrix input in arrays
+// sized by the number of nonzeros, which a handle never changes.  Under capture
+// the counts cannot be read back: the list is built by the graph itself, behind
+// a clear, and the traversal walks the whole of it (a cleared entry is a chunk
+// without edges, a hub that gathers nothing).
+static int ensure_hubs(spmx_handle_t h, int* nhubs, long long* nchunks) {
   cudaStream_t st = h->stream;
-  SPMX_CUDA(cudaStreamSynchronize(st));
-  dfree(h->ms_hchunk); dfree(h->ms_hvert); dfree(h->ms_hacc); dfree(h->ms_hcounters);
-  h->ms_hchunk = nullptr; h->ms_hvert = nullptr; h->ms_hacc = nullptr;
-  h->ms_hcounters = nullptr;
-  const long long nnz = std::max(h->nnz, 0);
-  const int max_hubs = (int)(nnz / (kHubDegree + 1) + 1);
-  const long long max_chunks = nnz / kHubDegree + max_hubs + 1;
-  SPMX_TRY(dalloc((void**)&h->ms_hchunk, sizeof(int4) * (size_t)max_chunks, "msbfs hub chunks"));
-  SPMX_TRY(dalloc((void**)&h->ms_hvert, 4 * (size_t)max_hubs, "msbfs hub vertices"));
-  SPMX_TRY(dalloc((void**)&h->ms_hacc, 8 * (size_t)max_hubs, "msbfs hub accumulators"));
-  SPMX_TRY(dalloc((void**)&h->ms_hcounters, 8, "msbfs hub totals"));
-  SPMX_CUDA(cudaMemsetAsync(h->ms_hcounters, 0, 8, st));
-  launch_hub_chunks(h->n, h->rowptr, kHubDegree, h->ms_hchunk, h->ms_hvert, h->ms_hcounters, max_hubs,
-                    (int)max_chunks, st);
-  int cnt[2] = {0, 0};
-  SPMX_CUDA(cudaMemcpyAsync(cnt, h->ms_hcounters, 8, cudaMemcpyDeviceToHost, st));
-  SPMX_CUDA(cudaStreamSynchronize(st));
-  if (cnt[0] > max_hubs || cnt[1] > max_chunks) return set_error(SPMX_ERR_OOB, "hub chunk capacity");
-  h->ms_nhubs = cnt[0];
-  h->ms_nhchunks = cnt[1];
-  h->ms_hub_rowptr = h->rowptr;
-  h->ms_hub_nnz = h->nnz;
+  if (!h->ms_hubs_ready) {
+    const long long nnz = std::max(h->nnz, 0);
+    const int max_hubs = (int)(nnz / (kHubDegree + 1) + 1);
+    const long long max_chunks = nnz / kHubDegree + max_hubs + 1;
+    if (!h->ms_hchunk) SPMX_TRY(dalloc((void**)&h->ms_hchunk, sizeof(int4) * (size_t)max_chunks, "msbfs hub chunks"));
+    if (!h->ms_hvert) SPMX_TRY(dalloc((void**)&h->ms_hvert, 4 * (size_t)max_hubs, "msbfs hub vertices"));
+    if (!h->ms_hacc) SPMX_TRY(dalloc((void**)&h->ms_hacc, 8 * (size_t)max_hubs, "msbfs hub accumulators"));
+    if (!h->ms_hcounters) SPMX_TRY(dalloc((void**)&h->ms_hcounters, 8, "msbfs hub totals"));
+    const bool capturing = stream_capturing(st);
+    if (capturing) {
+      SPMX_CUDA(cudaMemsetAsync(h->ms_hchunk, 0, sizeof(int4) * (size_t)max_chunks, st));
+      SPMX_CUDA(cudaMemsetAsync(h->ms_hvert, 0, 4 * (size_t)max_hubs, st));
+    }
+    SPMX_CUDA(cudaMemsetAsync(h->ms_hcounters, 0, 8, st));
+    launch_hub_chunks(h->n, h->rowptr, kHubDegree, h->ms_hchunk, h->ms_hvert, h->ms_hcounters, max_hubs,
+                      (int)max_chunks, st);
+    if (capturing) {
+      *nhubs = max_hubs;
+      *nchunks = max_chunks;
+      return SPMX_SUCCESS;
+    }
+    int cnt[2] = {0, 0};
+    SPMX_CUDA(cudaMemcpyAsync(cnt, h->ms_hcounters, 8, cudaMemcpyDeviceToHost, st));
+    SPMX_CUDA(cudaStreamSynchronize(st));
+    if (cnt[0] > max_hubs || cnt[1] > max_chunks) return set_error(SPMX_ERR_OOB, "hub chunk capacity");
+    h->ms_nhubs = cnt[0];
+    h->ms_nhchunks = cnt[1];
+    h->ms_hubs_ready = true;
+  }
+  *nhubs = h->ms_nhubs;
+  *nchunks = h->ms_nhchunks;
   return SPMX_SUCCESS;
 }
 
@@ -417,12 +429,14 @@ extern "C" int spmx_bfs_batched(spmx_handle_t h, const int* srcs, int nsrc, int*
   for (int s = 0; s < nsrc; ++s)
     if (srcs[s] < 0 || srcs[s] >= h->n) return set_error(SPMX_ERR_INVALID_VALUE, "source out of range");
   SPMX_TRY(ensure_msbfs(h));
-  SPMX_TRY(ensure_hubs(h));
+  int nhubs = 0;
+  long long nchunks = 0;
+  SPMX_TRY(ensure_hubs(h, &nhubs, &nchunks));
   cudaStream_t st = h->stream;
   const size_t n = (size_t)h->n;
   SPMX_CUDA(cudaMemsetAsync(h->ms_visit, 0, 32 * n, st));
-  if (h->ms_nhubs > 0) SPMX_CUDA(cudaMemsetAsync(h->ms_hacc, 0, 8 * (size_t)h->ms_nhubs, st));
-  HubChunks hub{h->ms_hchunk, h->ms_nhchunks, h->ms_hvert, h->ms_hacc, h->ms_nhubs, kHubDegree};
+  if (nhubs > 0) SPMX_CUDA(cudaMemsetAsync(h->ms_hacc, 0, 8 * (size_t)nhubs, st));
+  HubChunks hub{h->ms_hchunk, nchunks, h->ms_hvert, h->ms_hacc, nhubs, kHubDegree};
   MsBfsArgs a{h->n, nsrc, layout, h->num_sms, (long long)h->nnz, h->msbfs_alpha, {}, h->rowptr, h->col, levels,
               h->ms_visit, h->ms_front0, h->ms_front1, h->ms_next, (ulonglong4*)h->ms_planes, h->ms_q0, h->ms_q1,
               (BfsCtrl*)h->ms_ctrl, hub, h->d_err};

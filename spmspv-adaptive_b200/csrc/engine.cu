@@ -362,6 +362,7 @@ extern "C" int spmx_input_csr(spmx_handle_t h, int nnz, const int* rowptr,
   h->mat_feat_ready = false;
   h->std_row_ready = false;
   h->batch_chunk_ready = false;
+  h->ms_hubs_ready = false;  // the same arrays may hold another pattern now
   return SPMX_SUCCESS;
 }
 

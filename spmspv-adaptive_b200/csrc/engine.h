@@ -144,15 +144,15 @@ struct spmx_handle_s {
   // walk's, [4] number of hub rows
   int* batch_ctr = nullptr;
   int* batch_hub = nullptr;  // rows above kBatchHubRow nonzeros
-  // hub chunks of the multi-source pull (built once per matrix)
+  // hub chunks of the multi-source BFS (built once per matrix input, in arrays
+  // sized by nnz)
   int4* ms_hchunk = nullptr;
   int* ms_hvert = nullptr;
   unsigned long long* ms_hacc = nullptr;
   int* ms_hcounters = nullptr;
   long long ms_nhchunks = 0;
   int ms_nhubs = 0;
-  const int* ms_hub_rowptr = nullptr;
-  int ms_hub_nnz = -1;
+  bool ms_hubs_ready = false;
   double bfs_alpha = 14.0, bfs_beta = 24.0, msbfs_alpha = 12.0;
   unsigned* bfs_visited = nullptr;         // the allocation that holds this and the rest (ensure_bfs)
   unsigned* bfs_front = nullptr;
@@ -199,6 +199,13 @@ cudaError_t kernel_smem_limit(const void* kernel, size_t bytes);
   do {                                                                         \
     if (!(h)) return set_error(SPMX_ERR_INVALID_VALUE, "NULL handle");         \
   } while (0)
+
+// whether what is enqueued now goes into a graph instead of running
+inline bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
 
 // status of the last kernel launch on this thread
 inline int launch_ok(const char* what) {

@@ -159,7 +159,7 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   h->mat_feat_ready = false;
   h->std_row_ready = false;
   h->batch_chunk_ready = false;
-  h->ms_hub_rowptr = nullptr;  // the arrays stay where they are: tables kept by address are not the new matrix's
+  h->ms_hubs_ready = false;
   // a CSC derived from the previous CSR by spmx_to_csc is stale now
   if (h->has_csc && h->csc_colptr == h->own_colptr) h->has_csc = false;
   return SPMX_SUCCESS;
