@@ -190,7 +190,10 @@ int spmx_sparse2dense_outer(spmx_handle_t h, int ynnz, const int* d_key,
  * worst case (bin_len = nnz) so later calls never allocate. */
 int spmx_alloc_pre_buffer(spmx_handle_t h);
 int spmx_dealloc_pre_buffer(spmx_handle_t h);
-/* holaPreprocess / holaPostprocess — H:1654-1672 (block-start table) */
+/* holaPreprocess / holaPostprocess — H:1654-1672 (block-start table).  After an
+ * input with another row pointer, or InputCOO, the next call fills the table
+ * again by itself (it synchronises then); a pattern written anew into the same
+ * arrays needs this call again, as the tables below do after any new pattern. */
 int spmx_hola_preprocess(spmx_handle_t h);
 int spmx_hola_postprocess(spmx_handle_t h);
 /* setSigma / CSR5Preprocess / CSR5Postprocess — H:1396-1651.  sigma = -1

@@ -49,7 +49,7 @@ spmv_backward_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
   // rows at one position leave the largest index, the non-empty one
   for (int r = lo + (int)threadIdx.x; r < hi; r += NT) {
     const int p = __ldg(rowptr + r) - s;
-    if (p < e - s) atomicMax(&s_mark[p], r);
+    if ((unsigned)p < (unsigned)(e - s)) atomicMax(&s_mark[p], r);
   }
   __syncthreads();
   int loc[VT];

@@ -355,6 +355,7 @@ extern "C" int spmx_input_csr(spmx_handle_t h, int nnz, const int* rowptr,
   if (nnz != h->nnz) return set_error(SPMX_ERR_INVALID_VALUE, "nnz differs from the handle's nnz");
   if (!rowptr || (!col && nnz > 0))
     return set_error(SPMX_ERR_INVALID_VALUE, "NULL CSR array");
+  if (rowptr != h->rowptr) h->hola_rowptr = nullptr;  // values alone keep the tables
   h->rowptr = rowptr;
   h->col = col;
   h->val = val;
@@ -718,6 +719,39 @@ extern "C" int spmx_dealloc_pre_buffer(spmx_handle_t h) {
   return SPMX_SUCCESS;
 }
 
+// The chunk tables of the handle's pattern, in arrays that only nnz and the
+// chunk's size decide.
+static int hola_fill(spmx_handle_t h, HolaTables* t) {
+  SPMX_CUDA(cudaMemsetAsync(t->arrive, 0, 4 * (size_t)std::max(t->nchunks, 1), h->stream));
+  // d_iacc: how many chunks have only short rows, how many have not
+  SPMX_CUDA(cudaMemsetAsync(h->d_iacc, 0, 2 * sizeof(int), h->stream));
+  launch_chunk_rows(h->m, h->nnz, h->rowptr, t->K, t->nchunks, t->chunk_row, t->list, h->d_iacc, h->stream);
+  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned + 2, h->d_iacc, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  SPMX_CUDA(cudaStreamSynchronize(h->stream));
+  t->n_short = h->h_pinned[2] >= t->nchunks / 4 ? h->h_pinned[2] : 0;
+  return SPMX_SUCCESS;
+}
+
+// The tables for a launch.  Those of a pattern that the handle no longer holds
+// (InputCSR with another row pointer, or InputCOO) are filled again first; under
+// capture, where the number of short chunks cannot be read back, the graph fills
+// the row of every chunk, and all of them go through the scan.
+static int hola_tables(spmx_handle_t h, HolaTables* t) {
+  if (h->hola_rowptr != h->rowptr) {
+    if (stream_capturing(h->stream)) {
+      *t = h->hola;
+      t->n_short = 0;
+      SPMX_CUDA(cudaMemsetAsync(t->arrive, 0, 4 * (size_t)std::max(t->nchunks, 1), h->stream));
+      launch_chunk_rows(h->m, h->nnz, h->rowptr, t->K, t->nchunks, t->chunk_row, nullptr, nullptr, h->stream);
+      return SPMX_SUCCESS;
+    }
+    SPMX_TRY(hola_fill(h, &h->hola));
+    h->hola_rowptr = h->rowptr;
+  }
+  *t = h->hola;
+  return SPMX_SUCCESS;
+}
+
 extern "C" int spmx_hola_preprocess(spmx_handle_t h) {
   SPMX_CHECK_HANDLE(h);
   if (!h->has_csr) return set_error(SPMX_FORMAT_ERR_HOLA_SPMV, "Hola needs the CSR input");
@@ -730,15 +764,10 @@ extern "C" int spmx_hola_preprocess(spmx_handle_t h) {
   SPMX_TRY(dalloc((void**)&t.list, sizeof(int4) * (size_t)std::max(t.nchunks, 1), "hola chunk list"));
   SPMX_TRY(dalloc((void**)&t.carry, 8 * (size_t)std::max(2 * t.nchunks, 1), "hola carry"));
   SPMX_TRY(dalloc((void**)&t.arrive, 4 * (size_t)std::max(t.nchunks, 1), "hola arrive"));
-  SPMX_CUDA(cudaMemsetAsync(t.arrive, 0, 4 * (size_t)std::max(t.nchunks, 1), h->stream));
-  // d_iacc: how many chunks have only short rows, how many have not
-  SPMX_CUDA(cudaMemsetAsync(h->d_iacc, 0, 2 * sizeof(int), h->stream));
-  launch_chunk_rows(h->m, h->nnz, h->rowptr, t.K, t.nchunks, t.chunk_row, t.list, h->d_iacc, h->stream);
-  SPMX_CUDA(cudaMemcpyAsync(h->h_pinned + 2, h->d_iacc, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  SPMX_CUDA(cudaStreamSynchronize(h->stream));
-  t.n_short = h->h_pinned[2] >= t.nchunks / 4 ? h->h_pinned[2] : 0;
+  SPMX_TRY(hola_fill(h, &t));
   h->hola = t;
   h->hola_ready = true;
+  h->hola_rowptr = h->rowptr;
   return launch_ok("holaPreprocess");
 }
 
@@ -788,7 +817,9 @@ static int hola_spmv_impl(spmx_handle_t h, float alpha, float* y, bool gated) {
   SpmvArgs a;
   SPMX_TRY(spmv_common(h, alpha, y, gated, &a));
   if (!h->hola_ready) return set_error(SPMX_ERR_NOT_READY, "call spmx_hola_preprocess first");
-  if (launch_spmv_hola(a, h->hola, h->stream)) return set_error(SPMX_ERR_INVALID_VALUE, "bad Hola tile or launch");
+  HolaTables t;
+  SPMX_TRY(hola_tables(h, &t));
+  if (launch_spmv_hola(a, t, h->stream)) return set_error(SPMX_ERR_INVALID_VALUE, "bad Hola tile or launch");
   return launch_ok("hola spmv");
 }
 
@@ -847,7 +878,8 @@ static int backward_check(spmx_handle_t h, const float* x, const float* dy, floa
 static bool backward_by_csc(spmx_handle_t h) { return h->has_csc && (h->csc_val || h->nnz == 0); }
 
 // the dense-dy adjoint; without a CSC the caller has cleared dx
-static int backward_dense(spmx_handle_t h, const float* x, const float* dy, float* dx, float* dvals, DevGate gate) {
+static int backward_dense(spmx_handle_t h, const HolaTables& t, const float* x, const float* dy, float* dx,
+                          float* dvals, DevGate gate) {
   if (backward_by_csc(h)) {
     // dx = A^T dy as a gather over the CSC and dvals over the CSR, one launch
     const int g1 = h->naive_row_group > 0 ? h->naive_row_group
@@ -857,20 +889,24 @@ static int backward_dense(spmx_handle_t h, const float* x, const float* dy, floa
                              g2, dx, h->nnz > 0 ? dvals : nullptr, h->d_err, gate, h->stream);
     return launch_ok("spmv backward");
   }
-  if (launch_spmv_backward(h->m, h->n, h->nnz, h->rowptr, h->col, h->val, x, dy, h->hola, dx,
-                           dvals, h->d_err, gate, h->stream))
+  if (launch_spmv_backward(h->m, h->n, h->nnz, h->rowptr, h->col, h->val, x, dy, t, dx, dvals, h->d_err, gate,
+                           h->stream))
     return set_error(SPMX_ERR_INVALID_VALUE, "backward chunk geometry");
   return launch_ok("spmv backward");
 }
 
 // the Hola chunk table of the CSR-only adjoint, built on demand
-static int backward_tables(spmx_handle_t h) {
-  if (backward_by_csc(h) || (h->hola_ready && h->hola.K == 2048)) return SPMX_SUCCESS;
-  const int vt = h->hola_vt;
-  h->hola_vt = 8;
-  const int rc = spmx_hola_preprocess(h);
-  h->hola_vt = vt;
-  return rc;
+static int backward_tables(spmx_handle_t h, HolaTables* t) {
+  *t = HolaTables{};
+  if (backward_by_csc(h)) return SPMX_SUCCESS;
+  if (!h->hola_ready || h->hola.K != 2048) {
+    const int vt = h->hola_vt;
+    h->hola_vt = 8;
+    const int rc = spmx_hola_preprocess(h);
+    h->hola_vt = vt;
+    if (rc) return rc;
+  }
+  return hola_tables(h, t);
 }
 
 extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* dy, float* dx,
@@ -878,9 +914,10 @@ extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* 
   SPMX_CHECK_HANDLE(h);
   SPMX_TRY(backward_check(h, x, dy, dvals));
   if (!dx && !dvals) return SPMX_SUCCESS;
-  SPMX_TRY(backward_tables(h));
+  HolaTables t;
+  SPMX_TRY(backward_tables(h, &t));
   if (dx && !backward_by_csc(h)) SPMX_CUDA(cudaMemsetAsync(dx, 0, 4 * (size_t)h->n, h->stream));
-  return backward_dense(h, x, dy, dx, dvals, DevGate{});
+  return backward_dense(h, t, x, dy, dx, dvals, DevGate{});
 }
 
 // Both adjoints are launched behind the count of dy's nonzeros on the device, so
@@ -893,7 +930,8 @@ extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const fl
   limit = std::min(limit, h->m + 1);
   if (limit <= 0 || h->m == 0) return spmx_spmv_backward(h, x, dy, dx, dvals);
   if (!dx && !dvals) return SPMX_SUCCESS;
-  SPMX_TRY(backward_tables(h));
+  HolaTables t;
+  SPMX_TRY(backward_tables(h, &t));
   if (!scratch) return set_error(SPMX_ERR_INVALID_VALUE, "scratch is NULL");
   cudaStream_t st = h->stream;
   int* key = (int*)scratch;
@@ -904,7 +942,7 @@ extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const fl
     return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
   if (h->nnz == 0) dvals = nullptr;
   launch_backward_clear(h->n, h->nnz, dx, dvals, !backward_by_csc(h), h->num_sms, sparse, st);
-  SPMX_TRY(backward_dense(h, x, dy, dx, dvals, dense));
+  SPMX_TRY(backward_dense(h, t, x, dy, dx, dvals, dense));
   const int g = pow2_group((double)h->nnz / h->m);
   launch_spmv_backward_gated(h->m, h->n, h->rowptr, h->col, h->val, x, key, val, g, dx, dvals,
                              h->num_sms, h->d_err, sparse, st);

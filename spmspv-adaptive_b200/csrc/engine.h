@@ -84,6 +84,7 @@ struct spmx_handle_s {
   // Hola tables
   spmx::HolaTables hola{};
   bool hola_ready = false;
+  const int* hola_rowptr = nullptr;  // the row pointer they were filled from; null: a pattern that is gone
 
   // tuned parameters
   int naive_row_group = 0;    // 0 = derive from mean row length

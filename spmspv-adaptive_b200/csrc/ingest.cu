@@ -160,6 +160,7 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   h->std_row_ready = false;
   h->batch_chunk_ready = false;
   h->ms_hubs_ready = false;
+  h->hola_rowptr = nullptr;  // the arrays stay where they are, with another pattern in them
   // a CSC derived from the previous CSR by spmx_to_csc is stale now
   if (h->has_csc && h->csc_colptr == h->own_colptr) h->has_csc = false;
   return SPMX_SUCCESS;

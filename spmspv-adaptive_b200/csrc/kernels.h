@@ -38,6 +38,7 @@ constexpr int kShortRow = 32;
 // ---- spmv.cu
 int launch_spmv_naive(const SpmvArgs& a, int group, cudaStream_t st);
 int launch_spmv_hola(const SpmvArgs& a, const HolaTables& t, cudaStream_t st);
+// the first row of every chunk; with a list also which chunks have only short rows
 int launch_chunk_rows(int m, int nnz, const int* rowptr, int K, int nchunks, int* chunk_row,
                       int4* list, int* counts, cudaStream_t st);
 int hola_chunk_nnz(int vt);

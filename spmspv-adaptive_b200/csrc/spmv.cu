@@ -223,7 +223,8 @@ spmv_short_kernel(int n, int nnz, const int* __restrict__ rowptr, const int* __r
         a = __ldg(rowptr + r);
         b = __ldg(rowptr + r + 1);
       }
-      const int p1 = (WHOLE ? b : min(b, e)) - s;
+      // (a graph that outlives its pattern may find rows longer than the buffer)
+      const int p1 = WHOLE ? min(b - s, K + kShortRow) : min(b, e) - s;
       double sum = 0.0;
       for (int p = max(a, s) - s; p < p1; ++p) sum += s_p[p];
       if (r < lo) {
@@ -305,7 +306,7 @@ spmv_chunk_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
   __syncthreads();
   for (int r = lo + (int)threadIdx.x; r < hi; r += NT) {
     const int p = __ldg(rowptr + r) - s;
-    if (p < e - s) atomicOr(&s_flag[p >> 5], 1u << (p & 31));
+    if ((unsigned)p < (unsigned)(e - s)) atomicOr(&s_flag[p >> 5], 1u << (p & 31));
   }
   __syncthreads();
   // segmented scan: every row is summed from its own products only (no
@@ -336,7 +337,7 @@ spmv_chunk_kernel(int m, int n, int nnz, const int* __restrict__ rowptr,
     if (b == a) {
       y[r] = 0.f;
     } else if (b <= e) {
-      y[r] = (float)(alpha * sP[b - 1 - s]);
+      y[r] = (float)(alpha * sP[max(b - 1 - s, 0)]);
     } else {
       split_row_contribute<K>(r, c, 1, sP[e - 1 - s], rowptr, carry, arrive, alpha, y);
     }
@@ -391,7 +392,7 @@ int launch_chunk_rows(int m, int nnz, const int* rowptr, int K, int nchunks, int
   note_launch();
   chunk_rows_kernel<<<(threads + 255) / 256, 256, 0, st>>>(m, rowptr, K, nchunks,
                                                          chunk_row);
-  if (nchunks > 0) {
+  if (nchunks > 0 && list) {
     note_launch();
     chunk_split_kernel<<<(nchunks + 7) / 8, 256, 0, st>>>(rowptr, nnz, K, nchunks, chunk_row, list, counts);
   }
