@@ -187,6 +187,11 @@ csc_naive_kernel(CscArgs a, float* __restrict__ y) {
   }
 }
 
+static_assert(kCntLong % 2 == 0 && kCntLong + 2 <= kCntFeatSum, "an aligned 64-bit counter of its own");
+__host__ __device__ __forceinline__ unsigned long long* long_count(const CscArgs& a) {
+  return reinterpret_cast<unsigned long long*>(a.counts + kCntLong);
+}
+
 template <class T>
 __device__ __forceinline__ void row_add(T* y, float v) {
   // v + 0.0 is never -0.0, nor is a sum that it entered
@@ -306,12 +311,12 @@ csc_flat_kernel(CscArgs a, int elog, T* __restrict__ y, CscLong* queue, int qcap
     const int c0 = __shfl_sync(FULL, cs, sl), c1 = c0 + __shfl_sync(FULL, len, sl);
     const float x = __shfl_sync(FULL, xv, sl);
     const int nch = (c1 - c0 + kFlatChunk - 1) / kFlatChunk;
-    int at = 0;
-    if (lane == 0) at = atomicAdd(a.counts + kCntLong, nch);
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(long_count(a), (unsigned long long)nch);
     at = __shfl_sync(FULL, at, 0);
     for (int j = lane; j < nch; j += 32) {
       const int s0 = c0 + j * kFlatChunk, s1 = min(c1, s0 + kFlatChunk);
-      if (at + j < qcap) {
+      if (at + j < (unsigned long long)qcap) {
         queue[at + j] = CscLong{s0, s1, x};
       } else {  // only with repeated x keys: this lane's chunk on the spot
         for (int k = s0; k < s1; ++k) {
@@ -338,7 +343,7 @@ csc_flat_long_kernel(CscArgs a, T* __restrict__ y, const CscLong* queue, int qca
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   constexpr int U = 8;
-  const int cnt = min(*(volatile int*)(a.counts + kCntLong), qcap);
+  const int cnt = (int)min(*(volatile unsigned long long*)long_count(a), (unsigned long long)qcap);
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < cnt; c += nw) {
@@ -431,12 +436,12 @@ int launch_csc_lb(const CscArgs& a, const CscScratch& s, int variant, float* y,
 // c0 / c1 (optional) are cleared too: counters of the grid that follows.
 // NEG: y holds m / 2 doubles (16-byte aligned), which become -0.0.
 template <bool NEG>
-__global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, int* c1) {
+__global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, unsigned long long* c1) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (c0) *c0 = 0;
-    if (c1) *c1 = 0;
+    if (c1) *c1 = 0ull;
   }
   constexpr float hi = NEG ? -0.0f : 0.0f;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -455,7 +460,7 @@ __global__ void zero_fill_kernel(float* __restrict__ y, long long m, int* c0, in
 // whatever grid ran before it (the previous call's last kernel): its launch
 // and CTA start-up overlap that grid's tail (2.4 -> 1.2 us per kernel boundary
 // measured on B200), and its griddepcontrol.wait keeps the order.
-int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0, int* c1) {
+int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0, unsigned long long* c1) {
   if (m <= 0 && !c0 && !c1) return 0;
   const long long blocks = std::min<long long>((m + 1023) / 1024, (long long)num_sms * 4);
   note_launch();
@@ -583,7 +588,7 @@ static int launch_flat(const CscArgs& a, const CscScratch& s, T* y, long long co
   const long long blocks = std::min<long long>((words + 1023) / 1024, (long long)num_sms * 4);
   note_launch();
   if (launch_pdl(zero_fill_kernel<NEG>, dim3((unsigned)std::max(1LL, blocks)), dim3(256), 0, st,
-                 reinterpret_cast<float*>(y), words, a.counts + kCntBinlen, a.counts + kCntLong) != cudaSuccess)
+                 reinterpret_cast<float*>(y), words, a.counts + kCntBinlen, long_count(a)) != cudaSuccess)
     return -2;
   if (a.x_nnz <= 0) return 0;
   // entries per warp: enough that the grid is about one wave of warps

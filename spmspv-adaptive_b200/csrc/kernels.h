@@ -87,8 +87,8 @@ enum CounterSlot : int {
   kCntXnnz = 2,
   kCntBlocksTL = 3,
   kCntBlocksMG = 4,
-  kCntLong = 5,        // chunks of long columns
-  kCntDy = 6,          // nonzeros of the adjoint's dy
+  kCntDy = 5,          // nonzeros of the adjoint's dy
+  kCntLong = 6,        // chunks of long columns, 64-bit (slots 6..7): repeated x keys count past 2^31
   kCntFeatSum = 8,   // 64-bit (slots 8..9)
   kCntFeatMax = 10,
   kCntFeatMinInv = 11,
@@ -156,7 +156,8 @@ int launch_csc_naive_pairs(const CscArgs& a, const CscScratch& s, int group,
 
 // ---- vecconv.cu
 // y[0..m) = 0 with a kernel that lets the next grid launch early
-int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0 = nullptr, int* c1 = nullptr);
+int launch_zero_fill(float* y, long long m, int num_sms, cudaStream_t st, int* c0 = nullptr,
+                     unsigned long long* c1 = nullptr);
 // dense[0..len) from (key, val): a zero fill, then the scatter as a
 // programmatic dependent launch that reads its keys and values while the
 // fill runs; the scatter in turn lets the next grid start early
