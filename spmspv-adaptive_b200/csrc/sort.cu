@@ -405,11 +405,54 @@ int radix_sort_pairs(RadixBuffers& b, int n, int key_bits, int* err, cudaStream_
 // entry is written once, empty ranges included.  A thread owns four consecutive
 // positions, a warp reads 512 bytes per load, and the key before a thread's
 // first comes from its neighbour lane.
-__global__ void __launch_bounds__(256)
-sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int* __restrict__ ptr, int vec_ok) {
-  constexpr int U = 2;
-  const long long step = (long long)gridDim.x * blockDim.x * 4;
+//
+// A thread writes up to kBoundsNarrow entries by itself, a warp together a longer
+// gap; of that the whole tiles of kBoundsTile entries (counted from entry 0) are
+// left to the last `tiles` CTAs, each of which looks up the value of its tile's
+// first entry and fills the tile if the last has the same.  ToCSC of 8M columns
+// with all 2M nonzeros in 64 of them takes 0.14 ms so, 29.5 ms with one thread
+// alone on each gap (0.18 with the nonzeros spread out, either way); 16.8M keys
+// without a gap 39.5 us against 37.  Eight CTAs per SM: at 40 registers, six,
+// these took 44.
+constexpr int kBoundsNarrow = 32, kBoundsTile = 4096;
+
+// ptr[l..h] = p without the whole tiles in between (whole warp)
+__device__ __forceinline__ void bounds_fill(int* __restrict__ ptr, unsigned l, unsigned h, int p) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned c0 = (l + kBoundsTile - 1) / kBoundsTile * kBoundsTile, c1 = (h + 1) / kBoundsTile * kBoundsTile;
+  const unsigned end = c1 > c0 ? c0 : h + 1;
+  for (unsigned j = l + lane; j < end; j += 32) ptr[j] = p;
+  if (c1 > c0)
+    for (unsigned j = c1 + lane; j <= h; j += 32) ptr[j] = p;
+}
+
+__global__ void __launch_bounds__(256, 8)
+sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int* __restrict__ ptr, int vec_ok,
+                     int tiles) {
+  constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  if ((int)(gridDim.x - blockIdx.x) <= tiles) {
+    __shared__ int s_p;
+    const unsigned j0 = (unsigned)(blockIdx.x + tiles - gridDim.x) * kBoundsTile, last = j0 + kBoundsTile - 1;
+    if (threadIdx.x < 32) {
+      int l = 0, r = cnt;  // the first position whose key is >= j0 is in [l, r]; 32 probes per step
+      while (l < r) {
+        const int span = r - l, q = l + (int)(((long long)span * lane) >> 5);
+        const int c = __popc(__ballot_sync(FULL, __ldg(key + q) < j0));  // sorted: the first c are below
+        const int nl = c ? l + (int)(((long long)span * (c - 1)) >> 5) + 1 : l;
+        r = c < 32 ? l + (int)(((long long)span * c) >> 5) : r;
+        l = nl;
+      }
+      if (lane == 0) s_p = l == cnt || __ldg(key + l) >= last ? l : -1;
+    }
+    __syncthreads();
+    const int p = s_p;
+    if (p < 0) return;
+    for (int j = threadIdx.x; j < kBoundsTile; j += 256) ptr[j0 + j] = p;
+    return;
+  }
+  constexpr int U = 2;
+  const long long step = (long long)(gridDim.x - tiles) * blockDim.x * 4;
   const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   // whole warps stay in the loop: the condition is that of the warp's first lane
   for (long long b = first; b - 4 * lane <= cnt; b += U * step) {
@@ -424,17 +467,41 @@ sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int*
 #pragma unroll
         for (int q = 0; q < 4; ++q) k[u][q + 1] = i + q < cnt ? __ldg(key + i + q) : (unsigned)extent;
       }
-      k[u][0] = __shfl_up_sync(0xffffffffu, k[u][4], 1);
+      k[u][0] = __shfl_up_sync(FULL, k[u][4], 1);
       if (lane == 0 && i > 0 && i <= cnt) k[u][0] = __ldg(key + i - 1);
+    }
+    // sorted: no gap of the thread is wider than all of its keys are apart
+    bool wide = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      wide |= min(k[u][4], (unsigned)extent) - (b + u * step == 0 ? 0u : min(k[u][0], (unsigned)extent)) > kBoundsNarrow;
+    if (!__any_sync(FULL, wide)) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const long long i = b + u * step + q;
+          if (i > cnt) continue;
+          const int lo = i == 0 ? 0 : (int)min(k[u][q], (unsigned)extent) + 1;
+          const int hi = i == cnt ? extent : (int)min(k[u][q + 1], (unsigned)extent);
+          for (int j = lo; j <= hi; ++j) ptr[j] = (int)i;
+        }
+      }
+      continue;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const long long i = b + u * step + q;
-        if (i > cnt) continue;
         const int lo = i == 0 ? 0 : (int)min(k[u][q], (unsigned)extent) + 1;
-        const int hi = i == cnt ? extent : (int)min(k[u][q + 1], (unsigned)extent);
+        const int hi = i > cnt ? lo - 1 : i == cnt ? extent : (int)min(k[u][q + 1], (unsigned)extent);
+        for (unsigned w = __ballot_sync(FULL, hi - lo >= kBoundsNarrow); w; w &= w - 1) {
+          const int src = __ffs(w) - 1;
+          bounds_fill(ptr, (unsigned)__shfl_sync(FULL, lo, src), (unsigned)__shfl_sync(FULL, hi, src),
+                      (int)(i + 4 * (src - lane)));
+        }
+        if (hi - lo >= kBoundsNarrow) continue;
         for (int j = lo; j <= hi; ++j) ptr[j] = (int)i;
       }
     }
@@ -444,8 +511,9 @@ sorted_bounds_kernel(int cnt, const unsigned* __restrict__ key, int extent, int*
 int launch_sorted_bounds(int cnt, const unsigned* key, int extent, int* ptr, cudaStream_t st) {
   if (cnt <= 0) return cudaMemsetAsync(ptr, 0, 4 * ((size_t)extent + 1), st) == cudaSuccess ? 0 : -1;
   note_launch();
+  const int tiles = (int)(((long long)extent + 1) / kBoundsTile);
   const int grid = (int)std::min<long long>(((long long)cnt + 1 + 2047) / 2048, 148LL * 8);
-  sorted_bounds_kernel<<<grid, 256, 0, st>>>(cnt, key, extent, ptr, ((uintptr_t)key & 15u) == 0);
+  sorted_bounds_kernel<<<tiles + grid, 256, 0, st>>>(cnt, key, extent, ptr, ((uintptr_t)key & 15u) == 0, tiles);
   return 0;
 }
 
