@@ -17,6 +17,17 @@ import torch
 from .handle import SpmspvHandle
 
 
+def _sparse_limit(mode, threshold, m):
+    """The sparse adjoint is taken where dy has fewer nonzeros than this: all of
+    m where `mode` forces it, threshold * m otherwise (never for NaN)."""
+    if mode == "sparse":
+        return m + 1
+    most = threshold * m
+    if not most > 0:
+        return 0
+    return m + 1 if most > m else math.ceil(most)
+
+
 class SparseMatrix:
     """A CSR pattern on the GPU with a handle bound to it.
 
@@ -75,7 +86,7 @@ class SpMVFunction(torch.autograd.Function):
         if mode == "dense":
             op.h.spmv_backward(x, dy, dx, dvals)
         else:
-            limit = op.m + 1 if mode == "sparse" else min(math.ceil(op.sparse_threshold * op.m), op.m + 1)
+            limit = _sparse_limit(mode, op.sparse_threshold, op.m)
             # nothing waits for the handle's stream here: a dy that another
             # stream's allocator may hand out again is kept until it has been read
             if torch.cuda.current_stream(dy.device) != op.h.stream:
