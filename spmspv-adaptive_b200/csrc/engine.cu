@@ -926,9 +926,11 @@ extern "C" int spmx_spmv_backward(spmx_handle_t h, const float* x, const float* 
 extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const float* dy, int limit, void* scratch,
                                        float* dx, float* dvals) {
   SPMX_CHECK_HANDLE(h);
-  SPMX_TRY(backward_check(h, x, dy, dvals));
   limit = std::min(limit, h->m + 1);
-  if (limit <= 0 || h->m == 0) return spmx_spmv_backward(h, x, dy, dx, dvals);
+  // no rows: nothing to count, and dy may be a null pointer
+  if (h->m == 0 && limit > 0) return spmx_spmv_backward_sparse(h, x, nullptr, nullptr, 0, dx, dvals);
+  SPMX_TRY(backward_check(h, x, dy, dvals));
+  if (limit <= 0) return spmx_spmv_backward(h, x, dy, dx, dvals);
   if (!dx && !dvals) return SPMX_SUCCESS;
   HolaTables t;
   SPMX_TRY(backward_tables(h, &t));
