@@ -131,8 +131,10 @@ int spmx_copy_csc(spmx_handle_t h, int* d_row, int* d_colptr, float* d_val);
  * sort after ReadMTX (mtx.hpp:335-360) and the coo2csr of the reference's
  * drivers.  Synchronous; d_val may be NULL (pattern).  An index outside
  * [0,m) x [0,n) returns SPMX_ERR_INVALID_VALUE and leaves the handle as it
- * was.  Replaces the handle's CSR like spmx_input_csr (a CSC derived from
- * the previous CSR by spmx_to_csc is dropped). */
+ * was, as does a failed allocation.  A second call writes into the arrays of
+ * the first; if it fails after that (SPMX_ERR_CUDA), the handle has no matrix
+ * until the next input.  Replaces the handle's CSR like spmx_input_csr (a CSC
+ * derived from the previous CSR by spmx_to_csc is dropped). */
 int spmx_input_coo(spmx_handle_t h, int nnz, const int* d_row, const int* d_col,
                    const float* d_val);
 /* copy the handle's CSR into caller buffers (rowptr[m+1], col[nnz],

@@ -72,6 +72,19 @@ int key_bits(int extent) {
 
 using namespace spmx;
 
+// What the handle keeps of the matrix in its own CSR arrays, about to be written
+// or just written, is not that matrix's any more: features, chunk and hub tables,
+// and a CSC that spmx_to_csc derived from it.
+static void forget_csr(spmx_handle_t h) {
+  h->has_csr = false;
+  h->mat_feat_ready = false;
+  h->std_row_ready = false;
+  h->batch_chunk_ready = false;
+  h->ms_hubs_ready = false;
+  h->hola_rowptr = nullptr;
+  if (h->has_csc && h->csc_colptr == h->own_colptr) h->has_csc = false;
+}
+
 extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const int* col,
                               const float* val) {
   SPMX_CHECK_HANDLE(h);
@@ -111,6 +124,9 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   if (!ncol) rc = rc ? rc : dalloc((void**)&ncol, b, "csr col");
   if (val && !nval) rc = rc ? rc : dalloc((void**)&nval, b, "csr val");
   const unsigned* rows_sorted = (const unsigned*)row;
+  // a failure from here on leaves the handle without a matrix, unless the one it
+  // has is the caller's
+  if (!rc && h->own_csr_rowptr && h->rowptr == h->own_csr_rowptr) forget_csr(h);
   if (!rc && unsorted) {
     const int bits_c = key_bits(n), bits_r = key_bits(m);
     const int first = col_desc ? 0 : bits_c;
@@ -155,14 +171,8 @@ extern "C" int spmx_input_coo(spmx_handle_t h, int nnz, const int* row, const in
   h->rowptr = nrp;
   h->col = ncol;
   h->val = nval;
+  forget_csr(h);
   h->has_csr = true;
-  h->mat_feat_ready = false;
-  h->std_row_ready = false;
-  h->batch_chunk_ready = false;
-  h->ms_hubs_ready = false;
-  h->hola_rowptr = nullptr;  // the arrays stay where they are, with another pattern in them
-  // a CSC derived from the previous CSR by spmx_to_csc is stale now
-  if (h->has_csc && h->csc_colptr == h->own_colptr) h->has_csc = false;
   return SPMX_SUCCESS;
 }
 
