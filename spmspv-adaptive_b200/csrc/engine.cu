@@ -396,7 +396,7 @@ extern "C" int spmx_input_csc(spmx_handle_t h, int nnz, const int* csc_row,
 // buckets' shared-memory additions queue: one full row, x of 1M 489 us against 29,000.
 constexpr int kRowScanMax = 1 << 23;
 
-static bool row_scan_fits(spmx_handle_t h) {
+bool row_scan_fits(spmx_handle_t h) {
   return h->m <= kRowScanMax || (double)h->x_nnz * h->nnz >= (double)h->m / 4 * std::max(h->n, 1);
 }
 

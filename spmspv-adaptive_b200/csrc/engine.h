@@ -90,7 +90,7 @@ struct spmx_handle_s {
   int naive_row_group = 0;    // 0 = derive from mean row length
   int naive_col_group = 0;    // 0 = derive from mean column length
   int hola_vt = 8;
-  int lb_variant = SPMX_CSC_LB_MERGE;
+  int lb_variant = SPMX_CSC_LB_MERGE;  // blocks of the adaptive LB kernels; matters where products are sorted
   int lb_grid = 0;
 
   // cached features
@@ -200,6 +200,11 @@ cudaError_t kernel_smem_limit(const void* kernel, size_t bytes);
   do {                                                                         \
     if (!(h)) return set_error(SPMX_ERR_INVALID_VALUE, "NULL handle");         \
   } while (0)
+
+// whether the sorted write-back and the bucket method of the handle's x go
+// through dense rows; the blocks and bucket counts of their own kernels then play
+// no part
+bool row_scan_fits(spmx_handle_t h);
 
 // whether what is enqueued now goes into a graph instead of running
 inline bool stream_capturing(cudaStream_t st) {

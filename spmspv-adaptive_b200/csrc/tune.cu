@@ -8,8 +8,8 @@
 //     tiled (x window width) or round;
 //   - the lanes per row of the naive CSR kernel and per column of the naive
 //     CSC kernel;
-//   - merge-path vs fixed-nonzero blocks for the load-balanced CSC kernel;
-//   - the bucket count of the bucket kernel.
+//   - the bucket count of the bucket kernel, where the bucket kernels run (above
+//     8M rows, few products; through dense rows the count plays no part).
 // Results can be cached in a small text file keyed by a fingerprint of the
 // matrix (m, n, nnz and a sample of the row pointer), so a second process
 // applies them without timing.
@@ -51,7 +51,8 @@ __global__ void stride_keys_kernel(int* key, float* val, int k, int n) {
 
 struct Params {
   int spmv_type = SPMX_SPMV_HOLA, hola_vt = 8, tiled_rb = 0, tiled_win = 8192;
-  int row_group = 0, col_group = 0, lb_variant = SPMX_CSC_LB_MERGE, buckets = 256;
+  int row_group = 0, col_group = 0, buckets = 256;
+  int lb_variant = SPMX_CSC_LB_MERGE;  // not timed: a field of the cache file
   int csr5_sigma = -1;  // -1: the reference's rule
 };
 
@@ -278,6 +279,7 @@ extern "C" int spmx_autotune(spmx_handle_t h, const char* cache_path, int* spmv_
       }
       bt = 1e30f;
       for (int b : {64, 256, 1024}) {
+        if (row_scan_fits(h)) break;
         const float t = time_us([&] { return spmx_csc_bucket(h, 1.0f, nullptr, y, nullptr, nullptr, b); });
         if (t < bt) { bt = t; best.buckets = b; }
       }
