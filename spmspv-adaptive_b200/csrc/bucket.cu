@@ -137,7 +137,7 @@ bucket_reduce_kernel(int m, int rshift, int nb, const int* __restrict__ boff,
     if (tid == 0) { s_prefix = p; s_total = total; }
   }
   __syncthreads();
-  if (ykey) {
+  if (ykey || yval) {
     // words in order: round-robin rounds of NT words, exclusive scan per round
     unsigned run = s_prefix;
     for (int w0 = 0; w0 < nwords; w0 += NT) {
@@ -151,8 +151,8 @@ bucket_reduce_kernel(int m, int rshift, int nb, const int* __restrict__ boff,
         const int bit = __ffs(bb) - 1;
         bb &= bb - 1;
         const int rloc = wd * 32 + bit;
-        ykey[pos] = base_row + rloc;
-        yval[pos] = acc[rloc];
+        if (ykey) ykey[pos] = base_row + rloc;
+        if (yval) yval[pos] = acc[rloc];
         ++pos;
       }
       run += rt;
