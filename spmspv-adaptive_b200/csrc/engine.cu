@@ -227,7 +227,8 @@ extern "C" int spmx_create(int m, int n, int nnz, spmx_handle_t* out) {
   rc = rc ? rc : dalloc((void**)&h->ls.status, sizeof(unsigned long long) * h->ls.status_len,
                         "lookback status");
   rc = rc ? rc : dalloc((void**)&h->ls.ticket, sizeof(unsigned) * 4, "ticket");
-  rc = rc ? rc : dalloc((void**)&h->ls.counts, sizeof(unsigned) * h->ls.status_len, "range counts");
+  rc = rc ? rc : dalloc((void**)&h->ls.counts, sizeof(unsigned) * 2 * kCompactMaxRanges, "range counts");
+  if (!rc) h->inner_counts = h->ls.counts + kCompactMaxRanges;
   if (!rc && cudaMallocHost((void**)&h->h_pinned, sizeof(int) * 16) != cudaSuccess) {
     cudaGetLastError();
     rc = set_error(SPMX_ERR_ALLOC, "cudaMallocHost(pinned counters)");
@@ -579,7 +580,7 @@ extern "C" int spmx_sparse2bitarray(spmx_handle_t h) {
 
 static int dense_to_sparse(spmx_handle_t h, int len, const float* dense, int* key,
                            float* val, int slot, int* host_count) {
-  if (launch_compact_nonzero(len, dense, key, val, h->d_counts + slot, h->ls, h->stream, 0,
+  if (launch_compact_nonzero(len, dense, key, val, h->d_counts + slot, h->ls.counts, h->stream, 0,
                              host_count ? h->h_pinned : nullptr))
     return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
   SPMX_TRY(launch_ok("dense2sparse"));
@@ -621,13 +622,10 @@ static int ensure_scan_tiles(spmx_handle_t h, long long tiles) {
   if (tiles <= h->ls.status_len) return SPMX_SUCCESS;
   SPMX_CUDA(cudaStreamSynchronize(h->stream));
   dfree(h->ls.status);
-  dfree(h->ls.counts);
   h->ls.status = nullptr;
-  h->ls.counts = nullptr;
   h->ls.status_len = 0;
   const int len = (int)(tiles + 4);
   SPMX_TRY(dalloc((void**)&h->ls.status, sizeof(unsigned long long) * len, "lookback status"));
-  SPMX_TRY(dalloc((void**)&h->ls.counts, sizeof(unsigned) * len, "range counts"));
   SPMX_CUDA(cudaMemset(h->ls.status, 0, sizeof(unsigned long long) * len));
   h->ls.status_len = len;
   return SPMX_SUCCESS;
@@ -638,7 +636,6 @@ extern "C" int spmx_dense2sparse_outer(spmx_handle_t h, int m, const float* dens
   SPMX_CHECK_HANDLE(h);
   if (m < 0 || (m > 0 && (!dense || !key || !val)))
     return set_error(SPMX_ERR_INVALID_VALUE, "bad dense2sparse_outer arguments");
-  SPMX_TRY(ensure_scan_tiles(h, ((long long)m + 2047) / 2048));
   return dense_to_sparse(h, m, dense, key, val, kCntYnnz, ynnz);
 }
 
@@ -666,8 +663,7 @@ extern "C" int spmx_dense2sparse_to_host(spmx_handle_t h, int m, const float* de
     SPMX_TRY(host_mapped(h_key, "h_key"));
     SPMX_TRY(host_mapped(h_val, "h_val"));
   }
-  SPMX_TRY(ensure_scan_tiles(h, ((long long)m + 2047) / 2048));
-  if (launch_compact_nonzero(m, dense, h_key, h_val, h_count, h->ls, h->stream))
+  if (launch_compact_nonzero(m, dense, h_key, h_val, h_count, h->ls.counts, h->stream))
     return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
   return launch_ok("dense2sparse_to_host");
 }
@@ -940,7 +936,7 @@ extern "C" int spmx_spmv_backward_auto(spmx_handle_t h, const float* x, const fl
   float* val = (float*)scratch + std::min(limit, h->m);
   int* count = h->d_counts + kCntDy;
   const DevGate sparse{count, limit, true}, dense{count, limit, false};
-  if (launch_compact_nonzero(h->m, dy, key, val, count, h->ls, st, limit))
+  if (launch_compact_nonzero(h->m, dy, key, val, count, h->inner_counts, st, limit))
     return set_error(SPMX_ERR_INVALID_VALUE, "compaction capacity");
   if (h->nnz == 0) dvals = nullptr;
   launch_backward_clear(h->n, h->nnz, dx, dvals, !backward_by_csc(h), h->num_sms, sparse, st);
@@ -1026,7 +1022,7 @@ static int launch_row_scan(spmx_handle_t h, float alpha, float* y, int* ykey, fl
   SPMX_TRY(ensure_sort_scratch(h));
   if (launch_csc_flat_rows(a, h->cs, h->srow, h->col_max, h->row_max, h->num_sms, h->stream) ||
       launch_compact_rows(h->m, h->srow, y, ykey, yval, h->d_counts + kCntYnnz,
-                          h->d_counts + kCntBinlen, cap, h->d_err, h_counts, h->ls, h->stream))
+                          h->d_counts + kCntBinlen, cap, h->d_err, h_counts, h->inner_counts, h->stream))
     return set_error(SPMX_ERR_CUDA, "csc spmspv launch");
   return launch_ok("csc row scan");
 }

@@ -55,7 +55,10 @@ struct spmx_handle_s {
   unsigned long long* d_u64 = nullptr;  // 4 words
   int* h_pinned = nullptr;         // 16 ints of pinned host memory
 
-  spmx::ScanScratch ls{};          // look-back status + ticket
+  spmx::ScanScratch ls{};          // look-back status + ticket; range counts of the dense2sparse calls
+  // range counts of the compactions inside an SpMSpV or an adjoint, which may run
+  // beside a dense2sparse on another stream
+  unsigned* inner_counts = nullptr;
 
   // CSC SpMSpV scratch
   spmx::CscScratch cs{};

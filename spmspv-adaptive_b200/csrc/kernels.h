@@ -77,8 +77,11 @@ struct ScanScratch {
   unsigned long long* status;  // tile status words
   int status_len;              // capacity in tiles
   unsigned* ticket;            // 4 words, zeroed once: ticket, epoch, publish count
-  unsigned* counts;            // status_len per-range counts (the compaction's first pass)
+  unsigned* counts;            // kCompactMaxRanges per-range counts (the compaction's first pass)
 };
+
+// ranges of a compaction, each counted by a CTA before any is written
+constexpr int kCompactMaxRanges = 1024;
 
 // indices into the handle's device counter block
 enum CounterSlot : int {
@@ -170,14 +173,16 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st);
 // limit > 0: nothing but the count is written where it reaches the limit.
 // h_counts (optional, two ints of page-locked host memory; without a limit): the
 // count once the grid is done
+// range_counts: kCompactMaxRanges words that no compaction beside this one uses
 int launch_compact_nonzero(int len, const float* dense, int* key, float* val,
-                           int* d_count, ScanScratch& ls, cudaStream_t st, int limit = 0,
+                           int* d_count, unsigned* range_counts, cudaStream_t st, int limit = 0,
                            int* h_counts = nullptr);
 // keys/vals (each optional) of the entries of acc[0..len) other than -0.0, in
 // order; dense (optional): all of them, rounded, the others 0; count -> *d_count.
 // *total above cap >= 0: kDevErrCapacity.  h_counts (optional, page-locked host
 // memory): the count and *total once the grid is done
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        const int* total, int cap, int* err, int* h_counts, ScanScratch& ls, cudaStream_t st);
+                        const int* total, int cap, int* err, int* h_counts, unsigned* range_counts,
+                        cudaStream_t st);
 
 }  // namespace spmx

@@ -76,7 +76,6 @@ __global__ void dense2bits_kernel(int len, const float* __restrict__ dense,
 // for 1M elements whatever the look-back window: its CTAs sat at a barrier
 // while warp 0 took a ticket, published and looked back.  Here nothing waits
 // on another CTA.
-constexpr int kCompactMaxRanges = 1024;
 
 // T = double: the entries kept are those other than -0.0 (launch_compact_rows).
 __device__ __forceinline__ bool compact_keep(float v) { return v != 0.0f; }
@@ -247,8 +246,8 @@ int launch_dense2bits(int len, const float* dense, int* bits, cudaStream_t st) {
 }
 
 template <class T>
-static int launch_compact(int len, const T* in, float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
-                          cudaStream_t st, int limit, const int* total, int cap, int* err, int* h_counts) {
+static int launch_compact(int len, const T* in, float* dense, int* key, float* val, int* d_count,
+                          unsigned* range_counts, cudaStream_t st, int limit, const int* total, int cap, int* err, int* h_counts) {
   constexpr int NT = 256, VT = 8;
   if (len <= 0) {
     cudaMemsetAsync(d_count, 0, sizeof(int), st);
@@ -260,25 +259,26 @@ static int launch_compact(int len, const T* in, float* dense, int* key, float* v
   const long long subs = (len + sub - 1) / sub;
   const long long per = sub * ((subs + kCompactMaxRanges - 1) / kCompactMaxRanges);
   const long long ranges = (len + per - 1) / per;
-  if (ranges > ls.status_len || !ls.counts) return -1;
+  if (!range_counts) return -1;
   note_launch(2);
   if (launch_pdl(compact_count_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
-                 ls.counts) != cudaSuccess ||
+                 range_counts) != cudaSuccess ||
       launch_pdl(compact_write_kernel<NT, VT, T>, dim3((unsigned)ranges), dim3(NT), 0, st, (long long)len, per, in,
-                 (const unsigned*)ls.counts, dense, key, val, d_count, (unsigned)limit, total, cap, err,
+                 (const unsigned*)range_counts, dense, key, val, d_count, (unsigned)limit, total, cap, err,
                  h_counts) != cudaSuccess)
     return -2;
   return 0;
 }
 
-int launch_compact_nonzero(int len, const float* dense, int* key, float* val, int* d_count, ScanScratch& ls,
+int launch_compact_nonzero(int len, const float* dense, int* key, float* val, int* d_count, unsigned* range_counts,
                            cudaStream_t st, int limit, int* h_counts) {
-  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, ls, st, limit, nullptr, -1, nullptr, h_counts);
+  return launch_compact(len, dense, (float*)nullptr, key, val, d_count, range_counts, st, limit, nullptr, -1, nullptr, h_counts);
 }
 
 int launch_compact_rows(int len, const double* acc, float* dense, int* key, float* val, int* d_count,
-                        const int* total, int cap, int* err, int* h_counts, ScanScratch& ls, cudaStream_t st) {
-  return launch_compact(len, acc, dense, key, val, d_count, ls, st, 0, total, cap, err, h_counts);
+                        const int* total, int cap, int* err, int* h_counts, unsigned* range_counts,
+                        cudaStream_t st) {
+  return launch_compact(len, acc, dense, key, val, d_count, range_counts, st, 0, total, cap, err, h_counts);
 }
 
 }  // namespace spmx
