@@ -64,10 +64,13 @@ extern "C" {
 #define SPMX_SPMV_TILED 2  /* row-block x column-window tiles (no reference counterpart) */
 #define SPMX_SPMV_ROUND 3  /* column-ordered rounds, row-owner reduction (no reference counterpart) */
 
-/* ---- CSC SpMSpV work distributions and write-backs (H:1824-2201) */
+/* ---- CSC SpMSpV work distributions and write-backs (H:1824-2201).  The two
+ *      load-balanced distributions are one with a dense y (a warp balances the
+ *      columns of up to 32 x entries, long columns go by chunks), and all three
+ *      with a sorted y up to 8M rows; they part where products are sorted. */
 #define SPMX_CSC_NAIVE     0  /* group of threads per x nonzero            */
-#define SPMX_CSC_LB_MERGE  1  /* merge-path partition over (x entries, nnz) */
-#define SPMX_CSC_LB_TWOLAYER 2/* fixed nnz per CTA, block-start table      */
+#define SPMX_CSC_LB_MERGE  1  /* sorted products: merge-path blocks        */
+#define SPMX_CSC_LB_TWOLAYER 2/* sorted products: fixed nnz per CTA        */
 #define SPMX_CSC_BUCKET    3  /* dense rows; above 8M rows row-block buckets */
 #define SPMX_WB_ATOMIC     0  /* dense y via atomics (+ optional compaction)*/
 #define SPMX_WB_SORT       1  /* sorted (row,val) of every row reached      */
@@ -404,8 +407,8 @@ int spmx_run_adaptive(spmx_handle_t h, float alpha, float* d_y, int* kernel_used
 /* Per-matrix autotuner (no reference counterpart beyond the reference's
  * Hola-vs-CSR5 timing, TEST/generate_model_data.cu:487-516): times the
  * load-balanced SpMV back-ends (Hola 4/8/16 nonzeros per thread, CSR5, tiled
- * geometries), the naive kernels' lanes per row / column and the bucket count,
- * and keeps the fastest.
+ * geometries), the naive kernels' lanes per row / column and (where the bucket
+ * kernels run) the bucket count, and keeps the fastest.
  * cache_path (may be NULL): a text file of tuned parameters keyed by a matrix
  * fingerprint; a hit applies them without timing.  spmv_type_out (may be NULL)
  * receives the chosen SpMV back-end. */

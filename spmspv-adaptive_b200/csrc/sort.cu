@@ -14,10 +14,11 @@
 // never make a round trip through memory; the tile is put in digit order in
 // shared memory first, so a warp's stores cover runs of consecutive addresses.
 //
-// What bounds a pass: instruction issue and the shared-memory exchange (about
-// 130 warp instructions per 32 items with two payloads) ahead of DRAM, which
-// moves 2 x 12 bytes per item.  16.8M items with two payloads: 119 us per pass
-// (3.4 TB/s) and 34 us for the histogram; the form before (per-tile histogram,
+// What bounds a pass: the shared-memory pipe (86% busy; issue slots 49%, DRAM
+// 33%) with the ranking and the exchange, about 140 warp instructions per 32
+// items with two payloads; 32 warps per SM at 64 registers.  16.8M items with two
+// payloads: 119 us per pass (3.4 TB/s; 140 with two keys) and 34 us for the
+// histogram (105 for the five digits of two keys: issue slots, 71%); the form before (per-tile histogram,
 // scan of the histograms, scatter straight from registers, each 4-byte store in
 // a sector of its own) took 430 + 37 + 13 us per pass.  Measured beside it:
 // peers by __match_any_sync 210 us, by one ballot per digit bit 143 us, by the

@@ -127,7 +127,8 @@ __device__ __forceinline__ void split_row_contribute(
 // the up to kShortRow nonzeros past its end that its last row may have, so no row
 // is split; otherwise split rows meet as in spmv_chunk_kernel.
 //
-// What bounds it: instruction issue, then DRAM latency.  5-point Laplacian 2048^2
+// What bounds it: latency at 32 warps per SM (64 registers); L1/TEX is 68% busy,
+// issue slots 53%, DRAM 52%.  5-point Laplacian 2048^2
 // (21.0M nonzeros, 218 MB): 43 us (5.1 TB/s) with no check per element where the
 // chunk is inside the matrix and its largest column in range, 49 with them (47
 // warp instructions per 32 nonzeros), 97 by the segmented scan; one CTA per chunk
