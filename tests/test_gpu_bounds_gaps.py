@@ -66,11 +66,12 @@ def test_eight_million(torch_cuda, kind):
         h = SpmspvHandle(small, n, nnz)
         h.InputCOO(nnz, dev(other, torch), dev(col, torch))
         ts = []
-        for _ in range(6):
+        for _ in range(12):
             torch.cuda.synchronize()
             t0 = time.perf_counter()
             h.ToCSC()
             ts.append(time.perf_counter() - t0)
         return min(ts)
 
-    assert best(here) < 3 * best(even)
+    # host time of a synchronous call, best of twelve; a gap per thread took 12 to 160 times as long
+    assert best(here) < 8 * best(even)
